@@ -209,6 +209,8 @@ static int ctx_init(bwacuda_ctx *c)
     int pageable = 0;
     if ((e = cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, c->device)) != cudaSuccess) return cuda_status(e);
     c->pageable_access = pageable != 0;
+    if ((e = cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device)) != cudaSuccess) return cuda_status(e);
+    if (c->nsm < 1) c->nsm = 1;
     if ((e = c->d_misc.ensure(4096)) != cudaSuccess) return cuda_status(e);
     if ((e = c->h_misc.ensure(4096)) != cudaSuccess) return cuda_status(e);
     if ((e = cudaMemset(c->d_misc.p, 0, 4096)) != cudaSuccess) return cuda_status(e);
@@ -697,20 +699,44 @@ int launch_long_unbucketed(bwacuda_ctx *c, DevBuf &xl, const uint8_t *seq, const
 
 namespace bwacuda {
 
+// Lanes of a pair group (0: one job per group) and lanes per job of the 32-bit wavefront for a
+// launch of n jobs: what the options or the autotuner set, else by the jobs an SM gets.  Few jobs
+// leave lanes idle, so a job is spread over more of them and its latency sets the time; many jobs
+// want the fewest lanes, whose rows cost the fewest instructions.  Device-resident calls of 150 bp
+// queries against 750 bp windows on 152 SMs, microseconds:
+//   jobs      1 job in 32 / 16 / 8 lanes    2 jobs in 16 / 8 / 4 lanes
+//   1,024        309    323    408               407    480    666
+//   4,096        648    573    532               483    483    667
+//   16,384      2019   1657   1426              1155   1097    995
+//   200,000    22343  17663  14717             11283   9315   8603
+// (100 x 400, 60 x 700 and 240 x 1200 bp order the same way.)
+struct RescueShape {
+    int pair, lanes;
+};
+static RescueShape rescue_shape(const bwacuda_ctx *c, size_t n)
+{
+    const size_t per_sm = n / (size_t)c->nsm;
+    const int lanes = c->rescue_lanes ? c->rescue_lanes : (per_sm < 8 ? 32 : (per_sm < 24 ? 16 : 8));
+    if (c->rescue_pair >= 0) return {c->rescue_pair, c->rescue_lanes ? c->rescue_lanes : 16};
+    if (c->rescue_lanes || per_sm < 16) return {0, lanes};  // lanes set by the caller: the kernel they name
+    return {per_sm < 64 ? 8 : 4, lanes};
+}
+
 // Narrow-cell rescue jobs: the register wavefront when the padded query fits
 // 16 lanes x 32 columns (and the kernel choice allows it), else the
 // shared-memory thread-per-job kernel.  Wide jobs always go to the latter.
 cudaError_t rescue_narrow_launch(bwacuda_ctx *c, const RescueLaunch &L)
 {
     if (c->rescue_kernel == BWACUDA_RESCUE_AUTO && L.qcap <= rescue_wf_max_qpad() && L.only_wide != 2) {
-        if (!c->rescue_pair) return rescue_wf_launch(L, L.qcap, c->rescue_lanes);
+        const RescueShape sh = rescue_shape(c, L.n);
+        if (!sh.pair) return rescue_wf_launch(L, L.qcap, sh.lanes);
         // jobs whose values fit a byte: two per group; the rest in the 32-bit wavefront
         int cols = 0;
-        cudaError_t e = rescue_wf2_launch(L, L.qcap, c->rescue_pair, &cols);
+        cudaError_t e = rescue_wf2_launch(L, L.qcap, sh.pair, &cols);
         if (e != cudaSuccess) return e;
         RescueLaunch R = L;
         R.pair_cols = cols;
-        return rescue_wf_launch(R, R.qcap, c->rescue_lanes);
+        return rescue_wf_launch(R, R.qcap, sh.lanes);
     }
     return rescue_tpj_launch(L, false);
 }

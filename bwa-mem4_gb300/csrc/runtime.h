@@ -92,8 +92,9 @@ struct bwacuda_ctx {
     int ext_path = BWACUDA_PATH_BATCHED;
     bool use_graphs = true;
     int rescue_kernel = BWACUDA_RESCUE_AUTO;
-    int rescue_lanes = 16;  // lanes per job of the register wavefront (8, 16, 32)
-    int rescue_pair = 0;  // lanes of a group holding two byte-range jobs (rescue_wf2.cuh): 4, 8, 16; 0 off
+    int nsm = 1;            // SMs of the device
+    int rescue_lanes = 0;  // lanes per job of the register wavefront (8, 16, 32); 0: not set
+    int rescue_pair = -1;  // lanes of a group holding two byte-range jobs (rescue_wf2.cuh): 4, 8, 16; 0 off; -1: not set
     bool ungapped = false;  // ungapped-diagonal fast path on the batched extension path
     int long_lanes = 16;    // lanes per job of the group-per-job extension kernel (8, 16, 32)
     int long_slide = 1;     // thread-per-job window kernel on the open-ended buckets: 0 off, 1 auto, 2 always

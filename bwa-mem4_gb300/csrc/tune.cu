@@ -100,7 +100,7 @@ extern "C" int bwacuda_get_tuning(bwacuda_ctx *c, bwacuda_tuning *out)
     out->persist_block = tb;
     out->grab = grab;
     out->bucket_step = step;
-    out->rescue_lanes = c->rescue_lanes;
+    out->rescue_lanes = c->rescue_lanes ? c->rescue_lanes : 16;
     out->rescue_kernel = c->rescue_kernel;
     out->candidates = c->tune_candidates;
     out->ext_gcups = c->tuned_ext_gcups;
@@ -108,7 +108,7 @@ extern "C" int bwacuda_get_tuning(bwacuda_ctx *c, bwacuda_tuning *out)
     const int lq = batched_get_long(c);
     out->long_qlen = lq == INT_MAX ? 0 : lq;
     out->long_lanes = c->long_lanes;
-    out->rescue_pair = c->rescue_pair;
+    out->rescue_pair = c->rescue_pair > 0 ? c->rescue_pair : 0;
     out->reserved = 0;
     return BWACUDA_OK;
 }

@@ -131,7 +131,7 @@ typedef struct bwacuda_ctx bwacuda_ctx;
 #define BWACUDA_OPT_GRAB 7
 /* Batched extension: query-length bucket width below 257 columns (16, 32 or 64). */
 #define BWACUDA_OPT_BUCKET_STEP 8
-/* Rescue register wavefront: lanes per job (8, 16 or 32). */
+/* Rescue register wavefront: lanes per job (8, 16 or 32); set alone, one job per group. */
 #define BWACUDA_OPT_RESCUE_LANES 9
 /* Batched extension: settle jobs whose seed diagonal carries at most
  * (o_min + e_min - 1) / (a + b) mismatches in closed form before the DP (the
@@ -155,8 +155,9 @@ typedef struct bwacuda_ctx bwacuda_ctx;
 /* Mate rescue, register wavefront: 4, 8 or 16 = jobs whose every value fits a byte
  * (min(qlen, tlen) * max_sc <= 255, padded query <= 256 columns, bwa-shaped matrix) run two
  * per group of that many lanes, one in each 16-bit lane of the DPX instructions (4 lanes: the
- * most columns per lane); the others stay in the 32-bit wavefront.  1 = 4.  0 (default before
- * tuning) = one job per group.  Results never depend on it. */
+ * most columns per lane); the others stay in the 32-bit wavefront.  1 = 4.  0 = one job per
+ * group.  Until this option, BWACUDA_OPT_RESCUE_LANES or the autotuner sets a shape, each launch
+ * picks one by its number of jobs.  Results never depend on it. */
 #define BWACUDA_OPT_RESCUE_PAIR 14
 /* Batched extension, the open-ended query-length buckets (queries too long for a thread's
  * shared-memory row): 1 (default) = a thread-per-job kernel holding each job's row in a window
