@@ -259,6 +259,7 @@ extern "C" void bwacuda_ctx_destroy(bwacuda_ctx *c)
     ats_release(c);
     global_release(c);
     retry_release(c);
+    rescue_release(c);
     ref_release(c);
     batched_release(c);
     delete c;
@@ -1013,39 +1014,26 @@ extern "C" int bwacuda_ksw_local_fwd_batch(bwacuda_ctx *c, const bwacuda_fwd_job
 
 namespace {
 
-// Max query length over device jobs (synchronous: sizes the shared memory), and whether any
-// job carries a negative length (out[1] != 0).
-template <typename J>
-__global__ void qmax_kernel(const J *__restrict__ jobs, uint32_t n, int *__restrict__ out)
+// Max query length over device jobs (synchronous: sizes the shared memory).
+__global__ void qmax_kernel(const bwacuda_dev_ext_job *__restrict__ jobs, uint32_t n, int *__restrict__ out)
 {
-    int mx = 0, neg = 0;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    int mx = 0;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
         mx = max(mx, jobs[k].qlen);
-        neg |= jobs[k].qlen < 0 || jobs[k].tlen < 0;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        neg |= __shfl_xor_sync(0xffffffffu, neg, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(out, mx);
-        if (neg) atomicOr(out + 1, 1);
-    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
 }
 
-template <typename J>
-int device_qmax(bwacuda_ctx *c, const J *jobs, size_t n, cudaStream_t s, int *qmax, bool *negative = nullptr)
+int device_qmax(bwacuda_ctx *c, const bwacuda_dev_ext_job *jobs, size_t n, cudaStream_t s, int *qmax)
 {
     int *d = reinterpret_cast<int *>((char *)c->d_misc.p + 32);
-    cudaError_t e = cudaMemsetAsync(d, 0, 8, s);
+    cudaError_t e = cudaMemsetAsync(d, 0, 4, s);
     if (e != cudaSuccess) return cuda_status(e);
     uint32_t grid = (uint32_t)std::min<size_t>((n + 255) / 256, 1024);
-    if (grid) qmax_kernel<J><<<grid, 256, 0, s>>>(jobs, (uint32_t)n, d);
-    if ((e = cudaMemcpyAsync((char *)c->h_misc.p + 32, d, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_status(e);
+    if (grid) qmax_kernel<<<grid, 256, 0, s>>>(jobs, (uint32_t)n, d);
+    if ((e = cudaMemcpyAsync((char *)c->h_misc.p + 32, d, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_status(e);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_status(e);
     *qmax = *reinterpret_cast<int *>((char *)c->h_misc.p + 32);
-    if (negative) *negative = *reinterpret_cast<int *>((char *)c->h_misc.p + 36) != 0;
     return BWACUDA_OK;
 }
 
@@ -1132,66 +1120,6 @@ extern "C" int bwacuda_ksw_align2_device(bwacuda_ctx *c, const uint8_t *d_seq,
 
 namespace bwacuda {
 
-// One piece of a device-resident rescue call (n <= the context's piece size).
-static int ksw_align2_device_piece(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda_dev_rescue_job *d_jobs, size_t n,
-                                   const Scoring &sc, int minsc, int mode, int lanes, bwacuda_rescue_result *d_out,
-                                   cudaStream_t s)
-{
-    int rc;
-    int qmax = 0;
-    bool negative = false;
-    if ((rc = device_qmax(c, d_jobs, n, s, &qmax, &negative)) != BWACUDA_OK) return rc;
-    if (negative) return BWACUDA_EINVAL;  // a negative length would size the tracker scratch wrongly
-    const int qcap = (qmax + 15) / 16 * 16 + 16;
-    if ((size_t)qcap > rescue_tpj_smem_limit_qcap(false)) return BWACUDA_EUNSUPPORTED;
-    // tracker scratch: exclusive scan of per-job capacities, total read back to size the pool
-    cudaError_t e;
-    size_t tmp_need = 0;
-    rescue_scratch_offsets(d_jobs, n, nullptr, nullptr, 0, &tmp_need, s);
-    if ((e = c->d_dev_aux.ensure(n * 8 + tmp_need + 64)) != cudaSuccess) return cuda_status(e);
-    uint64_t *off = static_cast<uint64_t *>(c->d_dev_aux.p);
-    void *tmp = static_cast<char *>(c->d_dev_aux.p) + n * 8;
-    if ((e = rescue_scratch_offsets(d_jobs, n, off, tmp, tmp_need, nullptr, s)) != cudaSuccess) return cuda_status(e);
-    // total = off[n-1] + cap(n-1): read the last job's offset and tlen
-    uint64_t last_off = 0;
-    bwacuda_dev_rescue_job last;
-    if ((e = cudaMemcpyAsync(&last_off, off + n - 1, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_status(e);
-    if ((e = cudaMemcpyAsync(&last, d_jobs + n - 1, sizeof(last), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_status(e);
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_status(e);
-    const uint64_t total = last_off + rescue_scratch_entries(last.tlen);
-    if ((e = c->d_dev_scratch.ensure(total * sizeof(uint2) + 16)) != cudaSuccess) return cuda_status(e);
-    RescueLaunch L;
-    L.seq = d_seq;
-    L.jobs = d_jobs;
-    L.order = nullptr;
-    L.count_ptr = nullptr;
-    L.n = n;
-    L.sc = sc;
-    L.mode = mode;
-    L.lanes = lanes;
-    L.minsc = minsc;
-    L.qcap = qcap;
-    L.only_wide = 0;
-    L.scratch = static_cast<uint2 *>(c->d_dev_scratch.p);
-    L.scratch_off = off;
-    L.out_aln = d_out;
-    L.out_fwd = nullptr;
-    L.err = d_err(c);
-    L.stream = s;
-    const bool wide_fits = (size_t)qcap <= rescue_tpj_smem_limit_qcap(true);
-    L.only_wide = wide_fits ? 0 : 2;
-    if ((e = rescue_narrow_launch(c, L)) != cudaSuccess) return cuda_status(e);
-    if (wide_fits) {
-        L.only_wide = 1;
-        if ((e = rescue_tpj_launch(L, true)) != cudaSuccess) return cuda_status(e);
-        c->stats.kernel_launches += 1;
-    }
-    c->stats.kernel_launches += 4;
-    c->stats.rescue_jobs += n;
-    c->dev_pending_stream = s;
-    return BWACUDA_OK;
-}
-
 // bwacuda_ksw_align2_device with the context lock already held.
 int ksw_align2_device_locked(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda_dev_rescue_job *d_jobs, size_t n,
                              const bwacuda_scoring *scp, int minsc, int max_sc, int mode, int lanes,
@@ -1209,7 +1137,7 @@ int ksw_align2_device_locked(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda
     // consecutive pieces on the stream: the scans and kernels index a piece in 32 bits
     for (size_t off = 0; off < n; off += c->dev_piece) {
         const size_t m = std::min(c->dev_piece, n - off);
-        if ((rc = ksw_align2_device_piece(c, d_seq, d_jobs + off, m, sc, minsc, mode, lanes, d_out + off, s)))
+        if ((rc = rescue_device_piece(c, d_seq, d_jobs + off, m, sc, minsc, mode, lanes, d_out + off, s)))
             return rc;
     }
     return BWACUDA_OK;

@@ -67,6 +67,7 @@ struct AtsState;      // device-side gather of host buffers (ats.cu)
 struct GlobalState;   // ksw_global2 buffers (global.cu)
 struct RetryState;    // band-doubling retry buffers (retry.cu)
 struct RefState;      // reference in HBM for rescue windows (window.cu)
+struct RescueState;   // rescue batches: class streams and work buffers (rescue_batch.cu)
 
 int cuda_status(cudaError_t e);
 Scoring make_scoring(int m, const int8_t *mat, int o_del, int e_del, int o_ins, int e_ins);
@@ -110,6 +111,7 @@ struct bwacuda_ctx {
     bwacuda::GlobalState *global = nullptr;
     bwacuda::RetryState *retry = nullptr;
     bwacuda::RefState *ref = nullptr;
+    bwacuda::RescueState *rescue = nullptr;
     bwacuda::ServerState *server = nullptr;
 };
 
@@ -173,6 +175,12 @@ int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int 
 void ats_release(bwacuda_ctx *c);
 int ats_gather_ext(bwacuda_ctx *c, const bwacuda_ext_job *hj, size_t n, int w, DevBuf &seq, DevBuf &djobs,
                    DevBuf &tmp, HostBuf &htmp, cudaStream_t s);
+
+// rescue_batch.cu
+void rescue_release(bwacuda_ctx *c);
+int rescue_device_piece(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda_dev_rescue_job *d_jobs, size_t n,
+                        const Scoring &sc, int minsc, int mode, int lanes, bwacuda_rescue_result *d_out,
+                        cudaStream_t s);
 
 // retry.cu
 void retry_release(bwacuda_ctx *c);
