@@ -923,25 +923,38 @@ int rescue_host(bwacuda_ctx *c, const JobT *jobs, size_t n, int m, const int8_t 
     Scoring sc = make_scoring(m, mat, o_del, e_del, o_ins, e_ins);
     sc.max_sc = max_sc;  // the caller's max_sc sizes the padding rule and the score2 window
     const size_t osz = mode == 2 ? sizeof(bwacuda_fwd_result) : sizeof(bwacuda_rescue_result);
-    {   // reference batch-width label (statistics only)
-        std::vector<int> ql(n), tl(n);
+    bool standard = m == 5;
+    for (int i = 0; i < 4 && standard; ++i) {
+        for (int j = 0; j < 4; ++j)
+            if (mat[i * 5 + j] != (i == j ? mat[0] : mat[1])) standard = false;
+        if (mat[i * 5 + 4] != -1 || mat[20 + i] != -1) standard = false;
+    }
+    if (standard && mat[24] != -1) standard = false;
+    auto count_width = [&](bool u8ok, bool i16ok) {  // reference batch-width label (statistics only)
+        if (!standard) c->stats.rescue_width_i32++;
+        else if (u8ok) c->stats.rescue_width_u8++;
+        else if (i16ok) c->stats.rescue_width_i16++;
+        else c->stats.rescue_width_i32++;
+    };
+    if (c->pageable_access && c->host_gather != BWACUDA_GATHER_HOST) {
         bool u8ok = true, i16ok = true;
-        bool standard = m == 5;
-        for (int i = 0; i < 4 && standard; ++i) {
-            for (int j = 0; j < 4; ++j)
-                if (mat[i * 5 + j] != (i == j ? mat[0] : mat[1])) standard = false;
-            if (mat[i * 5 + 4] != -1 || mat[20 + i] != -1) standard = false;
-        }
-        if (standard && mat[24] != -1) standard = false;
+        uint64_t cells = 0;
+        rc = rescue_batch_gather(c, jobs, n, sc, minsc, mode, lanes, out, &u8ok, &i16ok, &cells);
+        const int st = collect_device_status(c, c->slot[0].stream, nullptr);
+        if (!rc) rc = st;
+        count_width(u8ok, i16ok);
+        c->stats.rescue_jobs += n;
+        c->stats.rescue_cells += cells;
+        return rc;
+    }
+    {
+        bool u8ok = true, i16ok = true;
         for (size_t k = 0; k < n; ++k) {
             long long ceil = (long long)std::min(jobs[k].qlen, jobs[k].tlen) * max_sc;
             if (!(ceil < 250 && jobs[k].qlen < 250)) u8ok = false;
             if (!(ceil < 30000 && jobs[k].tlen < 30000)) i16ok = false;
         }
-        if (!standard) c->stats.rescue_width_i32++;
-        else if (u8ok) c->stats.rescue_width_u8++;
-        else if (i16ok) c->stats.rescue_width_i16++;
-        else c->stats.rescue_width_i32++;
+        count_width(u8ok, i16ok);
     }
     const size_t CH = c->chunk_jobs;
     ResChunk pend[2] = {};

@@ -322,4 +322,217 @@ int rescue_device_piece(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda_dev_
     return BWACUDA_OK;
 }
 
+// ---------------------------------------------------------------- host buffers, gathered by the device
+
+namespace {
+
+constexpr int RG_THREADS = 128;
+// Jobs per chunk of the host route: while a chunk's kernels run, the next one is planned and
+// gathered on the other slot's stream.
+constexpr size_t RG_CHUNK = size_t(1) << 17;
+
+__device__ __forceinline__ void rescue_limits(const bwacuda_rescue_job &, bwacuda_dev_rescue_job &D)
+{
+    D.minsc = 0;
+    D.endsc = 0;
+}
+__device__ __forceinline__ void rescue_limits(const bwacuda_fwd_job &J, bwacuda_dev_rescue_job &D)
+{
+    D.minsc = J.minsc;
+    D.endsc = J.endsc;
+}
+
+// The only read of the caller's job array: every job is validated and surveyed, its reserve in the
+// sequence buffer and its tracker entries sized, and its fields left in its device descriptor (the
+// slice addresses in q_off / t_off; an invalid job empty).
+template <typename JobT>
+__global__ void __launch_bounds__(RG_THREADS) rescue_plan_kernel(const JobT *__restrict__ hjobs, uint32_t n, int max_sc,
+                                                                 uint64_t *__restrict__ sizes,
+                                                                 uint64_t *__restrict__ entries,
+                                                                 bwacuda_dev_rescue_job *__restrict__ djobs,
+                                                                 RescueStat *__restrict__ st)
+{
+    __shared__ uint32_t hist_s[RC_CLASSES];
+    if (threadIdx.x < RC_CLASSES) hist_s[threadIdx.x] = 0u;
+    __syncthreads();
+    SurveyAcc a;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const JobT J = hjobs[k];
+        const bool ok = J.qlen >= 0 && J.tlen >= 0 && (J.qlen == 0 || J.query != nullptr) &&
+                        (J.tlen == 0 || J.target != nullptr) && J.qlen <= 65000;
+        bwacuda_dev_rescue_job D;
+        D.q_off = reinterpret_cast<uint64_t>(J.query);
+        D.t_off = reinterpret_cast<uint64_t>(J.target);
+        D.qlen = ok ? J.qlen : 0;
+        D.tlen = ok ? J.tlen : 0;
+        rescue_limits(J, D);
+        djobs[k] = D;
+        sizes[k] = ok ? 16ull * (slice_words(J.query, J.qlen) + slice_words(J.target, J.tlen)) : 0u;
+        entries[k] = rescue_scratch_entries(D.tlen);
+        if (ok) a.job(J.qlen, J.tlen, max_sc, hist_s);
+        else a.bad = 1u;
+    }
+    a.flush(st, hist_s);
+}
+
+// A warp completes 32 jobs' descriptors and copies their slices (warp_gather_slices).
+__global__ void __launch_bounds__(RG_THREADS) rescue_gather_kernel(uint32_t n, const uint64_t *__restrict__ offs,
+                                                                   uint8_t *__restrict__ seq,
+                                                                   bwacuda_dev_rescue_job *__restrict__ djobs)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t k0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32u; k0 < n; k0 += gridDim.x * blockDim.x) {
+        const uint32_t k = k0 + lane;
+        uint64_t qa = 0, ta = 0, base = 0;
+        uint32_t qw = 0, tw = 0;
+        if (k < n) {
+            bwacuda_dev_rescue_job D = djobs[k];
+            base = offs[k];
+            qa = D.q_off;
+            ta = D.t_off;
+            qw = slice_words(reinterpret_cast<const uint8_t *>(qa), D.qlen);
+            tw = slice_words(reinterpret_cast<const uint8_t *>(ta), D.tlen);
+            D.q_off = base + (qa & 15);
+            D.t_off = base + 16ull * qw + (ta & 15);
+            djobs[k] = D;
+        }
+        warp_gather_slices(qa & ~15ull, ta & ~15ull, base, qw, tw, seq);
+    }
+}
+
+__global__ void __launch_bounds__(256) rescue_scatter_kernel(const uint32_t *__restrict__ src, size_t words,
+                                                             uint32_t *__restrict__ dst)
+{
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < words; i += (size_t)gridDim.x * blockDim.x)
+        dst[i] = src[i];
+}
+
+// One chunk on its slot's stream, up to the results in the caller's array.
+template <typename JobT>
+int rescue_host_chunk(bwacuda_ctx *c, int slot_i, const JobT *hj, size_t cn, const Scoring &sc, int minsc, int mode,
+                      int lanes, void *out, RescueStat *total)
+{
+    Slot &sl = c->slot[slot_i];
+    RescueWork &W = c->rescue->work[1 + slot_i];
+    cudaStream_t s = sl.stream;
+    cudaError_t e;
+    const uint32_t n = (uint32_t)cn;
+    const size_t osz = mode == 2 ? sizeof(bwacuda_fwd_result) : sizeof(bwacuda_rescue_result);
+    size_t tb = 0;
+    if ((e = cub::DeviceScan::ExclusiveSum(nullptr, tb, (const uint64_t *)nullptr, (uint64_t *)nullptr, (int)cn + 1)) !=
+        cudaSuccess)
+        return cuda_status(e);
+    const size_t n1 = cn + 1;
+    if ((e = W.stat.ensure(sizeof(RescueStat))) != cudaSuccess) return cuda_status(e);
+    if ((e = W.h_stat.ensure(sizeof(RescueStat) + 64)) != cudaSuccess) return cuda_status(e);
+    if ((e = sl.d_aux.ensure(n1 * 8 * 4 + tb + 64)) != cudaSuccess) return cuda_status(e);
+    if ((e = sl.d_jobs.ensure(cn * sizeof(bwacuda_dev_rescue_job))) != cudaSuccess) return cuda_status(e);
+    if ((e = sl.d_out.ensure(cn * osz)) != cudaSuccess) return cuda_status(e);
+    RescueStat *d_st = static_cast<RescueStat *>(W.stat.p);
+    uint64_t *sizes = static_cast<uint64_t *>(sl.d_aux.p), *entries = sizes + n1, *offs = entries + n1, *soff = offs + n1;
+    void *tmp = soff + n1;
+    bwacuda_dev_rescue_job *dj = static_cast<bwacuda_dev_rescue_job *>(sl.d_jobs.p);
+    if ((e = cudaMemsetAsync(d_st, 0, sizeof(RescueStat), s)) != cudaSuccess) return cuda_status(e);
+    if ((e = cudaMemsetAsync(sizes + cn, 0, 8, s)) != cudaSuccess) return cuda_status(e);
+    if ((e = cudaMemsetAsync(entries + cn, 0, 8, s)) != cudaSuccess) return cuda_status(e);
+    const uint32_t grid = (uint32_t)std::min<size_t>((cn + RG_THREADS - 1) / RG_THREADS, (size_t)c->nsm * 16);
+    rescue_plan_kernel<JobT><<<grid, RG_THREADS, 0, s>>>(hj, n, sc.max_sc, sizes, entries, dj, d_st);
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
+    if ((e = cub::DeviceScan::ExclusiveSum(tmp, tb, sizes, offs, (int)cn + 1, s)) != cudaSuccess) return cuda_status(e);
+    if ((e = cub::DeviceScan::ExclusiveSum(tmp, tb, entries, soff, (int)cn + 1, s)) != cudaSuccess) return cuda_status(e);
+    char *h = static_cast<char *>(W.h_stat.p);
+    uint64_t *h_tot = reinterpret_cast<uint64_t *>(h + sizeof(RescueStat));
+    if ((e = cudaMemcpyAsync(h, d_st, sizeof(RescueStat), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_status(e);
+    if ((e = cudaMemcpyAsync(h_tot, offs + cn, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_status(e);
+    if ((e = cudaMemcpyAsync(h_tot + 1, soff + cn, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_status(e);
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_status(e);
+    RescueStat st;
+    memcpy(&st, h, sizeof(st));
+    if (st.bad) return BWACUDA_EINVAL;
+    const int qcap = (st.qmax + 15) / 16 * 16 + 16;
+    if ((size_t)qcap > rescue_tpj_smem_limit_qcap(st.nwide > 0)) return BWACUDA_EUNSUPPORTED;
+    if ((e = sl.d_seq.ensure(h_tot[0] + 16)) != cudaSuccess) return cuda_status(e);
+    if ((e = sl.d_scratch.ensure(h_tot[1] * sizeof(uint2) + 16)) != cudaSuccess) return cuda_status(e);
+    rescue_gather_kernel<<<grid, RG_THREADS, 0, s>>>(n, offs, static_cast<uint8_t *>(sl.d_seq.p), dj);
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
+    RescueLaunch L;
+    L.seq = static_cast<const uint8_t *>(sl.d_seq.p);
+    L.jobs = dj;
+    L.order = nullptr;
+    L.count_ptr = nullptr;
+    L.n = cn;
+    L.sc = sc;
+    L.mode = mode;
+    L.lanes = lanes;
+    L.minsc = minsc;
+    L.qcap = qcap;
+    L.only_wide = 0;
+    L.scratch = static_cast<uint2 *>(sl.d_scratch.p);
+    L.scratch_off = soff;
+    L.out_aln = mode == 2 ? nullptr : static_cast<bwacuda_rescue_result *>(sl.d_out.p);
+    L.out_fwd = mode == 2 ? static_cast<bwacuda_fwd_result *>(sl.d_out.p) : nullptr;
+    L.err = reinterpret_cast<uint32_t *>(c->d_misc.p);
+    L.stream = s;
+    if ((e = rescue_launch_classes(c, W, st, L)) != cudaSuccess) return cuda_status(e);
+    if (st.nwide) {
+        L.only_wide = 1;
+        if ((e = rescue_tpj_launch(L, true)) != cudaSuccess) return cuda_status(e);
+        c->stats.kernel_launches += 1;
+    }
+    const size_t words = cn * (osz / 4);
+    rescue_scatter_kernel<<<(uint32_t)std::min<size_t>((words + 255) / 256, (size_t)c->nsm * 8), 256, 0, s>>>(
+        static_cast<const uint32_t *>(sl.d_out.p), words, static_cast<uint32_t *>(out));
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
+    c->stats.kernel_launches += 5;
+    total->not_u8 |= st.not_u8;
+    total->not_i16 |= st.not_i16;
+    total->cells += st.cells;
+    return cuda_status(cudaEventRecord(sl.done, s));
+}
+
+template <typename JobT>
+int rescue_batch_gather_t(bwacuda_ctx *c, const JobT *jobs, size_t n, const Scoring &sc, int minsc, int mode, int lanes,
+                          void *out, bool *u8ok, bool *i16ok, uint64_t *cells)
+{
+    if (!c->pageable_access) return BWACUDA_EUNSUPPORTED;
+    int rc = rescue_init(c);
+    if (rc) return rc;
+    const size_t osz = mode == 2 ? sizeof(bwacuda_fwd_result) : sizeof(bwacuda_rescue_result);
+    const size_t CH = std::min(c->chunk_jobs, RG_CHUNK);
+    RescueStat total{};
+    bool busy[2] = {false, false};
+    for (size_t c0 = 0, k = 0; c0 < n && rc == BWACUDA_OK; c0 += CH, ++k) {
+        const int si = (int)(k & 1);
+        if (busy[si]) {  // the slot's buffers are free once its last chunk's results are stored
+            const cudaError_t e = cudaEventSynchronize(c->slot[si].done);
+            if (e != cudaSuccess) { rc = cuda_status(e); break; }
+        }
+        const size_t cn = std::min(CH, n - c0);
+        rc = rescue_host_chunk<JobT>(c, si, jobs + c0, cn, sc, minsc, mode, lanes, static_cast<char *>(out) + c0 * osz,
+                                     &total);
+        busy[si] = true;
+    }
+    for (int si = 0; si < 2; ++si) {  // errors included: nothing is left running
+        const cudaError_t e = cudaStreamSynchronize(c->slot[si].stream);
+        if (!rc) rc = cuda_status(e);
+    }
+    *u8ok = !total.not_u8;
+    *i16ok = !total.not_i16;
+    *cells = total.cells;
+    return rc;
+}
+
+}  // namespace
+
+int rescue_batch_gather(bwacuda_ctx *c, const bwacuda_rescue_job *jobs, size_t n, const Scoring &sc, int minsc, int mode,
+                        int lanes, void *out, bool *u8ok, bool *i16ok, uint64_t *cells)
+{
+    return rescue_batch_gather_t(c, jobs, n, sc, minsc, mode, lanes, out, u8ok, i16ok, cells);
+}
+int rescue_batch_gather(bwacuda_ctx *c, const bwacuda_fwd_job *jobs, size_t n, const Scoring &sc, int minsc, int mode,
+                        int lanes, void *out, bool *u8ok, bool *i16ok, uint64_t *cells)
+{
+    return rescue_batch_gather_t(c, jobs, n, sc, minsc, mode, lanes, out, u8ok, i16ok, cells);
+}
+
 }  // namespace bwacuda

@@ -182,6 +182,13 @@ int rescue_device_piece(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda_dev_
                         const Scoring &sc, int minsc, int mode, int lanes, bwacuda_rescue_result *d_out,
                         cudaStream_t s);
 
+// Host-buffer rescue with the device gathering the caller's jobs and slices and storing the results
+// (devices that read pageable host memory); the reference's batch width tests and the cells come back.
+int rescue_batch_gather(bwacuda_ctx *c, const bwacuda_rescue_job *jobs, size_t n, const Scoring &sc, int minsc, int mode,
+                        int lanes, void *out, bool *u8ok, bool *i16ok, uint64_t *cells);
+int rescue_batch_gather(bwacuda_ctx *c, const bwacuda_fwd_job *jobs, size_t n, const Scoring &sc, int minsc, int mode,
+                        int lanes, void *out, bool *u8ok, bool *i16ok, uint64_t *cells);
+
 // retry.cu
 void retry_release(bwacuda_ctx *c);
 

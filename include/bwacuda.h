@@ -115,14 +115,15 @@ typedef struct bwacuda_ctx bwacuda_ctx;
 #define BWACUDA_OPT_RESCUE_KERNEL 5
 #define BWACUDA_RESCUE_AUTO 0
 #define BWACUDA_RESCUE_TPJ 1
-/* How host-buffer extension batches on the batched path reach the device.
+/* How host-buffer extension batches on the batched path, rescue batches and ksw_global2 batches
+ * reach the device.
  * DEVICE: GPU kernels read the caller's job array and sequence slices through
  * the host page tables (devices reporting cudaDevAttrPageableMemoryAccess, e.g.
  * Grace-Blackwell over NVLink-C2C) and write results straight into out[].
  * HOST: worker threads pack into pinned staging, then H2D/D2H copies.
  * AUTO (default): DEVICE where the device supports it, else HOST.  Asking for
  * DEVICE on a device without pageable access makes the calls fail with
- * BWACUDA_EUNSUPPORTED. */
+ * BWACUDA_EUNSUPPORTED (rescue batches are packed by the host there). */
 #define BWACUDA_OPT_HOST_GATHER 6
 #define BWACUDA_GATHER_AUTO 0
 #define BWACUDA_GATHER_HOST 1
