@@ -512,8 +512,8 @@ def long_query_jobs(B, m, seed):
 def long_query_config(B, ctx, st, stream, timed, world, m=20000, seed=7000):
     """ksw_extend2 on m queries of 2,000-10,000 bases (1% substitutions), tlen = qlen + 100,
     w = 100, device-resident: the group-per-job kernel at 8, 16 and 32 lanes per job on the plain
-    path (the long queries go straight to it) and on the batched path with the window kernel off,
-    then the batched path's default (the thread-per-job window kernel takes these jobs)."""
+    path (the long queries go straight to it) and on the batched path with the band kernel off,
+    then the batched path's default (the band kernel, whose groups split every row, takes these jobs)."""
     import torch
 
     js = long_query_jobs(B, m, seed)
@@ -547,8 +547,8 @@ def long_query_config(B, ctx, st, stream, timed, world, m=20000, seed=7000):
                         "w = 100, h0 20-60; queries too long for the full-row thread-per-job kernels",
             "value": rows[best]["value"], "unit": "GCUPS", "best": best, "runs": rows,
             "lanes_per_op": 2 if window else 1,
-            "kernel": ("ext_slide_kernel: one thread per job, 16-bit pair cells, the row in a window of the band "
-                       "sliding along the query" if window else
+            "kernel": ("ext_band_kernel: 8 lanes a job splitting every row, 16-bit pair cells, the row in a window of "
+                       "the band sliding along the query" if window else
                        "ext_long_kernel: one group of lanes per job, 32-bit lane arithmetic")}
 
 

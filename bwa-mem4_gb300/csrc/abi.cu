@@ -211,6 +211,7 @@ static int ctx_init(bwacuda_ctx *c)
     c->pageable_access = pageable != 0;
     if ((e = cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device)) != cudaSuccess) return cuda_status(e);
     if (c->nsm < 1) c->nsm = 1;
+    c->small_jobs = (size_t)c->nsm * EXT_SMALL_JOBS_PER_SM;
     if ((e = c->d_misc.ensure(4096)) != cudaSuccess) return cuda_status(e);
     if ((e = c->h_misc.ensure(4096)) != cudaSuccess) return cuda_status(e);
     if ((e = cudaMemset(c->d_misc.p, 0, 4096)) != cudaSuccess) return cuda_status(e);
@@ -322,6 +323,10 @@ extern "C" int bwacuda_set_option(bwacuda_ctx *c, int option, int64_t value)
     case BWACUDA_OPT_LONG_SLIDE:
         if (value < 0 || value > 2) return BWACUDA_EINVAL;
         return batched_set_long_slide(c, (int)value);
+    case BWACUDA_OPT_SMALL_BATCH:
+        if (value < 0 || value > ((int64_t)1 << 30)) return BWACUDA_EINVAL;
+        if (cudaSetDevice(c->device) != cudaSuccess) return BWACUDA_ECUDA;
+        return batched_set_small(c, (size_t)value);
     case BWACUDA_OPT_DEVICE_PIECE:
         if (value < 1 || value > ((int64_t)1 << 30)) return BWACUDA_EINVAL;
         c->dev_piece = (size_t)value;

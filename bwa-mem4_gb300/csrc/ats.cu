@@ -34,6 +34,7 @@
 
 #include <cub/device/device_scan.cuh>
 
+#include "ext_job.cuh"
 #include "kernels.h"
 #include "runtime.h"
 
@@ -57,7 +58,7 @@ constexpr int ATS_RESERVE_REGS = ATS_THREADS * 64;
 constexpr int ATS_RESERVE_THREADS = ATS_THREADS;
 constexpr int ATS_RING = 4;  // chunk buffers in flight
 
-__device__ __forceinline__ bool job_ok(const bwacuda_ext_job &J)
+__host__ __device__ __forceinline__ bool job_ok(const bwacuda_ext_job &J)
 {
     return J.qlen >= 0 && J.tlen >= 0 && J.h0 > 0 && (J.qlen == 0 || J.query != nullptr) &&
            (J.tlen == 0 || J.target != nullptr);
@@ -358,6 +359,39 @@ int ats_gather_ext(bwacuda_ctx *c, const bwacuda_ext_job *hj, size_t n, int w, D
     return BWACUDA_OK;
 }
 
+// The smallest calls: one kernel over the caller's own arrays (ext_band_direct_launch), no plan, no
+// gather, no sort -- 0.4-0.6 ms of launches and read-backs whatever the jobs.  The host checks the
+// job records (a few nanoseconds each); *taken = false leaves the call to the pipeline.
+static int extend_batch_direct(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, const BinRule &br,
+                               const ExtParams &P, int w, bwacuda_ext_result *out, bool *taken)
+{
+    *taken = false;
+    if (n > (size_t)c->nsm * EXT_DIRECT_JOBS_PER_SM || !batched_is_small(c, n, P) ||
+        !ext_pair_lanes_ok(P.sc.o_del, P.sc.e_del, P.sc.o_ins, P.sc.e_ins))
+        return BWACUDA_OK;
+    uint64_t bins[3] = {0, 0, 0};
+    for (size_t k = 0; k < n; ++k) {
+        const bwacuda_ext_job &J = jobs[k];
+        if (!job_ok(J)) return BWACUDA_OK;  // the pipeline reports it
+        if (!ext_band_direct_ok(J.qlen, J.tlen, J.h0, P.sc.max_sc)) return BWACUDA_OK;
+        bins[bin_label(br, J.qlen, J.tlen, J.h0)]++;
+    }
+    *taken = true;
+    cudaStream_t s = c->slot[0].stream;
+    const cudaError_t e = ext_band_direct_launch(jobs, (uint32_t)n, w, P, out, static_cast<uint32_t *>(c->d_misc.p),
+                                                 reinterpret_cast<unsigned long long *>((char *)c->d_misc.p + 8), s);
+    if (e != cudaSuccess) return cuda_status(e);
+    c->stats.kernel_launches += 1;
+    c->stats.ext_bin_u8 += bins[0];
+    c->stats.ext_bin_i16 += bins[1];
+    c->stats.ext_bin_i32 += bins[2];
+    uint64_t cells = 0;
+    const int rc = collect_device_status(c, s, &cells);
+    c->stats.ext_jobs += n;
+    c->stats.ext_cells += cells;
+    return rc;
+}
+
 // extend_batch with the device doing the gather; validated arguments, n > 0.
 int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int m, const int8_t *mat,
                      const ExtParams &P, int w, bwacuda_ext_result *out)
@@ -365,8 +399,11 @@ int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int 
     if (!c->pageable_access) return BWACUDA_EUNSUPPORTED;
     int rc = batched_prepare(c);
     if (rc) return rc;
-    if ((rc = ats_init(c)) != BWACUDA_OK) return rc;
     const BinRule br = bin_rule(m, mat);
+    bool taken = false;
+    rc = extend_batch_direct(c, jobs, n, br, P, w, out, &taken);
+    if (rc || taken) return rc;
+    if ((rc = ats_init(c)) != BWACUDA_OK) return rc;
     const size_t CH = std::min(c->chunk_jobs, ATS_MAX_CHUNK);
     uint32_t input_flags = 0;
     // chunks ramp up from 64k jobs, doubling: the extension starts after a short gather, and each

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstdint>
 #include <cstring>
 #include <vector>
 
@@ -16,6 +17,9 @@
 namespace bwacuda {
 
 constexpr int FAN = 4;  // bucket streams
+// Open-ended buckets: jobs per SM from which the band kernel gives a job 8 lanes, below it 32 (queries
+// of 2-10 kb on 152 SMs: 1,000 jobs 9.6 / 6.5 ms, 2,400 jobs 9.8 / 9.8, 20,000 jobs 23.1 / 42.4).
+constexpr int BAND_LANES8_JOBS = 14;
 
 // Device work buffers of one in-flight batch.
 struct BatchBufs {
@@ -192,6 +196,18 @@ int batched_set_long_slide(bwacuda_ctx *c, int mode)
     return BWACUDA_OK;
 }
 
+// Largest call that runs as a small batch; a new value invalidates captured graphs.
+int batched_set_small(bwacuda_ctx *c, size_t jobs)
+{
+    int rc = batched_init(c);
+    if (rc) return rc;
+    if (c->small_jobs != jobs) {
+        c->small_jobs = jobs;
+        c->batched->gen++;
+    }
+    return BWACUDA_OK;
+}
+
 void batched_get_tuning(bwacuda_ctx *c, int *tb, int *grab, int *step)
 {
     BatchedState *B = c->batched;
@@ -211,6 +227,66 @@ static cudaError_t ensure_bufs(BatchBufs &bb, size_t n)
     return bb.tmp.ensure(ext_sort_temp_bytes(n) + 256);
 }
 
+// Whether a call of n jobs runs as a small batch (the ungapped rule is part of the sorted path).
+bool batched_is_small(const bwacuda_ctx *c, size_t n, const ExtParams &P)
+{
+    return n <= c->small_jobs && !P.ug.enabled;
+}
+
+// A small batch: no buckets, the band kernel over every job and the
+// group-per-job kernels for what it leaves (32-bit values, queries and bands past its window).
+// Thread-per-job buckets take 0.3-0.5 ms however few jobs they hold.  32 lanes a job below 8 jobs
+// per SM, 16 below 20, else 8 (the times stand at EXT_SMALL_JOBS_PER_SM); with 8 the jobs are sorted
+// first, longest first: the four jobs of a warp step to its longest, and 20,000 queries of 2-10 kb in
+// caller order took 32.4 ms against 23.1.
+static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d_seq,
+                                 const bwacuda_dev_ext_job *d_jobs, size_t n, const ExtParams &P,
+                                 bwacuda_ext_result *d_out, cudaStream_t s, uint32_t *err, unsigned long long *cells)
+{
+    BatchedState *B = c->batched;
+    uint32_t *work = static_cast<uint32_t *>(bb.xl.p);
+    cudaError_t e = cudaMemsetAsync(work, 0, XL_WORK_WORDS * 4, s);
+    if (e != cudaSuccess) return e;
+    ExtLongLaunch X;
+    X.seq = d_seq;
+    X.jobs = d_jobs;
+    X.order = nullptr;
+    X.bounds = nullptr;
+    X.njobs = (uint32_t)n;
+    X.min_qlen = 0;
+    X.lanes = c->long_lanes;
+    X.ring_cols = XL_RING_DEFAULT;
+    X.P = P;
+    X.out = d_out;
+    X.err = err ? err : reinterpret_cast<uint32_t *>(c->d_misc.p);
+    X.cells = cells ? cells : reinterpret_cast<unsigned long long *>((char *)c->d_misc.p + 8);
+    X.defer = work + XL_WORK_WORDS;
+    X.defer_count = work + XL_WORK_DCOUNT;
+    X.band = 1;
+    X.reserve_regs = bb.reserve_regs;
+    X.reserve_threads = bb.reserve_threads;
+    X.sm_regs = B->sm_regs;
+    X.sm_threads = B->sm_threads;
+    X.stream = s;
+    const int lanes = n < (size_t)B->nsm * 8 ? 32 : (n < (size_t)B->nsm * 20 ? 16 : 8);
+    if (lanes == 8) {
+        uint32_t *order = static_cast<uint32_t *>(bb.idx_out.p);
+        if ((e = ext_sort_jobs(d_jobs, n, P.sc.max_sc, 1u, d_seq, P.ug, P.zdrop, d_out,
+                               static_cast<uint16_t *>(bb.keys_in.p), static_cast<uint16_t *>(bb.keys_out.p),
+                               static_cast<uint32_t *>(bb.idx_in.p), order, bb.tmp.p, bb.tmp.cap, s)) != cudaSuccess)
+            return e;
+        X.order = order;
+    }
+    if ((e = ext_band_launch(X, lanes, work + XL_WORK_BAND, 0u, UINT32_MAX, B->nsm)) != cudaSuccess) return e;
+    for (int w32 = 0; w32 < 2; ++w32) {
+        X.counter = work + (w32 ? XL_WORK_COUNTER32 : XL_WORK_COUNTER16);
+        if ((e = ext_long_launch(X, w32 != 0, B->nsm)) != cudaSuccess) return e;
+    }
+    for (int w32 = 0; w32 < 2; ++w32)
+        if ((e = ext_long_deferred_launch(X, w32 != 0, work, B->nsm)) != cudaSuccess) return e;
+    return cudaSuccess;
+}
+
 // Enqueue the batched sequence for n device-resident jobs on stream s.
 static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d_seq,
                                    const bwacuda_dev_ext_job *d_jobs, size_t n, const ExtParams &P,
@@ -219,6 +295,7 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
 {
     BatchedState *B = c->batched;
     const bool lanes = ext_pair_lanes_ok(P.sc.o_del, P.sc.e_del, P.sc.o_ins, P.sc.e_ins);
+    if (lanes && batched_is_small(c, n, P)) return enqueue_small(c, bb, d_seq, d_jobs, n, P, d_out, s, err, cells);
     cudaError_t e = ext_sort_and_bucket(d_jobs, n, P.sc.max_sc, lanes, d_seq, P.ug, P.zdrop, d_out,
                                         static_cast<uint16_t *>(bb.keys_in.p),
                                         static_cast<uint16_t *>(bb.keys_out.p), static_cast<uint32_t *>(bb.idx_in.p),
@@ -253,20 +330,23 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
     X.sm_regs = B->sm_regs;
     X.sm_threads = B->sm_threads;
     X.stream = bb.fan[0];
-    // the open-ended buckets of the 8- and 16-bit classes run the thread-per-job window kernel
-    // first (bands up to bwa-mem's default 100; wider ones stay with the group kernel), on
-    // buckets of at least a warp of jobs per SM unless BWACUDA_OPT_LONG_SLIDE forces it
-    const int slide_wc = c->long_slide && lanes ? ext_slide_window_for_band(100) : 0;
-    X.slide_min = c->long_slide == 2 ? 0u : (uint32_t)B->nsm * 32u;
+    // the open-ended buckets of the 8- and 16-bit classes run the band kernel (bands up to
+    // bwa-mem's default 100 and a column; wider ones stay with the group kernel): 8 lanes a job
+    // from BAND_LANES8_JOBS jobs per SM on (BWACUDA_OPT_LONG_SLIDE 2: always), 32 below
+    const bool use_band = c->long_slide && lanes;
+    const uint32_t cut = c->long_slide == 2 ? 0u : (uint32_t)(B->nsm * BAND_LANES8_JOBS);
     bool long16 = false, long32 = false;
     for (int b = B->nb - 1; b >= 0; --b) {
         if (B->defs[b].kernel != 1) continue;
         uint32_t *tab = static_cast<uint32_t *>(bb.table.p) + 4 * b;
         X.bounds = tab;
         X.counter = tab + 2;
-        X.slide_counter = tab + 3;
-        X.slide_wc = B->defs[b].qhi == EXT_QHI_OPEN ? slide_wc : 0;
         const bool w32 = B->defs[b].cls == 2;
+        X.band = use_band && !w32 && B->defs[b].qhi == EXT_QHI_OPEN;
+        if (X.band) {  // one of the two runs the bucket, the other exits at once
+            if ((e = ext_band_launch(X, 8, tab + 3, cut, UINT32_MAX, B->nsm)) != cudaSuccess) return e;
+            if (cut && (e = ext_band_launch(X, 32, tab + 3, 1u, cut, B->nsm)) != cudaSuccess) return e;
+        }
         if ((e = ext_long_launch(X, w32, B->nsm)) != cudaSuccess) return e;
         long16 |= !w32;
         long32 |= w32;

@@ -44,9 +44,11 @@ cudaError_t launch_first(const ExtLongLaunch &X, int nsm)
         const int cap_t = (X.sm_threads - X.reserve_threads) / XL_BLOCK;
         per_sm = std::max(1, std::min(per_sm, std::min(cap_r, cap_t)));
     }
-    kern<<<per_sm * nsm, XL_BLOCK, smem, X.stream>>>(X.seq, X.jobs, X.order, X.bounds, X.counter, X.njobs,
-                                                    X.min_qlen, ring, X.defer, X.defer_count, W32 ? 0 : X.slide_wc,
-                                                    X.slide_min, X.P, X.out, X.err, X.cells);
+    const size_t most = ((size_t)X.njobs * L + XL_BLOCK - 1) / XL_BLOCK;
+    const uint32_t grid = (uint32_t)std::min<size_t>((size_t)per_sm * nsm, std::max<size_t>(most, 1));
+    kern<<<grid, XL_BLOCK, smem, X.stream>>>(X.seq, X.jobs, X.order, X.bounds, X.counter, X.njobs, X.min_qlen, ring,
+                                            X.defer, X.defer_count, W32 ? 0 : X.band, X.P, X.out, X.err,
+                                            X.cells);
     return cudaGetLastError();
 }
 
@@ -69,8 +71,9 @@ cudaError_t launch_deferred(const ExtLongLaunch &X, const uint32_t *dbounds, uin
     int per_sm = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, smem)) != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidValue;
-    kern<<<per_sm * nsm, 32, smem, X.stream>>>(X.seq, X.jobs, X.defer, dbounds, dcounter, X.njobs, 0, R, nullptr,
-                                              nullptr, 0, 0u, X.P, X.out, X.err, X.cells);
+    const uint32_t grid = (uint32_t)std::min<size_t>((size_t)per_sm * nsm, std::max<size_t>(X.njobs, 1));
+    kern<<<grid, 32, smem, X.stream>>>(X.seq, X.jobs, X.defer, dbounds, dcounter, X.njobs, 0, R, nullptr, nullptr, 0,
+                                      X.P, X.out, X.err, X.cells);
     return cudaGetLastError();
 }
 
@@ -78,14 +81,7 @@ cudaError_t launch_deferred(const ExtLongLaunch &X, const uint32_t *dbounds, uin
 
 cudaError_t ext_long_launch(const ExtLongLaunch &X, bool w32, int nsm)
 {
-    if (w32) return launch_first_lanes<true>(X, nsm);
-    // the window kernel first (it exits at once when the bucket is below slide_min jobs); the
-    // group kernel then runs the jobs it left
-    if (X.slide_wc > 0) {
-        const cudaError_t e = ext_slide_launch(X, nsm);
-        if (e != cudaSuccess) return e;
-    }
-    return launch_first_lanes<false>(X, nsm);
+    return w32 ? launch_first_lanes<true>(X, nsm) : launch_first_lanes<false>(X, nsm);
 }
 
 cudaError_t ext_long_deferred_launch(const ExtLongLaunch &X, bool w32, uint32_t *work, int nsm)

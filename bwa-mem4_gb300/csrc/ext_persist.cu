@@ -133,7 +133,7 @@ __global__ void ext_bucket_bounds_kernel(const uint16_t *__restrict__ keys, uint
     table[b * 4 + 0] = lower_bound16(keys, n, key_lo);
     table[b * 4 + 1] = lower_bound16(keys, n, key_hi + 1);
     table[b * 4 + 2] = 0;  // work counter
-    table[b * 4 + 3] = 0;  // work counter of the window kernel (open-ended buckets)
+    table[b * 4 + 3] = 0;  // work counter of the band kernel (open-ended buckets)
 }
 
 }  // namespace
@@ -201,6 +201,20 @@ size_t ext_sort_temp_bytes(size_t n)
     return bytes;
 }
 
+// Keys and their sort: idx_out holds the job indices by key.  min_cls 1 sorts the 8- and 16-bit
+// classes as one.
+cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, uint32_t min_cls, const uint8_t *seq,
+                          const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint16_t *keys_in,
+                          uint16_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp, size_t tmp_bytes,
+                          cudaStream_t s)
+{
+    if (n == 0) return cudaSuccess;
+    uint32_t grid = (uint32_t)((n + 255) / 256);
+    if (grid > 8192) grid = 8192;
+    ext_keys_kernel<<<grid, 256, 0, s>>>(jobs, (uint32_t)n, max_sc, min_cls, seq, ug, zdrop, out, keys_in, idx_in);
+    return cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys_in, keys_out, idx_in, idx_out, (int)n, 0, 16, s);
+}
+
 cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, bool pair_lanes,
                                 const uint8_t *seq, const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint16_t *keys_in,
                                 uint16_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp,
@@ -208,12 +222,8 @@ cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int m
                                 cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    uint32_t grid = (uint32_t)((n + 255) / 256);
-    if (grid > 8192) grid = 8192;
-    ext_keys_kernel<<<grid, 256, 0, s>>>(jobs, (uint32_t)n, max_sc, pair_lanes ? 0u : 1u, seq, ug, zdrop, out,
-                                         keys_in, idx_in);
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys_in, keys_out, idx_in, idx_out, (int)n, 0,
-                                                    16, s);
+    const cudaError_t e = ext_sort_jobs(jobs, n, max_sc, pair_lanes ? 0u : 1u, seq, ug, zdrop, out, keys_in, keys_out,
+                                        idx_in, idx_out, tmp, tmp_bytes, s);
     if (e != cudaSuccess) return e;
     ext_bucket_bounds_kernel<<<1, EXT_MAX_BUCKETS, 0, s>>>(keys_out, (uint32_t)n, d_defs, nb, d_table);
     return cudaGetLastError();

@@ -41,6 +41,7 @@ size_t ext_tpj_smem_limit_qcap(bool wide);
 constexpr int XL_WORK_DCOUNT = 1;                              // [0] stays 0, [1] deferred jobs
 constexpr int XL_WORK_DCOUNTER16 = 2, XL_WORK_DCOUNTER32 = 3;  // work counters of the deferred launches
 constexpr int XL_WORK_COUNTER16 = 4, XL_WORK_COUNTER32 = 5;    // work counters of unbucketed first launches
+constexpr int XL_WORK_BAND = 6;                                // work counter of a small batch's band launch
 constexpr int XL_WORK_WORDS = 8;
 constexpr int XL_RING_MIN = 256, XL_RING_FIRST_MAX = 4096;
 constexpr int XL_RING_DEFAULT = 512;  // first-launch ring when the bands are not known on the host
@@ -61,21 +62,34 @@ struct ExtLongLaunch {
     unsigned long long *cells;
     uint32_t *defer;         // njobs entries: jobs set aside for the deferred launch
     uint32_t *defer_count;   // work + XL_WORK_DCOUNT
-    // thread-per-job window kernel (ext_slide.cu) ahead of the group kernel on 16-bit jobs:
-    // window columns (0: off), the fewest jobs [start, stop) must hold for it to run, and its
-    // zeroed work counter
-    int slide_wc = 0;
-    uint32_t slide_min = 0;
-    uint32_t *slide_counter = nullptr;
+    int band = 0;  // 1: the band kernel runs beside this launch, which leaves it the jobs of band_takes
     int reserve_regs = 0, reserve_threads = 0, sm_regs = 65536, sm_threads = 2048;
     cudaStream_t stream;
 };
 
 cudaError_t ext_long_launch(const ExtLongLaunch &X, bool w32, int nsm);
-// The window kernel alone (ext_long_launch runs it ahead of the group kernel when slide_wc > 0).
-cudaError_t ext_slide_launch(const ExtLongLaunch &X, int nsm);
-// Window columns for clamped bands up to w.
-int ext_slide_window_for_band(int w);
+// Batched calls of up to this many jobs per SM run unsorted in the band kernel, and host calls of up
+// to this many straight from the caller's arrays.  Device-resident calls on 152 SMs, microseconds
+// (read pairs / mixed lengths):
+//   jobs       sorted buckets   8 lanes (sorted)  16        32 lanes a job
+//   1,024       521 / 1369                    188 / 337      166 / 267
+//   2,048       551 / 1680                    201 / 347      203 / 303
+//   8,192       732 / 1747      330 / 531     379 / 494      394 / 485
+//   16,384      768 / 1795      402 / 630     610 / 719      620 / 682
+//   32,768      784 / 1948      510 / 668    1061 / 1130    1088 / 1126
+//   65,536      812 / 1972      847 / 910    1966 / 2015    2017 / 2039
+//   131,072     907 / 2130     1597 / 1595
+constexpr int EXT_SMALL_JOBS_PER_SM = 350;
+constexpr int EXT_DIRECT_JOBS_PER_SM = 24;
+// The band kernel (ext_band.cuh) with 8, 16 or 32 lanes a job over X's jobs that band_takes admits,
+// when [start, stop) holds count_lo or more and fewer than count_hi; counter: a zeroed device word.
+cudaError_t ext_band_launch(const ExtLongLaunch &X, int lanes, uint32_t *counter, uint32_t count_lo, uint32_t count_hi,
+                            int nsm);
+// A warp per job of a host job array the device reads in place; every job passed ext_band_direct_ok
+// (and has non-negative lengths and valid slices).
+bool ext_band_direct_ok(int qlen, int tlen, int h0, int max_sc);
+cudaError_t ext_band_direct_launch(const bwacuda_ext_job *hjobs, uint32_t n, int w, const ExtParams &P,
+                                   bwacuda_ext_result *hout, uint32_t *err, unsigned long long *cells, cudaStream_t s);
 cudaError_t ext_long_deferred_launch(const ExtLongLaunch &X, bool w32, uint32_t *work, int nsm);
 // First-launch ring for bands up to w (XL_RING_MIN .. XL_RING_FIRST_MAX columns).
 int ext_long_ring_for_band(int w);

@@ -98,7 +98,8 @@ struct bwacuda_ctx {
     int rescue_pair = -1;  // lanes of a group holding two byte-range jobs (rescue_wf2.cuh): 4, 8, 16; 0 off; -1: not set
     bool ungapped = false;  // ungapped-diagonal fast path on the batched extension path
     int long_lanes = 16;    // lanes per job of the group-per-job extension kernel (8, 16, 32)
-    int long_slide = 1;     // thread-per-job window kernel on the open-ended buckets: 0 off, 1 auto, 2 always
+    int long_slide = 1;     // band kernel on the open-ended buckets: 0 off, 1 lanes by the bucket's jobs, 2 always 8 lanes
+    size_t small_jobs = 0;  // batched calls of up to this many jobs run unsorted in the band kernel (set from the SM count)
     int tune_candidates = 0;        // last autotune call
     double tuned_ext_gcups = 0.0;   // best candidates' rates on their samples
     double tuned_rescue_gcups = 0.0;
@@ -154,6 +155,7 @@ int batched_set_long(bwacuda_ctx *c, int long_qlo);
 int batched_get_long(bwacuda_ctx *c);
 int batched_set_long_lanes(bwacuda_ctx *c, int lanes);
 int batched_set_long_slide(bwacuda_ctx *c, int mode);
+int batched_set_small(bwacuda_ctx *c, size_t jobs);
 
 struct BatchBufs;
 int batched_prepare(bwacuda_ctx *c);
@@ -167,6 +169,7 @@ cudaError_t batched_reserve(BatchBufs *bb, size_t n);
 // registers / threads per SM that bb's bucket kernels leave free (0, 0: none)
 void batched_set_reserve(BatchBufs *bb, int regs, int threads);
 int batched_nsm(bwacuda_ctx *c);
+bool batched_is_small(const bwacuda_ctx *c, size_t n, const ExtParams &P);
 int batched_bucket_count(bwacuda_ctx *c);
 
 // ats.cu

@@ -161,12 +161,17 @@ typedef struct bwacuda_ctx bwacuda_ctx;
  * picks one by its number of jobs.  Results never depend on it. */
 #define BWACUDA_OPT_RESCUE_PAIR 14
 /* Batched extension, the open-ended query-length buckets (queries too long for a thread's
- * shared-memory row): 1 (default) = a thread-per-job kernel holding each job's row in a window
- * of the band that slides along the query runs the jobs of bands up to 101 columns when the
- * bucket holds at least 32 jobs per SM, the group-per-job kernel the rest; 2 = the window
- * kernel whatever the bucket's size; 0 = the group-per-job kernel only.  Results never depend
- * on it. */
+ * shared-memory row): 1 (default) = a kernel whose groups of lanes split every row, the row held in
+ * a window of the band that slides along the query, runs the jobs of bands up to 101 columns (8
+ * lanes a job where the bucket fills the GPU, 32 where it does not), the group-per-job kernel the
+ * rest; 2 = 8 lanes whatever the bucket's size; 0 = the group-per-job kernel only.  Results never
+ * depend on it. */
 #define BWACUDA_OPT_LONG_SLIDE 15
+/* Batched extension: calls of up to this many jobs run without length buckets, a group of 8, 16 or
+ * 32 lanes per job splitting every row (a thread per job would leave most of the GPU idle).  Default:
+ * 350 jobs per SM; 0 = every call sorted into length buckets.  Calls with BWACUDA_OPT_UNGAPPED on
+ * are always sorted.  Results never depend on it. */
+#define BWACUDA_OPT_SMALL_BATCH 16
 
 int bwacuda_ctx_create(int device, bwacuda_ctx **out);
 void bwacuda_ctx_destroy(bwacuda_ctx *ctx);
