@@ -26,6 +26,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
+#include "global_tag.cuh"
 #include "kernels.h"
 #include "runtime.h"
 
@@ -66,6 +67,7 @@ constexpr int GLB_NEG16 = -24576;
 // what a DP kernel leaves in ncig[k] for the traceback kernel: the direction-byte layout
 constexpr int GLB_TB_ROWS = -1;   // a row's bytes from column beg (32-bit cell kernel)
 constexpr int GLB_TB_PAIRS = -2;  // from column beg & ~1 (pair kernel)
+constexpr int GLB_TB_TAGGED = -3; // the tagged kernel's nibbles (global_tag.cuh), its own traceback kernel
 constexpr int GLB_TB_AHEAD = 4;     // traceback cells loaded together down the diagonal
 constexpr int GLB_SIDE_STREAMS = 2;  // streams beside the context's for the bucket DP launches
 constexpr int GLB_NARROW_D = 8000;
@@ -95,6 +97,10 @@ __host__ __device__ inline int global_bucket(int qlen)
     return qlen <= 64 ? 0 : qlen <= 128 ? 1 : qlen <= 192 ? 2 : qlen <= 256 ? 3 : qlen <= 320 ? 4 : qlen <= 448 ? 5
            : qlen <= 640 ? 6 : 7;
 }
+
+// Launch classes of the device route: the length buckets of the tagged kernel (global_tag.cuh), then
+// those of the alignments it does not take.
+constexpr int GLB_NCLASSES = 2 * GLB_NBUCKETS;
 
 // Band slots a job needs.
 __host__ __device__ inline int global_band_slots(int qlen, int w)
@@ -727,14 +733,15 @@ __device__ __forceinline__ bool gjob_ok(const bwacuda_global_job &J)
 // bucket.  flags[0]: input error bits.  bstat[2b], bstat[2b+1]: bucket b's max
 // band slots and max query length.
 __global__ void glb_plan_kernel(const bwacuda_global_job *__restrict__ hj, uint32_t n, int qlim,
-                                GlbNarrowRule nr, uint64_t *__restrict__ seq_sz, uint64_t *__restrict__ cig_sz,
+                                GlbNarrowRule nr, gtag::TagRule tr, uint64_t *__restrict__ seq_sz, uint64_t *__restrict__ cig_sz,
                                 uint64_t *__restrict__ z_sz, uint32_t *__restrict__ keys, uint32_t *__restrict__ idx,
-                                uint32_t *__restrict__ flags, uint32_t *__restrict__ bstat, uint32_t *__restrict__ bwide)
+                                uint32_t *__restrict__ flags, uint32_t *__restrict__ bstat, uint32_t *__restrict__ bwide,
+                                int4 *__restrict__ dims)
 {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t k0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); k0 < n; k0 += stride) {
         const uint32_t k = k0 + (threadIdx.x & 31u);
-        int ql = 0, tl = 0, bs = 0, bucket = 0;
+        int ql = 0, tl = 0, bs = 0, bl = 0, bucket = 0;
         bool bad = false, wide = false;
         if (k < n) {
             const bwacuda_global_job J = hj[k];
@@ -744,13 +751,20 @@ __global__ void glb_plan_kernel(const bwacuda_global_job *__restrict__ hj, uint3
             tl = ok ? J.tlen : 0;
             seq_sz[k] = ok ? 16ull * (slice_words(J.query, ql) + slice_words(J.target, tl)) : 0u;
             cig_sz[k] = (uint64_t)ql + (uint64_t)tl + 1u;
-            z_sz[k] = (uint64_t)tl * (uint64_t)global_zrow(ql, J.w);
-            bs = global_band_slots(ql, J.w);
-            bucket = global_bucket(ql);
-            wide = !global_narrow(ql, tl, nr);
+            const bool tag = gtag::tag_ok(ql, tl, J.w, tr);
+            dims[k] = make_int4(ql, tl, J.w, 0);
+            z_sz[k] = tag ? 0u : (uint64_t)tl * (uint64_t)global_zrow(ql, J.w);
+            // the class's largest band: right and left of the diagonal (tagged), or slots (the others)
+            bs = tag ? gtag::band_right(J.w, ql) : global_band_slots(ql, J.w);
+            bl = tag ? gtag::band_left(J.w, tl) : 0;
+            bucket = global_bucket(ql) + (tag ? 0 : GLB_NBUCKETS);
+            wide = !tag && !global_narrow(ql, tl, nr);
+            // alignments of one band, then of one length, side by side: neighbours share a thread of
+            // the tagged kernel when their bands agree
             const uint32_t qk = ql > 1023 ? 0u : 1023u - (uint32_t)ql;
-            const uint32_t tk = tl > 4095 ? 0u : 4095u - (uint32_t)tl;
-            keys[k] = ((uint32_t)bucket << 22) | (qk << 12) | tk;
+            const uint32_t wk = J.w > 127 ? 127u : (J.w > 0 ? (uint32_t)J.w : 0u);
+            const uint32_t tk = tl > 2047 ? 0u : 2047u - (uint32_t)tl;
+            keys[k] = ((uint32_t)bucket << 28) | (qk << 18) | (wk << 11) | tk;
             idx[k] = k;
         }
         const unsigned live = __ballot_sync(0xffffffffu, k < n);
@@ -760,11 +774,14 @@ __global__ void glb_plan_kernel(const bwacuda_global_job *__restrict__ hj, uint3
         if (k < n) {
             const unsigned bmax = __reduce_max_sync(grp, (unsigned)bs);
             const unsigned qmax = __reduce_max_sync(grp, (unsigned)ql);
+            const unsigned lmax = __reduce_max_sync(grp, (unsigned)bl);
             const unsigned anyw = __reduce_or_sync(grp, wide ? 1u : 0u);
             if ((int)(threadIdx.x & 31u) == __ffs(grp) - 1) {
                 atomicMax(bstat + 2 * bucket, bmax);
                 atomicMax(bstat + 2 * bucket + 1, qmax);
-                if (anyw) atomicOr(bwide + bucket, 1u);
+                // other classes: a job too wide for 16-bit cells; tagged ones: the widest left band
+                if (bucket >= GLB_NBUCKETS) { if (anyw) atomicOr(bwide + bucket, 1u); }
+                else atomicMax(bwide + bucket, lmax);
             }
         }
     }
@@ -774,16 +791,167 @@ __global__ void glb_plan_kernel(const bwacuda_global_job *__restrict__ hj, uint3
 __global__ void glb_bucket_bounds_kernel(const uint32_t *__restrict__ keys, uint32_t n, uint32_t *__restrict__ bounds)
 {
     const int b = threadIdx.x;
-    if (b >= GLB_NBUCKETS) return;
+    if (b >= GLB_NCLASSES) return;
     for (int side = 0; side < 2; ++side) {
-        const uint32_t v = (uint32_t)(b + side) << 22;
+        const uint64_t v = (uint64_t)(b + side) << 28;
         uint32_t lo = 0, hi = n;
         while (lo < hi) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (keys[mid] < v) lo = mid + 1;
+            if ((uint64_t)keys[mid] < v) lo = mid + 1;
             else hi = mid;
         }
         bounds[2 * b + side] = lo;
+    }
+}
+
+// The tagged kernel's warp groups: bucket after bucket, 64 sorted alignments a group (the last of a
+// bucket shorter); a warp works out each group's rows and steps and the bytes of its directions
+// (sizes[0 .. ngroups_max]; groups past the last one take none).
+__global__ void glb_warp_groups_kernel(const int4 *__restrict__ dims, const uint32_t *__restrict__ order, const uint32_t *__restrict__ bounds,
+                                       gtag::TagRule tr, uint32_t ngroups_max, gtag::WarpGroup *__restrict__ groups,
+                                       uint64_t *__restrict__ sizes)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w <= ngroups_max; w += (gridDim.x * blockDim.x) >> 5) {
+        uint32_t left = w, pos = 0, count = 0;
+        for (int b = 0; b < GLB_NBUCKETS; ++b) {
+            const uint32_t c = bounds[2 * b + 1] - bounds[2 * b], ng = (c + 63u) / 64u;
+            if (left < ng) {
+                pos = bounds[2 * b] + 64u * left;
+                count = min(64u, c - 64u * left);
+                break;
+            }
+            left -= ng;
+        }
+        unsigned rows = 0, ng = 0;
+        if (2 * lane < count) {
+            const int4 A = dims[order[pos + 2 * lane]];  // qlen, tlen, w
+            const bool has1 = 2 * lane + 1 < count;
+            const int4 B = has1 ? dims[order[pos + 2 * lane + 1]] : A;
+            const gtag::PairGeo g = gtag::pair_geo(A.x, A.y, A.z, has1, B.x, B.y, B.z, tr);
+            rows = (unsigned)g.t;
+            ng = (unsigned)gtag::groups(g.wl, g.wr);
+            if (!g.dual && has1) {
+                const gtag::PairGeo h = gtag::pair_geo(B.x, B.y, B.z, false, B.x, B.y, B.z, tr);
+                rows = max(rows, (unsigned)h.t);
+                ng = max(ng, (unsigned)gtag::groups(h.wl, h.wr));
+            }
+        }
+        rows = __reduce_max_sync(0xffffffffu, rows);
+        ng = __reduce_max_sync(0xffffffffu, ng);
+        if (lane == 0) {
+            sizes[w] = (uint64_t)((rows + 1u) / 2u) * ng * 512u;
+            if (w < ngroups_max) {
+                gtag::WarpGroup g;
+                g.z_off = 0;
+                g.pos = pos;
+                g.count = (uint16_t)count;
+                g.ng = (uint16_t)ng;
+                groups[w] = g;
+            }
+        }
+    }
+}
+
+// The groups' offsets, once scanned.
+__global__ void glb_group_offsets_kernel(const uint64_t *__restrict__ offs, uint32_t ngroups,
+                                         gtag::WarpGroup *__restrict__ groups)
+{
+    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < ngroups; w += gridDim.x * blockDim.x)
+        groups[w].z_off = offs[w];
+}
+
+// Traceback over the tagged kernel's directions (sw.rs:700-738): warps 2w and 2w + 1 walk group w's
+// first and second alignments of the pairs, lane for lane as the DP's threads lay, so a warp's loads
+// fall into the same 512-byte rows.  In state M the walk usually stays on the diagonal, which keeps its
+// step group: four row pairs (eight rows) of it are loaded together.
+__global__ void __launch_bounds__(256) glb_tag_traceback_kernel(const GlobalDevJob *__restrict__ jobs,
+                                                                const uint32_t *__restrict__ order,
+                                                                const gtag::WarpGroup *__restrict__ groups,
+                                                                uint32_t ngroups, gtag::TagRule tr,
+                                                                const uint8_t *__restrict__ z,
+                                                                uint32_t *__restrict__ cig, int32_t *__restrict__ ncig)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t x = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < 2 * ngroups; x += (gridDim.x * blockDim.x) >> 5) {
+        const gtag::WarpGroup wg = groups[x >> 1];
+        const uint32_t half = x & 1u, at = 2 * lane + half;
+        if (at >= wg.count) continue;
+        const uint32_t k = order[wg.pos + at];
+        if (ncig[k] != GLB_TB_TAGGED) continue;
+        const GlobalDevJob J = jobs[k];
+        int wl = gtag::band_left(J.w, J.tlen);
+        if ((at ^ 1u) < wg.count) {  // the pass's left band is the pair's
+            const GlobalDevJob O = jobs[order[wg.pos + (at ^ 1u)]];
+            const gtag::PairGeo g = gtag::pair_geo(J.qlen, J.tlen, J.w, true, O.qlen, O.tlen, O.w, tr);
+            if (g.dual) wl = g.wl;
+        }
+        const uint32_t *zw = reinterpret_cast<const uint32_t *>(z + wg.z_off) + lane * 4u + half;
+        const size_t prow = (size_t)wg.ng * 128u;  // words of a row pair
+        uint32_t *cg = cig + J.cig_off;
+        int nc = 0, i = J.tlen - 1, j = J.qlen - 1;
+        uint32_t run_op = 4u, run = 0u;  // the open CIGAR run
+        auto push = [&](uint32_t op, uint32_t len) {
+            if (op == run_op) {
+                run += len;
+                return;
+            }
+            if (run) cg[nc++] = (run << 4) | run_op;
+            run_op = op;
+            run = len;
+        };
+        uint32_t which = 0;
+        while (i >= 0 && j >= 0) {
+            const int p = i >> 1, s = j - (i & ~1) + wl, g = s >> 3;
+            if (which == 0 && (i & 1)) {
+                // four row pairs down the diagonal: the odd row's step is s in each, the even row's s - 1
+                uint32_t w1[4], w0[4];
+                const int ge = (s - 1) >> 3;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const uint32_t *q = zw + (size_t)max(p - t, 0) * prow;
+                    w1[t] = q[(size_t)g * 128u + 2u];
+                    w0[t] = q[(size_t)max(ge, 0) * 128u];
+                }
+                uint32_t left = 0u, d1 = 4u * ((uint32_t)(s & 7) ^ 3u), d0 = 4u * ((uint32_t)((s - 1) & 7) ^ 3u);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    if (left) break;
+                    if (i < 0 || j < 0) break;
+                    uint32_t h = (w1[t] >> d1) & 3u;
+                    if (h != 3u) { left = 1u; break; }
+                    push(0, 1);
+                    --i;
+                    --j;
+                    if (i < 0 || j < 0) break;
+                    h = (w0[t] >> d0) & 3u;
+                    if (h != 3u) { left = 1u; break; }
+                    push(0, 1);
+                    --i;
+                    --j;
+                }
+                if (!left) continue;  // the walk is still on the diagonal, or done
+            }
+            // one cell
+            const int p1 = i >> 1, s1 = j - (i & ~1) + wl;
+            const uint32_t d = zw[(size_t)p1 * prow + (size_t)(s1 >> 3) * 128u + 2u * (uint32_t)(i & 1)] >>
+                               (4u * ((uint32_t)(s1 & 7) ^ 3u));
+            if (which == 0) which = (d & 3u) == 3u ? 0u : ((d & 3u) == 1u ? 1u : 2u);
+            else if (which == 1) which = d & 4u ? 0u : 1u;
+            else which = d & 8u ? 0u : 2u;
+            if (which == 0) { push(0, 1); --i; --j; }
+            else if (which == 1) { push(2, 1); --i; }
+            else { push(1, 1); --j; }
+        }
+        if (i >= 0) push(2, (uint32_t)(i + 1));
+        if (j >= 0) push(1, (uint32_t)(j + 1));
+        if (run) cg[nc++] = (run << 4) | run_op;
+        for (int a = 0, b = nc - 1; a < b; ++a, --b) {
+            const uint32_t v = cg[a];
+            cg[a] = cg[b];
+            cg[b] = v;
+        }
+        ncig[k] = nc;
     }
 }
 
@@ -926,6 +1094,73 @@ cudaError_t launch_global(const uint8_t *seq, const GlobalDevJob *jobs, const ui
                                      s);
 }
 
+// The tagged kernel over sorted alignments [start, start + count) whose bands reach at most wl / wr
+// columns left / right of the diagonal; the block size that keeps the most warps resident.
+template <int TB>
+cudaError_t launch_tag_tb(const uint8_t *seq, const GlobalDevJob *jobs, const uint32_t *order, uint32_t start,
+                          uint32_t count, const Scoring &sc, const gtag::TagRule &tr, int max_slots, int max_sel,
+                          size_t smem, const gtag::WarpGroup *groups, uint32_t gbase, uint8_t *z, int32_t *score,
+                          int32_t *ncig, uint32_t *err, unsigned long long *cells, cudaStream_t s)
+{
+    const bool sym = sc.o_del + sc.e_del == sc.o_ins + sc.e_ins;
+    auto kern = sym ? gtag::tag_kernel<TB, true, GlobalDevJob> : gtag::tag_kernel<TB, false, GlobalDevJob>;
+    // process-wide per kernel: always the ceiling (concurrent contexts must not shrink it)
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT - 1024);
+    if (e != cudaSuccess) return e;
+    const uint32_t threads = tr.single ? count : (count + 1) / 2;
+    kern<<<(threads + TB - 1) / TB, TB, smem, s>>>(seq, jobs, order, start, count, sc, tr, max_slots, max_sel, groups,
+                                                  gbase, z, score, ncig, GLB_TB_TAGGED, ERR_RANGE, err, cells);
+    return cudaGetLastError();
+}
+
+// Shared memory of TB threads of the tagged kernel.
+size_t tag_smem(int wl, int wr, int qmax, int tb) { return gtag::thread_bytes(wl, wr, qmax) * (size_t)tb; }
+
+cudaError_t launch_tag(const uint8_t *seq, const GlobalDevJob *jobs, const uint32_t *order, uint32_t start,
+                       uint32_t count, const Scoring &sc, const gtag::TagRule &tr, int wl, int wr, int qmax,
+                       const gtag::WarpGroup *groups, uint32_t gbase, uint8_t *z, int32_t *score, int32_t *ncig,
+                       uint32_t *err, unsigned long long *cells, cudaStream_t s)
+{
+    int best = 32, warps = 0;
+    for (int tb = 128; tb >= 32; tb >>= 1) {
+        const size_t sm = tag_smem(wl, wr, qmax, tb);
+        if (sm > SMEM_LIMIT - 1024) continue;
+        const int r = std::min<int>(32, (int)((228u * 1024u) / (sm + 1280u))) * tb / 32;
+        if (r >= warps) {  // smaller blocks on ties: a launch is only a few waves
+            warps = r;
+            best = tb;
+        }
+    }
+    const int ms = gtag::slots(wl, wr), mq = (gtag::sel_count(qmax, wl, wr) + 3) & ~3;
+    const size_t smem = tag_smem(wl, wr, qmax, best);
+    if (best == 128)
+        return launch_tag_tb<128>(seq, jobs, order, start, count, sc, tr, ms, mq, smem, groups, gbase, z, score, ncig,
+                                  err, cells, s);
+    if (best == 64)
+        return launch_tag_tb<64>(seq, jobs, order, start, count, sc, tr, ms, mq, smem, groups, gbase, z, score, ncig,
+                                 err, cells, s);
+    return launch_tag_tb<32>(seq, jobs, order, start, count, sc, tr, ms, mq, smem, groups, gbase, z, score, ncig, err,
+                             cells, s);
+}
+
+// The scorings the tagged kernel takes.
+gtag::TagRule tag_rule(const Scoring &sc, int m, const int8_t *mat)
+{
+    gtag::TagRule r;
+    int mn = 0, mx = 0;
+    for (int i = 0; i < m * m; ++i) {
+        mn = std::min(mn, (int)mat[i]);
+        mx = std::max(mx, (int)mat[i]);
+    }
+    r.mn = -mn;
+    r.mx = mx;
+    r.oe = std::max(sc.o_del + sc.e_del, sc.o_ins + sc.e_ins);
+    r.e = std::max(sc.e_del, sc.e_ins);
+    r.ok = m <= 5 && r.mn <= gtag::MAX_ENTRY && mx <= gtag::MAX_ENTRY && sc.o_del <= gtag::MAX_OE &&
+           sc.o_ins <= gtag::MAX_OE && r.e <= gtag::MAX_OE && r.oe <= gtag::MAX_OE;
+    return r;
+}
+
 // The traceback of jobs order[base .. base + count), after their DP launches.
 cudaError_t launch_global_traceback(const GlobalDevJob *jobs, const uint32_t *order, uint32_t base, uint32_t count,
                                     const uint8_t *z, uint32_t *cig, int32_t *ncig, uint32_t *err, int nsm,
@@ -962,7 +1197,7 @@ struct GlobalBufs {
     HostBuf h_seq, h_jobs, h_res;
     DevBuf d_seq, d_jobs, d_z, d_cig, d_res, d_doff, d_dense, d_tmp;
     // device-gather route
-    DevBuf d_sz, d_flags;
+    DevBuf d_sz, d_flags, d_groups, d_tz;
     HostBuf h_tot;
 };
 
@@ -992,7 +1227,7 @@ void global_release(bwacuda_ctx *c)
     b.h_seq.release(); b.h_jobs.release(); b.h_res.release();
     b.d_seq.release(); b.d_jobs.release(); b.d_z.release(); b.d_cig.release(); b.d_res.release();
     b.d_doff.release(); b.d_dense.release(); b.d_tmp.release();
-    b.d_sz.release(); b.d_flags.release(); b.h_tot.release();
+    b.d_sz.release(); b.d_flags.release(); b.h_tot.release(); b.d_groups.release(); b.d_tz.release();
     for (int x = 0; x < GlobalState::NSIDE; ++x) {
         if (c->global->side[x]) {
             cudaStreamSynchronize(c->global->side[x]);
@@ -1015,7 +1250,7 @@ namespace {
 // run as kernels that read and write the caller's host arrays through the host
 // page tables; the host launches and reads back four words per chunk.
 int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n, const Scoring &sc,
-                        const GlbNarrowRule &nrule, int32_t *score, uint64_t *cigar_off, uint32_t *cigar,
+                        const GlbNarrowRule &nrule, gtag::TagRule trule, int32_t *score, uint64_t *cigar_off, uint32_t *cigar,
                         size_t cigar_cap)
 {
     GlobalState &G = *c->global;
@@ -1035,51 +1270,68 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
     bool short_buf = false;
     int rc = BWACUDA_OK;
     cudaError_t e = cudaSuccess;
-    if ((e = b.d_flags.ensure(256)) != cudaSuccess) return cuda_status(e);
-    if ((e = b.h_tot.ensure(512)) != cudaSuccess) return cuda_status(e);
+    if ((e = b.d_flags.ensure(512)) != cudaSuccess) return cuda_status(e);
+    if ((e = b.h_tot.ensure(1024)) != cudaSuccess) return cuda_status(e);
     uint64_t *ht = static_cast<uint64_t *>(b.h_tot.p);
     for (size_t c0 = 0, cn = 0; c0 < n && rc == BWACUDA_OK; c0 += cn) {
         cn = std::min(chunk, n - c0);
         const bwacuda_global_job *hj = jobs + c0;
+        // one alignment a thread below a warp of them per SM: 300 alignments in 0.82 ms against 1.21 in
+        // pairs, of which some always differ and take two passes
+        trule.single = cn < (size_t)nsm * 32;
         // planning arrays: seq / cig / z sizes and offsets (cn + 1 each), keys and indices (two
         // copies each for the sort)
         const size_t n1 = cn + 1;
-        if ((e = b.d_sz.ensure(n1 * 6 * 8 + n1 * 4 * 4 + 256)) != cudaSuccess) break;
+        const size_t ngmax = cn / 64 + GLB_NBUCKETS, g1n = ngmax + 1;
+        if ((e = b.d_sz.ensure(n1 * 6 * 8 + n1 * 16 + n1 * 4 * 4 + g1n * 16 + 256)) != cudaSuccess) break;
+        if ((e = b.d_groups.ensure(g1n * sizeof(gtag::WarpGroup))) != cudaSuccess) break;
         uint64_t *seq_sz = static_cast<uint64_t *>(b.d_sz.p), *seq_off = seq_sz + n1;
         uint64_t *cig_sz = seq_off + n1, *cig_off = cig_sz + n1;
         uint64_t *z_sz = cig_off + n1, *z_off = z_sz + n1;
-        uint32_t *keys = reinterpret_cast<uint32_t *>(z_off + n1), *keys2 = keys + n1;
+        uint64_t *tz_sz = z_off + n1, *tz_off = tz_sz + g1n;  // the tagged kernel's warp groups
+        // 16-byte records from an aligned start
+        int4 *dims = reinterpret_cast<int4 *>((reinterpret_cast<uintptr_t>(tz_off + g1n) + 15) & ~(uintptr_t)15);
+        uint32_t *keys = reinterpret_cast<uint32_t *>(dims + n1), *keys2 = keys + n1;
         uint32_t *idx = keys2 + n1, *order = idx + n1;
-        // [0] errors, [16..31] bucket stats, [32..47] bounds, [48..55] bucket holds a job too wide for 16-bit cells
+        gtag::WarpGroup *wgroups = static_cast<gtag::WarpGroup *>(b.d_groups.p);
+        // [0] errors, [16..47] class stats, [48..79] bounds, [80..95] the class's left band (tagged) or
+        // whether it holds a job too wide for 16-bit cells
         uint32_t *flags = static_cast<uint32_t *>(b.d_flags.p);
-        uint32_t *bstat = flags + 16, *bounds = flags + 32, *bwide = flags + 48;
+        uint32_t *bstat = flags + 16, *bounds = flags + 48, *bwide = flags + 80;
         size_t t1 = 0, t2 = 0, t3 = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, t1, (const uint64_t *)nullptr, (uint64_t *)nullptr, (int)cn + 1);
         cub::DeviceScan::ExclusiveSum(nullptr, t2, (const int32_t *)nullptr, (uint64_t *)nullptr, (int)cn + 1);
         cub::DeviceRadixSort::SortPairs(nullptr, t3, (const uint32_t *)nullptr, (uint32_t *)nullptr,
-                                        (const uint32_t *)nullptr, (uint32_t *)nullptr, (int)cn, 0, 25);
+                                        (const uint32_t *)nullptr, (uint32_t *)nullptr, (int)cn, 0, 32);
         if ((e = b.d_tmp.ensure(std::max(std::max(t1, t2), t3) + 64)) != cudaSuccess) break;
-        if ((e = cudaMemsetAsync(flags, 0, 256, s)) != cudaSuccess) break;
+        if ((e = cudaMemsetAsync(flags, 0, 512, s)) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(seq_sz + cn, 0, 8, s)) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(cig_sz + cn, 0, 8, s)) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(z_sz + cn, 0, 8, s)) != cudaSuccess) break;
         uint32_t grid = (uint32_t)std::min<size_t>((cn + 255) / 256, (size_t)nsm * 8);
-        glb_plan_kernel<<<grid, 256, 0, s>>>(hj, (uint32_t)cn, qlim, nrule, seq_sz, cig_sz, z_sz, keys, idx, flags,
-                                             bstat, bwide);
+        glb_plan_kernel<<<grid, 256, 0, s>>>(hj, (uint32_t)cn, qlim, nrule, trule, seq_sz, cig_sz, z_sz, keys, idx, flags,
+                                             bstat, bwide, dims);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, seq_sz, seq_off, (int)cn + 1, s)) != cudaSuccess) break;
         if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, cig_sz, cig_off, (int)cn + 1, s)) != cudaSuccess) break;
         if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, z_sz, z_off, (int)cn + 1, s)) != cudaSuccess) break;
-        if ((e = cub::DeviceRadixSort::SortPairs(b.d_tmp.p, t3, keys, keys2, idx, order, (int)cn, 0, 25, s)) != cudaSuccess)
+        if ((e = cub::DeviceRadixSort::SortPairs(b.d_tmp.p, t3, keys, keys2, idx, order, (int)cn, 0, 32, s)) != cudaSuccess)
             break;
         glb_bucket_bounds_kernel<<<1, 32, 0, s>>>(keys2, (uint32_t)cn, bounds);
+        glb_warp_groups_kernel<<<(uint32_t)std::min<size_t>((g1n * 32 + 255) / 256, (size_t)nsm * 8), 256, 0, s>>>(
+            dims, order, bounds, trule, (uint32_t)ngmax, wgroups, tz_sz);
+        if ((e = cudaGetLastError()) != cudaSuccess) break;
+        if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, tz_sz, tz_off, (int)g1n, s)) != cudaSuccess) break;
+        glb_group_offsets_kernel<<<(uint32_t)std::min<size_t>((ngmax + 255) / 256, 1024), 256, 0, s>>>(
+            tz_off, (uint32_t)ngmax, wgroups);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(ht + 0, seq_off + cn, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(ht + 1, cig_off + cn, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(ht + 2, z_off + cn, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
-        if ((e = cudaMemcpyAsync(ht + 3, flags, 256, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
+        if ((e = cudaMemcpyAsync(ht + 3, tz_off + ngmax, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
+        if ((e = cudaMemcpyAsync(ht + 4, flags, 512, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) break;
-        const uint32_t *hf = reinterpret_cast<const uint32_t *>(ht + 3);
+        const uint32_t *hf = reinterpret_cast<const uint32_t *>(ht + 4);
         if (hf[0] & 1u) {
             // an invalid job, or a query longer than the kernel takes: find which on the host
             rc = BWACUDA_EINVAL;
@@ -1087,7 +1339,7 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
                 if (hj[k].qlen > qlim && hj[k].qlen >= 0 && hj[k].tlen >= 0) rc = BWACUDA_EUNSUPPORTED;
             break;
         }
-        if (ht[2] > kMaxZBytes && cn > 1024) {  // plan this range again in halves
+        if (ht[2] + ht[3] > kMaxZBytes && cn > 1024) {  // plan this range again in halves
             chunk = cn / 2;
             cn = 0;
             continue;
@@ -1095,6 +1347,7 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         if ((e = b.d_seq.ensure(ht[0] + 16)) != cudaSuccess) break;
         if ((e = b.d_cig.ensure(ht[1] * 4 + 16)) != cudaSuccess) break;
         if ((e = b.d_z.ensure(ht[2] + 16)) != cudaSuccess) break;
+        if ((e = b.d_tz.ensure(ht[3] + 16)) != cudaSuccess) break;
         if ((e = b.d_jobs.ensure(cn * sizeof(GlobalDevJob))) != cudaSuccess) break;
         if ((e = b.d_res.ensure((cn + 1) * 8 + 16)) != cudaSuccess) break;
         if ((e = b.d_doff.ensure((cn + 1) * 8)) != cudaSuccess) break;
@@ -1110,18 +1363,27 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         // queries first, round-robin over the context's stream and the side streams so a
         // bucket's blocks fill the last partial wave of the ones before it; the tracebacks
         // follow all of them
-        const uint32_t *hb = hf + 16, *hbd = hf + 32, *hbw = hf + 48;
+        const uint32_t *hb = hf + 16, *hbd = hf + 48, *hbw = hf + 80;
+        uint32_t gfirst[GLB_NBUCKETS + 1] = {0};  // first warp group of each tagged class
+        for (int bk = 0; bk < GLB_NBUCKETS; ++bk)
+            gfirst[bk + 1] = gfirst[bk] + (hbd[2 * bk + 1] - hbd[2 * bk] + 63u) / 64u;
         if ((e = cudaEventRecord(G.ready, s)) != cudaSuccess) break;
         for (int x = 0; x < GlobalState::NSIDE && e == cudaSuccess; ++x) e = cudaStreamWaitEvent(G.side[x], G.ready, 0);
         if (e != cudaSuccess) break;
         int nl = 0;
-        for (int bk = GLB_NBUCKETS - 1; bk >= 0 && e == cudaSuccess; --bk) {
+        for (int bk = GLB_NCLASSES - 1; bk >= 0 && e == cudaSuccess; --bk) {
             const uint32_t b0 = hbd[2 * bk], b1 = hbd[2 * bk + 1];
             if (b1 <= b0) continue;
-            e = launch_global(static_cast<const uint8_t *>(b.d_seq.p), dj, order, b0, b1 - b0, sc, (int)hb[2 * bk],
-                              (int)hb[2 * bk + 1], hbw[bk] == 0u, static_cast<uint8_t *>(b.d_z.p),
-                              static_cast<uint32_t *>(b.d_cig.p), d_score, d_ncig, d_err, d_cells,
-                              nl % (GlobalState::NSIDE + 1) ? G.side[nl % (GlobalState::NSIDE + 1) - 1] : s);
+            cudaStream_t bs = nl % (GlobalState::NSIDE + 1) ? G.side[nl % (GlobalState::NSIDE + 1) - 1] : s;
+            const uint8_t *sq = static_cast<const uint8_t *>(b.d_seq.p);
+            if (bk < GLB_NBUCKETS)
+                e = launch_tag(sq, dj, order, b0, b1 - b0, sc, trule, (int)hbw[bk], (int)hb[2 * bk], (int)hb[2 * bk + 1],
+                               wgroups, gfirst[bk], static_cast<uint8_t *>(b.d_tz.p), d_score, d_ncig, d_err, d_cells,
+                               bs);
+            else
+                e = launch_global(sq, dj, order, b0, b1 - b0, sc, (int)hb[2 * bk], (int)hb[2 * bk + 1], hbw[bk] == 0u,
+                                  static_cast<uint8_t *>(b.d_z.p), static_cast<uint32_t *>(b.d_cig.p), d_score, d_ncig,
+                                  d_err, d_cells, bs);
             ++nl;
             c->stats.kernel_launches += 1;
         }
@@ -1133,7 +1395,16 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
             for (int x = 0; x < GlobalState::NSIDE; ++x) cudaStreamSynchronize(G.side[x]);  // nothing runs on
             break;
         }
-        if ((e = launch_global_traceback(dj, nullptr, 0, (uint32_t)cn, static_cast<const uint8_t *>(b.d_z.p),
+        const uint32_t ntag = hbd[2 * GLB_NBUCKETS];  // the tagged classes sort first
+        if (ntag) {
+            const uint32_t ng = gfirst[GLB_NBUCKETS];
+            glb_tag_traceback_kernel<<<(uint32_t)std::min<size_t>(((size_t)ng * 64 + 255) / 256, (size_t)nsm * 8), 256, 0,
+                                       s>>>(dj, order, wgroups, ng, trule, static_cast<const uint8_t *>(b.d_tz.p),
+                                            static_cast<uint32_t *>(b.d_cig.p), d_ncig);
+            if ((e = cudaGetLastError()) != cudaSuccess) break;
+        }
+        if (ntag < cn &&
+            (e = launch_global_traceback(dj, order, ntag, (uint32_t)cn - ntag, static_cast<const uint8_t *>(b.d_z.p),
                                          static_cast<uint32_t *>(b.d_cig.p), d_ncig, d_err, nsm, s)) != cudaSuccess)
             break;
         if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t2, d_ncig, d_doff, (int)cn + 1, s)) != cudaSuccess) break;
@@ -1141,11 +1412,11 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         glb_store_kernel<<<grid, 256, 0, s>>>(dj, (uint32_t)cn, d_score, static_cast<const uint32_t *>(b.d_cig.p), d_ncig,
                                              d_doff, out_base, cigar ? cigar_cap : 0, score + c0, cigar_off + c0, cigar);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
-        if ((e = cudaMemcpyAsync(ht + 40, d_doff + cn, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
+        if ((e = cudaMemcpyAsync(ht + 100, d_doff + cn, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) break;
-        if (!cigar || out_base + ht[40] > cigar_cap) short_buf = true;
-        out_base += ht[40];
-        c->stats.kernel_launches += 11;
+        if (!cigar || out_base + ht[100] > cigar_cap) short_buf = true;
+        out_base += ht[100];
+        c->stats.kernel_launches += 14;
     }
     if (e != cudaSuccess) return cuda_status(e);
     if (rc) {
@@ -1183,8 +1454,8 @@ extern "C" int bwacuda_ksw_global2_batch(bwacuda_ctx *c, const bwacuda_global_jo
     if (device_gather) {
         if (!c->pageable_access) return BWACUDA_EUNSUPPORTED;
         const Scoring scd = make_scoring(m, mat, o_del, e_del, o_ins, e_ins);
-        return global_batch_device(c, jobs, n, scd, global_narrow_rule(scd, m, mat), score, cigar_off, cigar,
-                                   cigar_cap);
+        return global_batch_device(c, jobs, n, scd, global_narrow_rule(scd, m, mat), tag_rule(scd, m, mat), score,
+                                   cigar_off, cigar, cigar_cap);
     }
     const int qlim = global_max_qlen();
     for (size_t k = 0; k < n; ++k) {
