@@ -219,8 +219,8 @@ void batched_get_tuning(bwacuda_ctx *c, int *tb, int *grab, int *step)
 static cudaError_t ensure_bufs(BatchBufs &bb, size_t n)
 {
     cudaError_t e;
-    if ((e = bb.keys_in.ensure(n * 2 + 16)) != cudaSuccess) return e;
-    if ((e = bb.keys_out.ensure(n * 2 + 16)) != cudaSuccess) return e;
+    if ((e = bb.keys_in.ensure(n * 4 + 16)) != cudaSuccess) return e;
+    if ((e = bb.keys_out.ensure(n * 4 + 16)) != cudaSuccess) return e;
     if ((e = bb.idx_in.ensure(n * 4 + 16)) != cudaSuccess) return e;
     if ((e = bb.idx_out.ensure(n * 4 + 16)) != cudaSuccess) return e;
     if ((e = bb.xl.ensure(((size_t)XL_WORK_WORDS + n) * 4 + 16)) != cudaSuccess) return e;
@@ -272,7 +272,7 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
     if (lanes == 8) {
         uint32_t *order = static_cast<uint32_t *>(bb.idx_out.p);
         if ((e = ext_sort_jobs(d_jobs, n, P.sc.max_sc, 1u, d_seq, P.ug, P.zdrop, d_out,
-                               static_cast<uint16_t *>(bb.keys_in.p), static_cast<uint16_t *>(bb.keys_out.p),
+                               static_cast<uint32_t *>(bb.keys_in.p), static_cast<uint32_t *>(bb.keys_out.p),
                                static_cast<uint32_t *>(bb.idx_in.p), order, bb.tmp.p, bb.tmp.cap, s)) != cudaSuccess)
             return e;
         X.order = order;
@@ -297,8 +297,8 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
     const bool lanes = ext_pair_lanes_ok(P.sc.o_del, P.sc.e_del, P.sc.o_ins, P.sc.e_ins);
     if (lanes && batched_is_small(c, n, P)) return enqueue_small(c, bb, d_seq, d_jobs, n, P, d_out, s, err, cells);
     cudaError_t e = ext_sort_and_bucket(d_jobs, n, P.sc.max_sc, lanes, d_seq, P.ug, P.zdrop, d_out,
-                                        static_cast<uint16_t *>(bb.keys_in.p),
-                                        static_cast<uint16_t *>(bb.keys_out.p), static_cast<uint32_t *>(bb.idx_in.p),
+                                        static_cast<uint32_t *>(bb.keys_in.p),
+                                        static_cast<uint32_t *>(bb.keys_out.p), static_cast<uint32_t *>(bb.idx_in.p),
                                         static_cast<uint32_t *>(bb.idx_out.p), bb.tmp.p, bb.tmp.cap,
                                         static_cast<const ExtBucketDef *>(B->d_defs.p), B->nb,
                                         static_cast<uint32_t *>(bb.table.p), s);

@@ -95,6 +95,24 @@ struct TargetStream {
     }
 };
 
+// Sixteen bases from column j on of a slice of n bases, four a word (0 past its end); every word of the
+// slice is loaded once, all together.
+__device__ __forceinline__ void load16(const uint8_t *q, int n, int j, uint32_t (&v)[4])
+{
+    const uintptr_t a = reinterpret_cast<uintptr_t>(q);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3) + (j >> 2);
+    const int off = (int)(a & 3), last = off + n - j;  // bytes of the slice from word w[0] on
+    uint32_t x[5];
+#pragma unroll
+    for (int u = 0; u < 5; ++u) x[u] = 4 * u < last && n > j ? w[u] : 0u;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        v[u] = __funnelshift_r(x[u], x[u + 1], 8 * off);
+        const int left = n - j - 4 * u;  // bases of the slice in this word
+        if (left < 4) v[u] &= left > 0 ? (1u << (8 * left)) - 1u : 0u;
+    }
+}
+
 // Runs job J; returns the ExtendResult, adds the inner-loop iterations to ncells.
 template <class F, int TB>
 __device__ __forceinline__ bwacuda_ext_result ext_run_job(typename F::T *__restrict__ cell,

@@ -140,24 +140,6 @@ __device__ __forceinline__ uint32_t fix_n(uint32_t s2, uint32_t c, uint32_t n2)
     return (s2 & ~mk) | (n2 & mk);
 }
 
-// Sixteen bases from column j on of a slice of n bases, four a word (0 past its end); every word of the
-// slice is loaded once, all together.
-__device__ __forceinline__ void load16(const uint8_t *q, int n, int j, uint32_t (&v)[4])
-{
-    const uintptr_t a = reinterpret_cast<uintptr_t>(q);
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3) + (j >> 2);
-    const int off = (int)(a & 3), last = off + n - j;  // bytes of the slice from word w[0] on
-    uint32_t x[5];
-#pragma unroll
-    for (int u = 0; u < 5; ++u) x[u] = 4 * u < last && n > j ? w[u] : 0u;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        v[u] = __funnelshift_r(x[u], x[u + 1], 8 * off);
-        const int left = n - j - 4 * u;  // bases of the slice in this word
-        if (left < 4) v[u] &= left > 0 ? (1u << (8 * left)) - 1u : 0u;
-    }
-}
-
 // A thread's two alignments: whether they share a pass (equal bands, and the larger sizes still fit),
 // and the sizes of the pass.
 struct PairGeo {

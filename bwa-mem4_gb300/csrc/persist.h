@@ -51,13 +51,13 @@ cudaError_t ext_sort_prefer_shared();
 // pair_lanes false (gap costs too large for 16-bit lanes) keeps every job out of
 // the 8-bit class.
 cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, uint32_t min_cls, const uint8_t *seq,
-                          const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint16_t *keys_in,
-                          uint16_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp, size_t tmp_bytes,
+                          const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
+                          uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp, size_t tmp_bytes,
                           cudaStream_t s);
 cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, bool pair_lanes,
                                 const uint8_t *seq,
-                                const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint16_t *keys_in,
-                                uint16_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp,
+                                const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
+                                uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp,
                                 size_t tmp_bytes, const ExtBucketDef *d_defs, int nb, uint32_t *d_table,
                                 cudaStream_t s);
 // per-grab instantiations (ext_persist_g1.cu, _g2.cu, _g4.cu)
