@@ -20,6 +20,15 @@ constexpr int FAN = 4;  // bucket streams
 // Open-ended buckets: jobs per SM from which the band kernel gives a job 8 lanes, below it 32 (queries
 // of 2-10 kb on 152 SMs: 1,000 jobs 9.6 / 6.5 ms, 2,400 jobs 9.8 / 9.8, 20,000 jobs 23.1 / 42.4).
 constexpr int BAND_LANES8_JOBS = 14;
+// Two jobs a thread (ext_dual.cuh) from this many jobs per SM on, in the 8-bit buckets of up to this
+// many columns (longer ones leave an SM too few of its warps).  Milliseconds on 152 SMs, one / two jobs
+// a thread:        read pairs     mixed lengths    1% errors and N bases
+//     131,072     0.87 / 0.92      1.89 / 2.09      0.94 / 1.45
+//     524,288     2.01 / 1.79      2.46 / 2.66      2.17 / 2.29
+//   1,048,576     3.43 / 3.14      4.09 / 4.00      3.96 / 3.90
+//   4,194,304    12.63 / 11.26    14.95 / 13.40    14.42 / 13.90
+constexpr int EXT_DUAL_JOBS_PER_SM = 5000;
+constexpr int EXT_DUAL_QCAP = 129;
 
 // Device work buffers of one in-flight batch.
 struct BatchBufs {
@@ -271,7 +280,7 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
     const int lanes = n < (size_t)B->nsm * 8 ? 32 : (n < (size_t)B->nsm * 20 ? 16 : 8);
     if (lanes == 8) {
         uint32_t *order = static_cast<uint32_t *>(bb.idx_out.p);
-        if ((e = ext_sort_jobs(d_jobs, n, P.sc.max_sc, 1u, d_seq, P.ug, P.zdrop, d_out,
+        if ((e = ext_sort_jobs(d_jobs, n, P.sc.max_sc, 1u, false, d_seq, P.ug, P.zdrop, d_out,
                                static_cast<uint32_t *>(bb.keys_in.p), static_cast<uint32_t *>(bb.keys_out.p),
                                static_cast<uint32_t *>(bb.idx_in.p), order, bb.tmp.p, bb.tmp.cap, s)) != cudaSuccess)
             return e;
@@ -296,7 +305,9 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
     BatchedState *B = c->batched;
     const bool lanes = ext_pair_lanes_ok(P.sc.o_del, P.sc.e_del, P.sc.o_ins, P.sc.e_ins);
     if (lanes && batched_is_small(c, n, P)) return enqueue_small(c, bb, d_seq, d_jobs, n, P, d_out, s, err, cells);
-    cudaError_t e = ext_sort_and_bucket(d_jobs, n, P.sc.max_sc, lanes, d_seq, P.ug, P.zdrop, d_out,
+    // two jobs a thread in the 8-bit buckets of large batches
+    const bool dual = lanes && P.sc.m <= 5 && n >= (size_t)B->nsm * EXT_DUAL_JOBS_PER_SM;
+    cudaError_t e = ext_sort_and_bucket(d_jobs, n, P.sc.max_sc, lanes, dual, d_seq, P.ug, P.zdrop, d_out,
                                         static_cast<uint32_t *>(bb.keys_in.p),
                                         static_cast<uint32_t *>(bb.keys_out.p), static_cast<uint32_t *>(bb.idx_in.p),
                                         static_cast<uint32_t *>(bb.idx_out.p), bb.tmp.p, bb.tmp.cap,
@@ -371,7 +382,9 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
         if (B->defs[b].kernel == 1) continue;
         L.stream = bb.fan[k++ % FAN];
         uint32_t *tab = static_cast<uint32_t *>(bb.table.p) + 4 * b;
-        if ((e = ext_persist_launch(L, B->defs[b], tab, B->nsm, B->tb)) != cudaSuccess) return e;
+        e = dual && B->defs[b].cls == 0 && B->defs[b].qcap <= EXT_DUAL_QCAP ? ext_dual_launch(L, B->defs[b], tab, B->nsm)
+                                        : ext_persist_launch(L, B->defs[b], tab, B->nsm, B->tb);
+        if (e != cudaSuccess) return e;
     }
     for (int f = 0; f < FAN; ++f) {
         if ((e = cudaEventRecord(bb.join[f], bb.fan[f])) != cudaSuccess) return e;

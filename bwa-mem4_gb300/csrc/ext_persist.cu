@@ -90,13 +90,22 @@ __device__ bool ungapped_hit(const uint8_t *q, int qlen, const uint8_t *t, int t
 // Sort keys; with the ungapped rule on, jobs it settles get their result here
 // and key class 3, which no bucket covers.
 __global__ void ext_keys_kernel(const bwacuda_dev_ext_job *__restrict__ jobs, uint32_t n, int max_sc,
-                                uint32_t min_cls, const uint8_t *__restrict__ seq, const UngappedRule ug, int zdrop,
+                                uint32_t min_cls, int n_to_16, const uint8_t *__restrict__ seq, const UngappedRule ug, int zdrop,
                                 bwacuda_ext_result *__restrict__ out, uint32_t *__restrict__ keys,
                                 uint32_t *__restrict__ idx)
 {
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const bwacuda_dev_ext_job J = jobs[k];
         uint32_t key = ext_sort_key(J, max_sc, min_cls);
+        if (n_to_16 && key < (1u << 20) && J.qlen > 0) {  // an 8-bit job: any code of 4 or more?
+            uint32_t any = 0u;
+            for (int j = 0; j < J.qlen; j += 16) {
+                uint32_t v[4];
+                load16(seq + J.q_off, J.qlen, j, v);
+                any |= v[0] | v[1] | v[2] | v[3];
+            }
+            if (any & 0xfcfcfcfcu) key |= 1u << 20;
+        }
         if (ug.enabled) {
             bwacuda_ext_result r;
             if (ungapped_hit(seq + J.q_off, J.qlen, seq + J.t_off, J.tlen, J.h0, ug, zdrop, r)) {
@@ -207,27 +216,29 @@ size_t ext_sort_temp_bytes(size_t n)
 }
 
 // Keys and their sort: idx_out holds the job indices by key.  min_cls 1 sorts the 8- and 16-bit
-// classes as one.
-cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, uint32_t min_cls, const uint8_t *seq,
-                          const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
+// classes as one; n_to_16 puts 8-bit jobs whose query holds an N into the 16-bit class (the kernel of
+// two jobs a thread scores codes 0..3 only).
+cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, uint32_t min_cls, bool n_to_16,
+                          const uint8_t *seq, const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
                           uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp, size_t tmp_bytes,
                           cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
     uint32_t grid = (uint32_t)((n + 255) / 256);
     if (grid > 8192) grid = 8192;
-    ext_keys_kernel<<<grid, 256, 0, s>>>(jobs, (uint32_t)n, max_sc, min_cls, seq, ug, zdrop, out, keys_in, idx_in);
+    ext_keys_kernel<<<grid, 256, 0, s>>>(jobs, (uint32_t)n, max_sc, min_cls, n_to_16 ? 1 : 0, seq, ug, zdrop, out, keys_in,
+                                         idx_in);
     return cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys_in, keys_out, idx_in, idx_out, (int)n, 0, EXT_KEY_BITS, s);
 }
 
-cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, bool pair_lanes,
+cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, bool pair_lanes, bool n_to_16,
                                 const uint8_t *seq, const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
                                 uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp,
                                 size_t tmp_bytes, const ExtBucketDef *d_defs, int nb, uint32_t *d_table,
                                 cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    const cudaError_t e = ext_sort_jobs(jobs, n, max_sc, pair_lanes ? 0u : 1u, seq, ug, zdrop, out, keys_in, keys_out,
+    const cudaError_t e = ext_sort_jobs(jobs, n, max_sc, pair_lanes ? 0u : 1u, n_to_16, seq, ug, zdrop, out, keys_in, keys_out,
                                         idx_in, idx_out, tmp, tmp_bytes, s);
     if (e != cudaSuccess) return e;
     ext_bucket_bounds_kernel<<<1, EXT_MAX_BUCKETS, 0, s>>>(keys_out, (uint32_t)n, d_defs, nb, d_table);

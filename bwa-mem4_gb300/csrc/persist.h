@@ -50,11 +50,13 @@ cudaError_t ext_sort_prefer_shared();
 // With P.ug enabled the key kernel also settles ungapped hits (results written to out).
 // pair_lanes false (gap costs too large for 16-bit lanes) keeps every job out of
 // the 8-bit class.
-cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, uint32_t min_cls, const uint8_t *seq,
-                          const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
+// An 8-bit bucket with two jobs per thread (ext_dual.cuh): scorings of at most five letters.
+cudaError_t ext_dual_launch(const PersistLaunch &L, const ExtBucketDef &d, uint32_t *d_bucket_table, int nsm);
+cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, uint32_t min_cls, bool n_to_16,
+                          const uint8_t *seq, const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
                           uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp, size_t tmp_bytes,
                           cudaStream_t s);
-cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, bool pair_lanes,
+cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, bool pair_lanes, bool n_to_16,
                                 const uint8_t *seq,
                                 const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
                                 uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp,
