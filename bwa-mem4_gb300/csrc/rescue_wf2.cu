@@ -25,6 +25,10 @@ bool pair_scoring_ok(const Scoring &sc, int *npen)
 {
     if (sc.m > 5 || sc.o_del < 0 || sc.e_del < 0 || sc.o_ins < 0 || sc.e_ins < 0) return false;
     if (sc.o_del + sc.e_del > 128) return false;
+    // a matrix entry above the caller's max_sc would take values past the byte its rule promises
+    for (int t = 0; t < sc.m; ++t)
+        for (int q = 0; q < sc.m; ++q)
+            if ((int8_t)((sc.prof[t][q >> 2] >> (8 * (q & 3))) & 0xffu) > sc.max_sc) return false;
     *npen = 0;
     if (sc.m < 5) return true;
     const int8_t n0 = (int8_t)(sc.prof[0][1] & 0xffu);  // mat[0][4]

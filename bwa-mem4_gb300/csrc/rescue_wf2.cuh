@@ -5,8 +5,8 @@
 // wavefront (ksw_local_fwd, crates/bwa-extend/src/sw.rs:921-1075; start recovery of
 // batched_ksw_align2 / ksw_align2), cell for cell.
 //
-// A job qualifies when every value fits a byte: min(qlen, tlen) * max_sc <= 255 (a local score
-// gains at most max_sc per diagonal step, gaps never add), and its padded query (forward and
+// A job qualifies when every value fits a byte: qlen * max_sc <= 255 (a local score gains at most
+// max_sc per column, gaps never add), and its padded query (forward and
 // reverse) fits 256 columns -- the reference's own 8-bit rescue class (min(q, t) * a < 250 and
 // q < 250, crates/bwa-neon/src/matesw.rs:780-795) lies inside it.  Then the row-maximum key
 // of a job is 16 bits, (H << 8) | (255 - column): the largest H, and among equal H the smallest
@@ -65,7 +65,7 @@ struct Lane2 {
     uint32_t nf;              // 0 in the group's first lane, 1 elsewhere (zeroes the values it receives)
     uint2 *qw;                // the lane's query-profile words of jobs A and B in shared memory, column c
                               // at qw[c * WF2_THREADS] (read once per row; registers hold the DP state)
-    uint32_t cw[(C + 3) / 4]; // key column bytes 255 - j, four columns a word
+    uint32_t kbase;           // 255 - j of the lane's last column j, in both 16-bit lanes
 };
 
 // Gap constants, each 16-bit value in both lanes.
@@ -101,7 +101,7 @@ __device__ __forceinline__ void build_qprof(uint32_t *qp, const Scoring &sc, int
 // Loads the lane's columns of job h (0: A, the low 16-bit lanes; 1: B, the high ones): forward
 // (query[j]) or the reversed prefix (query[qe0 - j]); columns [qlen, qpad) are ksw padding
 // (score 0, part of the row maxima), columns >= qpad do not exist (score -128, never a row
-// maximum).  Job A's call also writes the key column bytes.
+// maximum).
 template <int L, int C>
 __device__ __forceinline__ void load_query2_half(Lane2<L, C> &W, const uint32_t *qp, const uint8_t *q, int ql, int qpd,
                                                  bool rev, int qe0, int h, int m, bool &bad)
@@ -109,10 +109,6 @@ __device__ __forceinline__ void load_query2_half(Lane2<L, C> &W, const uint32_t 
 #pragma unroll
     for (int c = 0; c < C; ++c) {
         const int j = W.k * C + c;
-        if (h == 0) {
-            if ((c & 3) == 0) W.cw[c >> 2] = 0u;
-            W.cw[c >> 2] |= ((uint32_t)(255 - j) & 0xffu) << (8 * (c & 3));
-        }
         uint32_t w = j < qpd ? 0u : NOCOL;
         if (j < ql) {
             const uint32_t code = rev ? q[qe0 - j] : q[j];
@@ -148,13 +144,18 @@ __device__ __forceinline__ uint32_t score2(uint2 q, uint32_t selT, int c, uint32
 // One row of the lane's C columns for both jobs.  hd: H of row i-1 at the column left of the
 // lane's first; f, key: F and the row key entering from the left; on return f, key leave to the
 // right and Hp holds row i.
+// The row-maximum keys (H << 8) | (255 - column) form as multiply-adds H * 256 + (C - 1 - c) on the
+// otherwise idle multiply pipe (k256 = 256, not a constant to the compiler, which would make it a shift
+// of the ALU pipe that bounds this kernel), the lane's columns' start added once a row; H is at most 255
+// in every lane (a column's H is at most (column + 1) * max_sc, rescue_pair_job_ok), so nothing carries.
+// 262,144 windows of 750 bp: 11.02 ms with a permute per column and key.
 template <int C, bool SYM, bool SLOW>
-__device__ __forceinline__ void row2(const uint2 *qw, const uint32_t *cw, uint32_t (&Hp)[C], uint32_t (&E)[C],
+__device__ __forceinline__ void row2(const uint2 *qw, uint32_t kbase, uint32_t k256, uint32_t (&Hp)[C], uint32_t (&E)[C],
                                      uint32_t &f, uint32_t &key, uint32_t hd, uint32_t selT, const Gap2 &g,
                                      uint32_t selN, int ra, int pa, int rb, int pb, uint32_t npa, uint32_t npb)
 {
     uint32_t m0 = __viaddmax_s16x2_relu(hd, score2<SLOW>(qw[0], selT, 0, selN, ra, pa, rb, pb, npa, npb), E[0]);
-    uint32_t kprev = 0u;
+    uint32_t kprev = 0u, kmax = 0u;
 #pragma unroll
     for (int c = 0; c < C; ++c) {
         // M0 of the next column first: it is the last reader of this column's previous-row H,
@@ -164,9 +165,8 @@ __device__ __forceinline__ void row2(const uint2 *qw, const uint32_t *cw, uint32
             m0n = __viaddmax_s16x2_relu(
                 Hp[c], score2<SLOW>(qw[(c + 1) * WF2_THREADS], selT, c + 1, selN, ra, pa, rb, pb, npa, npb), E[c + 1]);
         const uint32_t h = __vimax_s16x2_relu(m0, f);  // H = max(M0, F)
-        // row-maximum key per job: (H << 8) | (255 - column); selector bytes: column, H_A, column, H_B
-        const uint32_t kk = prmt(h, cw[c >> 2], (uint32_t)((4 + (c & 3)) * 0x101 + 0x2000));
-        if (c & 1) key = __vimax3_u16x2(key, kprev, kk);
+        const uint32_t kk = h * k256 + (uint32_t)(C - 1 - c) * 0x10001u;
+        if (c & 1) kmax = __vimax3_u16x2(kmax, kprev, kk);
         else kprev = kk;
         if constexpr (SYM) {
             const uint32_t t = __viaddmax_s16x2(h, g.noe_del, MIN2);  // H - (o + e), both gaps open from it
@@ -181,7 +181,8 @@ __device__ __forceinline__ void row2(const uint2 *qw, const uint32_t *cw, uint32
         Hp[c] = h;
         m0 = m0n;
     }
-    if (C & 1) key = __vimax3_u16x2(key, kprev, kprev);
+    if (C & 1) kmax = __vimax3_u16x2(kmax, kprev, kprev);
+    key = __viaddmax_u16x2(kmax, kbase, key);
 }
 
 // One local-SW pass of both jobs of every group in the warp, in lockstep.  tlen[h] = 0 makes half
@@ -191,7 +192,7 @@ __device__ __forceinline__ void row2(const uint2 *qw, const uint32_t *cw, uint32
 // and padded length per job.  Returns the results in every lane.
 template <int L, int C, bool SYM, bool TMAP>
 __device__ Out2 pass2(const Lane2<L, C> &W, const uint8_t *const t[2], const int tlen[2], const int te0[2],
-                      const Gap2 &g, int npen, int m, bool stop, const int endsc[2], uint16_t *const rk[2],
+                      const Gap2 &g, uint32_t k256, int npen, int m, bool stop, const int endsc[2], uint16_t *const rk[2],
                       const int ql[2], const int qp[2], bool &bad)
 {
     const int k = W.k;
@@ -256,9 +257,9 @@ __device__ Out2 pass2(const Lane2<L, C> &W, const uint8_t *const t[2], const int
                 if (live_a) bad |= tca >= (uint32_t)m;
                 if (live_b) bad |= tcb >= (uint32_t)m;
                 const uint32_t selN = (live_a && tca >= 4u ? 0x54u : 0x10u) | (live_b && tcb >= 4u ? 0x7600u : 0x3200u);
-                row2<C, SYM, true>(W.qw, W.cw, Hp, E, f, key, hprev, selT, g, selN, ra, pa, rb, pb, npa, npb);
+                row2<C, SYM, true>(W.qw, W.kbase, k256, Hp, E, f, key, hprev, selT, g, selN, ra, pa, rb, pb, npa, npb);
             } else {
-                row2<C, SYM, false>(W.qw, W.cw, Hp, E, f, key, hprev, selT, g, 0u, 0, 0, 0, 0, 0u, 0u);
+                row2<C, SYM, false>(W.qw, W.kbase, k256, Hp, E, f, key, hprev, selT, g, 0u, 0, 0, 0, 0, 0u, 0u);
             }
             send_h = Hp[C - 1];
             send_f = f;
@@ -395,7 +396,7 @@ template <int L, int C, bool SYM>
 __global__ void __launch_bounds__(WF2_THREADS, wf2_min_blocks<C>())
 rescue_wf2_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_rescue_job *__restrict__ jobs,
                   const uint32_t *__restrict__ order, uint32_t n, const __grid_constant__ Scoring sc, int mode,
-                  int lanes_fixed, int minsc_all, int npen, uint2 *__restrict__ scratch,
+                  int lanes_fixed, int minsc_all, int npen, uint32_t k256, uint2 *__restrict__ scratch,
                   const uint64_t *__restrict__ scratch_off, bwacuda_rescue_result *__restrict__ out_aln,
                   bwacuda_fwd_result *__restrict__ out_fwd, uint32_t *__restrict__ err)
 {
@@ -408,6 +409,7 @@ rescue_wf2_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_rescue_job 
     W.k = threadIdx.x % L;
     W.qw = qw_s + threadIdx.x;
     W.nf = W.k != 0 ? 1u : 0u;
+    W.kbase = (uint32_t)(255 - (W.k * C + C - 1)) * 0x10001u;
     const bool last = W.k == L - 1;
     bool act[2];
     uint32_t jid[2] = {0u, 0u};
@@ -446,7 +448,7 @@ rescue_wf2_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_rescue_job 
             rk[h] = v.rk;
         }
         const int te0z[2] = {0, 0};
-        fw = pass2<L, C, SYM, false>(W, t, tlen, te0z, g, npen, sc.m, mode == 2, endsc, rk, qlen, qpad, bad);
+        fw = pass2<L, C, SYM, false>(W, t, tlen, te0z, g, k256, npen, sc.m, mode == 2, endsc, rk, qlen, qpad, bad);
     }
     __syncwarp();  // the last lane's key stores before the scans of lanes L - 1 (job A) and L - 2 (job B)
     {
@@ -502,7 +504,7 @@ rescue_wf2_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_rescue_job 
             rk[h] = v.rk;
             load_query2_half<L, C>(W, qp_s, v.q, rq[h], rqpad[h], true, fw.qe[h], h, sc.m, bad);
         }
-        const Out2 rv = pass2<L, C, SYM, true>(W, t, rt, te0, g, npen, sc.m, true, stopsc, rk, rq, rqpad, bad);
+        const Out2 rv = pass2<L, C, SYM, true>(W, t, rt, te0, g, k256, npen, sc.m, true, stopsc, rk, rq, rqpad, bad);
         if (last) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
@@ -531,7 +533,7 @@ cudaError_t launch_wf2(const RescueLaunch &Lr, int npen)
     const uint32_t grid = (uint32_t)((total + threads - 1) / threads);
     if (grid == 0) return cudaSuccess;
     rescue_wf2_kernel<L, C, SYM><<<grid, threads, 0, Lr.stream>>>(Lr.seq, Lr.jobs, Lr.order, (uint32_t)Lr.n, Lr.sc,
-                                                                  Lr.mode, Lr.lanes, Lr.minsc, npen, Lr.scratch,
+                                                                  Lr.mode, Lr.lanes, Lr.minsc, npen, 256u, Lr.scratch,
                                                                   Lr.scratch_off, Lr.out_aln, Lr.out_fwd, Lr.err);
     return cudaGetLastError();
 }

@@ -154,7 +154,7 @@ typedef struct bwacuda_ctx bwacuda_ctx;
 /* Lanes per job of the group-per-job extension kernel: 8, 16 (default) or 32. */
 #define BWACUDA_OPT_LONG_LANES 13
 /* Mate rescue, register wavefront: 4, 8 or 16 = jobs whose every value fits a byte
- * (min(qlen, tlen) * max_sc <= 255, padded query <= 256 columns, bwa-shaped matrix) run two
+ * (qlen * max_sc <= 255, padded query <= 256 columns, bwa-shaped matrix) run two
  * per group of that many lanes, one in each 16-bit lane of the DPX instructions (4 lanes: the
  * most columns per lane); the others stay in the 32-bit wavefront.  1 = 4.  0 = one job per
  * group.  Until this option, BWACUDA_OPT_RESCUE_LANES or the autotuner sets a shape, each launch

@@ -99,3 +99,32 @@ def test_invalid_jobs(fresh):
     js = _ragged(2000, seed=23, qlens=(100, 150))  # and the context still works
     want, _ = oracle.align2_batch(js, minsc=19)
     assert np.array_equal(fresh.ksw_align2_batch(js, minsc=19), want)
+
+
+@pytest.mark.parametrize("max_sc", [1, 2])
+def test_matrix_above_max_sc(fresh, max_sc):
+    """Entries above the caller's max_sc take scores past what its width rule promises."""
+    js = _ragged(3000, seed=31, qlens=(40, 100, 150, 240))
+    mat = oracle.scmat(3, 4)
+    want, _ = oracle.align2_batch(js, mat, minsc=19, max_sc=max_sc)
+    assert want["score"].max() > 255
+    assert np.array_equal(fresh.ksw_align2_batch(js, mat, minsc=19, max_sc=max_sc), want)
+
+
+@pytest.mark.parametrize("a,b", [(1, 4), (2, 3)])
+def test_pairs_whose_targets_end_apart(fresh, a, b):
+    """Long queries against short and long targets in turn: a job's lane computes rows past its target
+    while its neighbour has rows."""
+    rng = np.random.default_rng(41)
+    qs, ts = [], []
+    for k in range(3000):
+        t = rng.integers(0, 4, 400 if k & 1 else int(rng.integers(1, 60))).astype(np.uint8)
+        unit = rng.integers(0, 4, int(rng.integers(1, 4))).astype(np.uint8)
+        q = np.resize(unit, 250 // a)  # repeats: rows past the target keep matching
+        t[:min(len(t), 60)] = np.resize(unit, min(len(t), 60))
+        qs.append(q)
+        ts.append(t)
+    js = B.JobSet.from_lists(qs, ts)
+    mat = oracle.scmat(a, b)
+    want, _ = oracle.align2_batch(js, mat, minsc=19, max_sc=a)
+    assert np.array_equal(fresh.ksw_align2_batch(js, mat, minsc=19, max_sc=a), want)
