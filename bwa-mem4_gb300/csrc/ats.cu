@@ -45,13 +45,19 @@ namespace {
 constexpr uint32_t ERR_INPUT = 8u;
 constexpr size_t ATS_MAX_CHUNK = size_t(1) << 24;  // 32-bit word indexing in the scatter
 constexpr int ATS_FLAG_BYTES = 32;                 // u32 input flag, pad, u64 bins[3]
-// Blocks per SM (of ATS_THREADS threads) of the pipeline's length / gather /
-// scatter launches.  They run beside the persistent DP kernels, in the room
-// those leave free (ATS_RESERVE_*): one block per SM with eight 16-byte loads in
-// flight per lane keeps about 2.4 MB of host reads outstanding, and a second one
-// would take room from the extension.
-constexpr int ATS_BLOCKS_PER_SM = 1;
+// Blocks (of ATS_THREADS threads) of the pipeline's length / gather / scatter launches.  Later
+// chunks' lengths and gathers run beside the persistent DP kernels, in the room those leave free
+// (ATS_RESERVE_*), with a block for every other SM: eight 16-byte loads in flight per lane keep
+// 1.2 MB of host reads outstanding, which still fills the host link, and a block slows the
+// extension blocks of its SM.  2M read pairs: a block on every SM 8.40 ms, two 8.6, one for two SMs
+// 7.75, one for four 7.7-7.9; 700k jobs 3.74 and 3.60, 1.3M 5.42 and 5.13.  The first chunk's run
+// alone and take a block per SM, like the scatter (every other SM: no gain).
 constexpr int ATS_THREADS = 128;
+inline uint32_t ats_grid(size_t items, int nsm, bool alone)
+{
+    const size_t most = alone ? (size_t)nsm : ((size_t)nsm + 1) / 2;
+    return (uint32_t)std::min<size_t>((items + ATS_THREADS - 1) / ATS_THREADS, most);
+}
 // What the persistent kernels leave free per SM while the pipeline runs: one
 // ATS_THREADS block at the gather kernel's register bound (64 per thread).
 constexpr int ATS_RESERVE_REGS = ATS_THREADS * 64;
@@ -238,7 +244,8 @@ int ats_retire(bwacuda_ctx *c, AtsChunk &R, uint32_t *input_flags)
 // Steps 1-2 of a chunk on the plan stream: lengths and validation (the only read of the
 // caller's job array: each job lands in its device descriptor), the offset scan, the byte total
 // back to the host.  Enqueued while the previous chunk's gather runs.
-cudaError_t ats_plan_chunk(bwacuda_ctx *c, AtsChunk &R, const bwacuda_ext_job *hj, size_t cn, const BinRule &br)
+cudaError_t ats_plan_chunk(bwacuda_ctx *c, AtsChunk &R, const bwacuda_ext_job *hj, size_t cn, const BinRule &br,
+                           bool first)
 {
     cudaStream_t p = c->ats->pstream;
     cudaError_t e;
@@ -258,8 +265,7 @@ cudaError_t ats_plan_chunk(bwacuda_ctx *c, AtsChunk &R, const bwacuda_ext_job *h
     uint32_t *flags = static_cast<uint32_t *>(R.flags.p);
     if ((e = cudaMemsetAsync(flags, 0, ATS_FLAG_BYTES, p)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(sizes + cn, 0, 8, p)) != cudaSuccess) return e;
-    const uint32_t grid = (uint32_t)std::min<size_t>((cn + ATS_THREADS - 1) / ATS_THREADS,
-                                                     (size_t)batched_nsm(c) * ATS_BLOCKS_PER_SM);
+    const uint32_t grid = ats_grid(cn, batched_nsm(c), first);
     ats_lengths_kernel<<<grid, ATS_THREADS, 0, p>>>(hj, (uint32_t)cn, br, sizes, flags,
                                                     static_cast<bwacuda_dev_ext_job *>(R.djobs.p));
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -271,7 +277,7 @@ cudaError_t ats_plan_chunk(bwacuda_ctx *c, AtsChunk &R, const bwacuda_ext_job *h
 
 // Step 3 on the gather stream, once the chunk is planned: the host reads the byte total (it
 // sizes the sequence buffer), then the gather.
-cudaError_t ats_gather_chunk(bwacuda_ctx *c, AtsChunk &R, size_t cn, int w)
+cudaError_t ats_gather_chunk(bwacuda_ctx *c, AtsChunk &R, size_t cn, int w, bool first)
 {
     cudaStream_t g = c->ats->gstream;
     cudaError_t e;
@@ -279,8 +285,7 @@ cudaError_t ats_gather_chunk(bwacuda_ctx *c, AtsChunk &R, size_t cn, int w)
     const uint64_t total = *static_cast<const uint64_t *>(R.h_total.p);
     if ((e = R.seq.ensure(total + 16)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(g, R.planned, 0)) != cudaSuccess) return e;
-    const uint32_t grid = (uint32_t)std::min<size_t>((cn + ATS_THREADS - 1) / ATS_THREADS,
-                                                     (size_t)batched_nsm(c) * ATS_BLOCKS_PER_SM);
+    const uint32_t grid = ats_grid(cn, batched_nsm(c), first);
     ats_gather_kernel<<<grid, ATS_THREADS, 0, g>>>((uint32_t)cn, static_cast<const uint64_t *>(R.offs.p), w,
                                                    static_cast<uint8_t *>(R.seq.p),
                                                    static_cast<bwacuda_dev_ext_job *>(R.djobs.p));
@@ -303,8 +308,7 @@ cudaError_t ats_extend_chunk(bwacuda_ctx *c, AtsChunk &R, int si, size_t cn, con
     batched_set_reserve(bb, 0, 0);
     if (e != cudaSuccess) return e;
     const uint32_t words = (uint32_t)(cn * (sizeof(bwacuda_ext_result) / 4));
-    const uint32_t grid = (uint32_t)std::min<size_t>((words + ATS_THREADS - 1) / ATS_THREADS,
-                                                     (size_t)batched_nsm(c) * ATS_BLOCKS_PER_SM);
+    const uint32_t grid = ats_grid(words, batched_nsm(c), true);
     ats_scatter_kernel<<<grid, ATS_THREADS, 0, s>>>(static_cast<const uint32_t *>(R.dout.p), words,
                                                     reinterpret_cast<uint32_t *>(hout));
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -425,7 +429,7 @@ int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int 
     {
         AtsChunk &R0 = c->ats->ring[0];
         if ((rc = ats_retire(c, R0, &input_flags)) == BWACUDA_OK) {
-            const cudaError_t e = ats_plan_chunk(c, R0, jobs, chunk_len(0, 0), br);
+            const cudaError_t e = ats_plan_chunk(c, R0, jobs, chunk_len(0, 0), br, true);
             if (e != cudaSuccess) rc = cuda_status(e);
         }
     }
@@ -433,7 +437,7 @@ int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int 
     for (size_t c0 = 0, cn = 0; c0 < n && rc == BWACUDA_OK; c0 += cn, ++k) {
         cn = chunk_len(k, c0);
         AtsChunk &R = c->ats->ring[k % ATS_RING];
-        cudaError_t e = ats_gather_chunk(c, R, cn, w);
+        cudaError_t e = ats_gather_chunk(c, R, cn, w, k == 0);
         if (e == cudaSuccess) e = ats_extend_chunk(c, R, (int)(k & 1), cn, P, out + c0);
         if (e != cudaSuccess) {
             rc = cuda_status(e);
@@ -445,7 +449,7 @@ int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int 
         if (c1 < n) {
             AtsChunk &R1 = c->ats->ring[(k + 1) % ATS_RING];
             if ((rc = ats_retire(c, R1, &input_flags)) != BWACUDA_OK) break;
-            if ((e = ats_plan_chunk(c, R1, jobs + c1, chunk_len(k + 1, c1), br)) != cudaSuccess) {
+            if ((e = ats_plan_chunk(c, R1, jobs + c1, chunk_len(k + 1, c1), br, false)) != cudaSuccess) {
                 rc = cuda_status(e);
                 break;
             }
