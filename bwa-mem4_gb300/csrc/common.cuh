@@ -108,7 +108,9 @@ __host__ __device__ inline uint32_t slice_words(const uint8_t *src, int len)
 // seq + base_l with base_l = base_0 + 16 * (words of lanes < l) -- the layout an
 // exclusive scan of 16 * (qw + tw) over consecutive jobs gives -- so flat word x
 // is stored at seq + base_0 + 16 x.  All 32 lanes must call it, and lane 0 must
-// carry a job (possibly empty).
+// carry a job (possibly empty).  CONSECUTIVE false: any 16-byte aligned bases, each
+// lane's own (two more shuffles a word).
+template <bool CONSECUTIVE = true>
 __device__ __forceinline__ void warp_gather_slices(uint64_t qa, uint64_t ta, uint64_t base, uint32_t qw, uint32_t tw,
                                                    uint8_t *seq)
 {
@@ -126,6 +128,7 @@ __device__ __forceinline__ void warp_gather_slices(uint64_t qa, uint64_t ta, uin
     constexpr int U = 8;
     for (uint32_t x0 = 0; x0 < total; x0 += 32u * U) {
         uint4 v[U];
+        uint64_t at[U];  // CONSECUTIVE false: destinations
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint32_t x = x0 + (uint32_t)u * 32u + lane;
@@ -140,6 +143,7 @@ __device__ __forceinline__ void warp_gather_slices(uint64_t qa, uint64_t ta, uin
             const uint64_t qa_j = __shfl_sync(0xffffffffu, qa, j);
             const uint64_t ta_j = __shfl_sync(0xffffffffu, ta, j);
             const uint32_t wi = x - pre_j;
+            if constexpr (!CONSECUTIVE) at[u] = __shfl_sync(0xffffffffu, base, j) + 16ull * wi;
             if (x < total)
                 v[u] = wi < qw_j ? reinterpret_cast<const uint4 *>(qa_j)[wi]
                                  : reinterpret_cast<const uint4 *>(ta_j)[wi - qw_j];
@@ -147,7 +151,10 @@ __device__ __forceinline__ void warp_gather_slices(uint64_t qa, uint64_t ta, uin
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint32_t x = x0 + (uint32_t)u * 32u + lane;
-            if (x < total) dst[x] = v[u];
+            if (x < total) {
+                if constexpr (CONSECUTIVE) dst[x] = v[u];
+                else *reinterpret_cast<uint4 *>(seq + at[u]) = v[u];
+            }
         }
     }
 }

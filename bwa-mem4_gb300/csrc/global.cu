@@ -69,7 +69,7 @@ constexpr int GLB_TB_ROWS = -1;   // a row's bytes from column beg (32-bit cell 
 constexpr int GLB_TB_PAIRS = -2;  // from column beg & ~1 (pair kernel)
 constexpr int GLB_TB_TAGGED = -3; // the tagged kernel's nibbles (global_tag.cuh), its own traceback kernel
 constexpr int GLB_TB_AHEAD = 4;     // traceback cells loaded together down the diagonal
-constexpr int GLB_SIDE_STREAMS = 2;  // streams beside the context's for the bucket DP launches
+constexpr int GLB_SIDE_STREAMS = 3;  // streams beside the context's for the class DP launches
 constexpr int GLB_NARROW_D = 8000;
 struct GlbNarrowRule {
     int cost;  // max(o_del + e_del, o_ins + e_ins, -min score, max score)
@@ -736,7 +736,7 @@ __global__ void glb_plan_kernel(const bwacuda_global_job *__restrict__ hj, uint3
                                 GlbNarrowRule nr, gtag::TagRule tr, uint64_t *__restrict__ seq_sz, uint64_t *__restrict__ cig_sz,
                                 uint64_t *__restrict__ z_sz, uint32_t *__restrict__ keys, uint32_t *__restrict__ idx,
                                 uint32_t *__restrict__ flags, uint32_t *__restrict__ bstat, uint32_t *__restrict__ bwide,
-                                int4 *__restrict__ dims)
+                                int4 *__restrict__ dims, GlobalDevJob *__restrict__ dj)
 {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t k0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); k0 < n; k0 += stride) {
@@ -753,6 +753,16 @@ __global__ void glb_plan_kernel(const bwacuda_global_job *__restrict__ hj, uint3
             cig_sz[k] = (uint64_t)ql + (uint64_t)tl + 1u;
             const bool tag = gtag::tag_ok(ql, tl, J.w, tr);
             dims[k] = make_int4(ql, tl, J.w, 0);
+            GlobalDevJob D;
+            D.q_off = reinterpret_cast<uint64_t>(J.query);  // the slice addresses, for the gather
+            D.t_off = reinterpret_cast<uint64_t>(J.target);
+            D.z_off = 0;
+            D.cig_off = 0;
+            D.qlen = ql;
+            D.tlen = tl;
+            D.w = J.w;
+            D.zrow = global_zrow(ql, J.w);
+            dj[k] = D;
             z_sz[k] = tag ? 0u : (uint64_t)tl * (uint64_t)global_zrow(ql, J.w);
             // the class's largest band: right and left of the diagonal (tagged), or slots (the others)
             bs = tag ? gtag::band_right(J.w, ql) : global_band_slots(ql, J.w);
@@ -955,41 +965,37 @@ __global__ void __launch_bounds__(256) glb_tag_traceback_kernel(const GlobalDevJ
     }
 }
 
-// One warp per 32 jobs: lane l writes its job's descriptor, then the warp copies the
-// 32 jobs' slices as aligned 16-byte words (warp_gather_slices).
-__global__ void __launch_bounds__(256) glb_gather_kernel(const bwacuda_global_job *__restrict__ hj, uint32_t n,
+// The slices of alignments order[base .. base + count), one class of the chunk (or all), into HBM: a warp
+// takes 32 of them, completes their descriptors (the plan left the slice addresses in q_off / t_off,
+// so the caller's job array crosses the host link once) and copies the slices as aligned 16-byte
+// words (warp_gather_slices).
+__global__ void __launch_bounds__(256) glb_gather_kernel(const uint32_t *__restrict__ order, uint32_t base, uint32_t count,
                                                          const uint64_t *__restrict__ seq_off,
                                                          const uint64_t *__restrict__ cig_off,
                                                          const uint64_t *__restrict__ z_off,
                                                          uint8_t *__restrict__ seq, GlobalDevJob *__restrict__ dj)
 {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t ngroups = (n + 31) / 32;
+    const uint32_t ngroups = (count + 31) / 32;
     for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ngroups; g += (gridDim.x * blockDim.x) >> 5) {
-        const uint32_t k = g * 32 + lane;
-        uint64_t qa = 0, ta = 0, base = 0;
+        const uint32_t x = g * 32 + lane;
+        uint64_t qa = 0, ta = 0, at = 0;
         uint32_t qw = 0, tw = 0;
-        if (k < n) {
-            const bwacuda_global_job J = hj[k];
-            const bool ok = gjob_ok(J);
-            const int ql = ok ? J.qlen : 0, tl = ok ? J.tlen : 0;
-            base = seq_off[k];
-            qa = reinterpret_cast<uint64_t>(J.query);
-            ta = reinterpret_cast<uint64_t>(J.target);
-            qw = slice_words(J.query, ql);
-            tw = slice_words(J.target, tl);
-            GlobalDevJob D;
-            D.q_off = base + (qa & 15);
-            D.t_off = base + 16ull * qw + (ta & 15);
+        if (x < count) {
+            const uint32_t k = order[base + x];
+            GlobalDevJob D = dj[k];
+            at = seq_off[k];
+            qa = D.q_off;
+            ta = D.t_off;
+            qw = slice_words(reinterpret_cast<const uint8_t *>(qa), D.qlen);
+            tw = slice_words(reinterpret_cast<const uint8_t *>(ta), D.tlen);
+            D.q_off = at + (qa & 15);
+            D.t_off = at + 16ull * qw + (ta & 15);
             D.z_off = z_off[k];
             D.cig_off = cig_off[k];
-            D.qlen = ql;
-            D.tlen = tl;
-            D.w = J.w;
-            D.zrow = global_zrow(ql, J.w);
             dj[k] = D;
         }
-        warp_gather_slices(qa & ~15ull, ta & ~15ull, base, qw, tw, seq);
+        warp_gather_slices<false>(qa & ~15ull, ta & ~15ull, at, qw, tw, seq);
     }
 }
 
@@ -1211,7 +1217,13 @@ struct GlobalState {
     cudaError_t init_streams()
     {
         cudaError_t e = cudaSuccess;
-        if (!ready) e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+        if (!ready) {
+            // it runs beside the DP kernels, and an SM keeps the shared-memory split of the first kernel
+            // placed on it while empty
+            e = cudaFuncSetAttribute(glb_gather_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     cudaSharedmemCarveoutMaxShared);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+        }
         for (int x = 0; x < NSIDE && e == cudaSuccess; ++x) {
             if (!side[x]) e = cudaStreamCreateWithFlags(&side[x], cudaStreamNonBlocking);
             if (e == cudaSuccess && !done[x]) e = cudaEventCreateWithFlags(&done[x], cudaEventDisableTiming);
@@ -1309,8 +1321,10 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         if ((e = cudaMemsetAsync(cig_sz + cn, 0, 8, s)) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(z_sz + cn, 0, 8, s)) != cudaSuccess) break;
         uint32_t grid = (uint32_t)std::min<size_t>((cn + 255) / 256, (size_t)nsm * 8);
+        if ((e = b.d_jobs.ensure(cn * sizeof(GlobalDevJob))) != cudaSuccess) break;
+        GlobalDevJob *dj = static_cast<GlobalDevJob *>(b.d_jobs.p);
         glb_plan_kernel<<<grid, 256, 0, s>>>(hj, (uint32_t)cn, qlim, nrule, trule, seq_sz, cig_sz, z_sz, keys, idx, flags,
-                                             bstat, bwide, dims);
+                                             bstat, bwide, dims, dj);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, seq_sz, seq_off, (int)cn + 1, s)) != cudaSuccess) break;
         if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, cig_sz, cig_off, (int)cn + 1, s)) != cudaSuccess) break;
@@ -1348,44 +1362,63 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         if ((e = b.d_cig.ensure(ht[1] * 4 + 16)) != cudaSuccess) break;
         if ((e = b.d_z.ensure(ht[2] + 16)) != cudaSuccess) break;
         if ((e = b.d_tz.ensure(ht[3] + 16)) != cudaSuccess) break;
-        if ((e = b.d_jobs.ensure(cn * sizeof(GlobalDevJob))) != cudaSuccess) break;
         if ((e = b.d_res.ensure((cn + 1) * 8 + 16)) != cudaSuccess) break;
         if ((e = b.d_doff.ensure((cn + 1) * 8)) != cudaSuccess) break;
-        GlobalDevJob *dj = static_cast<GlobalDevJob *>(b.d_jobs.p);
-        glb_gather_kernel<<<grid, 256, 0, s>>>(hj, (uint32_t)cn, seq_off, cig_off, z_off,
-                                              static_cast<uint8_t *>(b.d_seq.p), dj);
-        if ((e = cudaGetLastError()) != cudaSuccess) break;
         int32_t *d_score = static_cast<int32_t *>(b.d_res.p);
         int32_t *d_ncig = d_score + cn + 1;
         uint64_t *d_doff = static_cast<uint64_t *>(b.d_doff.p);
         if ((e = cudaMemsetAsync(d_ncig + cn, 0, 4, s)) != cudaSuccess) break;
-        // one DP launch per non-empty length bucket, sized by the bucket's own maxima, longest
-        // queries first, round-robin over the context's stream and the side streams so a
-        // bucket's blocks fill the last partial wave of the ones before it; the tracebacks
-        // follow all of them
+        // class after class, longest queries first: the class's gather on the context's stream (the
+        // gathers follow one another on the host link), then its DP, sized by the class's own maxima,
+        // and its traceback on one of the side streams, so the later gathers run beside the DP and a
+        // class's blocks fill the last partial wave of the ones before it: 500,000 alignments of 100,
+        // 150 and 250 bases 4.34 ms with one gather in front and the tracebacks behind, 3.76 so; 200,000
+        // 2.20 and 2.03.  Below a warp of alignments per SM the gathers are launches, not link time:
+        // one for all classes, in the caller's order (2,000: 0.725 ms against 0.738).
         const uint32_t *hb = hf + 16, *hbd = hf + 48, *hbw = hf + 80;
         uint32_t gfirst[GLB_NBUCKETS + 1] = {0};  // first warp group of each tagged class
         for (int bk = 0; bk < GLB_NBUCKETS; ++bk)
             gfirst[bk + 1] = gfirst[bk] + (hbd[2 * bk + 1] - hbd[2 * bk] + 63u) / 64u;
-        if ((e = cudaEventRecord(G.ready, s)) != cudaSuccess) break;
-        for (int x = 0; x < GlobalState::NSIDE && e == cudaSuccess; ++x) e = cudaStreamWaitEvent(G.side[x], G.ready, 0);
-        if (e != cudaSuccess) break;
         int nl = 0;
         for (int bk = GLB_NCLASSES - 1; bk >= 0 && e == cudaSuccess; --bk) {
-            const uint32_t b0 = hbd[2 * bk], b1 = hbd[2 * bk + 1];
+            const uint32_t b0 = hbd[2 * bk], b1 = hbd[2 * bk + 1], cnt = b1 - b0;
             if (b1 <= b0) continue;
-            cudaStream_t bs = nl % (GlobalState::NSIDE + 1) ? G.side[nl % (GlobalState::NSIDE + 1) - 1] : s;
+            cudaStream_t bs = G.side[nl % GlobalState::NSIDE];
+            if (trule.single && nl % (GlobalState::NSIDE + 1) == 0) bs = s;
             const uint8_t *sq = static_cast<const uint8_t *>(b.d_seq.p);
-            if (bk < GLB_NBUCKETS)
-                e = launch_tag(sq, dj, order, b0, b1 - b0, sc, trule, (int)hbw[bk], (int)hb[2 * bk], (int)hb[2 * bk + 1],
+            if (nl == 0 || !trule.single) {
+                // beside the DP, a small block for every other SM, as in the extension's pipeline
+                const uint32_t g0 = trule.single ? 0u : b0, gn = trule.single ? (uint32_t)cn : cnt;
+                const int tb = nl ? 128 : 256;
+                const size_t most = nl ? ((size_t)nsm + 1) / 2 : (size_t)nsm * 8;
+                glb_gather_kernel<<<(uint32_t)std::min<size_t>((gn + tb - 1) / tb, most), tb, 0, s>>>(
+                    trule.single ? idx : order, g0, gn, seq_off, cig_off, z_off, static_cast<uint8_t *>(b.d_seq.p), dj);
+                if ((e = cudaGetLastError()) != cudaSuccess) break;
+                c->stats.kernel_launches += 1;
+            }
+            if ((nl == 0 || !trule.single) && (e = cudaEventRecord(G.ready, s)) != cudaSuccess) break;
+            if (bs != s && (e = cudaStreamWaitEvent(bs, G.ready, 0)) != cudaSuccess) break;
+            if (bk < GLB_NBUCKETS) {
+                e = launch_tag(sq, dj, order, b0, cnt, sc, trule, (int)hbw[bk], (int)hb[2 * bk], (int)hb[2 * bk + 1],
                                wgroups, gfirst[bk], static_cast<uint8_t *>(b.d_tz.p), d_score, d_ncig, d_err, d_cells,
                                bs);
-            else
-                e = launch_global(sq, dj, order, b0, b1 - b0, sc, (int)hb[2 * bk], (int)hb[2 * bk + 1], hbw[bk] == 0u,
+                if (e != cudaSuccess) break;
+                const uint32_t ng = gfirst[bk + 1] - gfirst[bk];
+                glb_tag_traceback_kernel<<<(uint32_t)std::min<size_t>(((size_t)ng * 64 + 255) / 256, (size_t)nsm * 8), 256,
+                                           0, bs>>>(dj, order, wgroups + gfirst[bk], ng, trule,
+                                                    static_cast<const uint8_t *>(b.d_tz.p),
+                                                    static_cast<uint32_t *>(b.d_cig.p), d_ncig);
+                e = cudaGetLastError();
+            } else {
+                e = launch_global(sq, dj, order, b0, cnt, sc, (int)hb[2 * bk], (int)hb[2 * bk + 1], hbw[bk] == 0u,
                                   static_cast<uint8_t *>(b.d_z.p), static_cast<uint32_t *>(b.d_cig.p), d_score, d_ncig,
                                   d_err, d_cells, bs);
+                if (e == cudaSuccess)
+                    e = launch_global_traceback(dj, order, b0, cnt, static_cast<const uint8_t *>(b.d_z.p),
+                                                static_cast<uint32_t *>(b.d_cig.p), d_ncig, d_err, nsm, bs);
+            }
             ++nl;
-            c->stats.kernel_launches += 1;
+            c->stats.kernel_launches += 2;
         }
         for (int x = 0; x < GlobalState::NSIDE && e == cudaSuccess; ++x) {
             e = cudaEventRecord(G.done[x], G.side[x]);
@@ -1395,18 +1428,6 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
             for (int x = 0; x < GlobalState::NSIDE; ++x) cudaStreamSynchronize(G.side[x]);  // nothing runs on
             break;
         }
-        const uint32_t ntag = hbd[2 * GLB_NBUCKETS];  // the tagged classes sort first
-        if (ntag) {
-            const uint32_t ng = gfirst[GLB_NBUCKETS];
-            glb_tag_traceback_kernel<<<(uint32_t)std::min<size_t>(((size_t)ng * 64 + 255) / 256, (size_t)nsm * 8), 256, 0,
-                                       s>>>(dj, order, wgroups, ng, trule, static_cast<const uint8_t *>(b.d_tz.p),
-                                            static_cast<uint32_t *>(b.d_cig.p), d_ncig);
-            if ((e = cudaGetLastError()) != cudaSuccess) break;
-        }
-        if (ntag < cn &&
-            (e = launch_global_traceback(dj, order, ntag, (uint32_t)cn - ntag, static_cast<const uint8_t *>(b.d_z.p),
-                                         static_cast<uint32_t *>(b.d_cig.p), d_ncig, d_err, nsm, s)) != cudaSuccess)
-            break;
         if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t2, d_ncig, d_doff, (int)cn + 1, s)) != cudaSuccess) break;
         grid = (uint32_t)std::min<size_t>((cn + 255) / 256, (size_t)nsm * 8);
         glb_store_kernel<<<grid, 256, 0, s>>>(dj, (uint32_t)cn, d_score, static_cast<const uint32_t *>(b.d_cig.p), d_ncig,
@@ -1416,7 +1437,7 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) break;
         if (!cigar || out_base + ht[100] > cigar_cap) short_buf = true;
         out_base += ht[100];
-        c->stats.kernel_launches += 14;
+        c->stats.kernel_launches += 12;
     }
     if (e != cudaSuccess) return cuda_status(e);
     if (rc) {
