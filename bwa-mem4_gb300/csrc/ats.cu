@@ -295,7 +295,7 @@ cudaError_t ats_gather_chunk(bwacuda_ctx *c, AtsChunk &R, size_t cn, int w, bool
 
 // Steps 4-5 on extension stream s: the batched extension once the gather is in,
 // then the results into the caller's out[] and the flags back to the host.
-cudaError_t ats_extend_chunk(bwacuda_ctx *c, AtsChunk &R, int si, size_t cn, const ExtParams &P,
+cudaError_t ats_extend_chunk(bwacuda_ctx *c, AtsChunk &R, int si, size_t cn, size_t n, const ExtParams &P,
                              bwacuda_ext_result *hout)
 {
     cudaStream_t s = c->slot[si].stream;
@@ -303,9 +303,11 @@ cudaError_t ats_extend_chunk(bwacuda_ctx *c, AtsChunk &R, int si, size_t cn, con
     if ((e = cudaStreamWaitEvent(s, R.gathered, 0)) != cudaSuccess) return e;
     BatchBufs *bb = batched_slot_bufs(c, si);
     batched_set_reserve(bb, ATS_RESERVE_REGS, ATS_RESERVE_THREADS);
+    batched_set_call(bb, n);
     e = batched_enqueue(c, bb, static_cast<const uint8_t *>(R.seq.p), static_cast<const bwacuda_dev_ext_job *>(R.djobs.p),
                         cn, P, static_cast<bwacuda_ext_result *>(R.dout.p), s, nullptr, nullptr);
     batched_set_reserve(bb, 0, 0);
+    batched_set_call(bb, 0);
     if (e != cudaSuccess) return e;
     const uint32_t words = (uint32_t)(cn * (sizeof(bwacuda_ext_result) / 4));
     const uint32_t grid = ats_grid(words, batched_nsm(c), true);
@@ -438,7 +440,7 @@ int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int 
         cn = chunk_len(k, c0);
         AtsChunk &R = c->ats->ring[k % ATS_RING];
         cudaError_t e = ats_gather_chunk(c, R, cn, w, k == 0);
-        if (e == cudaSuccess) e = ats_extend_chunk(c, R, (int)(k & 1), cn, P, out + c0);
+        if (e == cudaSuccess) e = ats_extend_chunk(c, R, (int)(k & 1), cn, n, P, out + c0);
         if (e != cudaSuccess) {
             rc = cuda_status(e);
             break;

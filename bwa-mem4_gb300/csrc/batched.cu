@@ -16,7 +16,16 @@
 
 namespace bwacuda {
 
-constexpr int FAN = 4;  // bucket streams
+// Bucket streams: FAN, or FAN_WIDE for calls below EXT_WIDE_JOBS_PER_SM jobs per SM.  There a bucket's
+// time is its longest jobs' and it leaves most of an SM free, so the eight length classes run at once;
+// above, the buckets fill the GPU one after another, and the long ones finish later when they share it
+// from the start.  Device-resident, four streams / eight, microseconds, mixed lengths: 60,000 jobs
+// 2010 / 1240, 120,000 1970 / 1310, 250,000 2110 / 1870, 500,000 2500 / 2770, 1M 3840 / 4340; read
+// pairs: 250,000 1260 / 1120.  The others are created at their first use: every stream of a process
+// takes a place in the few hardware queues, and 2M read pairs through host buffers took 3% longer with
+// eight created and four in use.
+constexpr int FAN = 4, FAN_WIDE = 8;
+constexpr int EXT_WIDE_JOBS_PER_SM = 2200;
 // Open-ended buckets: jobs per SM from which the band kernel gives a job 8 lanes, below it 32 (queries
 // of 2-10 kb on 152 SMs: 1,000 jobs 9.6 / 6.5 ms, 2,400 jobs 9.8 / 9.8, 20,000 jobs 23.1 / 42.4).
 constexpr int BAND_LANES8_JOBS = 14;
@@ -34,8 +43,8 @@ constexpr int EXT_DUAL_QCAP = 129;
 struct BatchBufs {
     DevBuf keys_in, keys_out, idx_in, idx_out, tmp, table;
     DevBuf xl;  // group-per-job buckets: work words and the deferred-job list
-    cudaStream_t fan[FAN] = {};
-    cudaEvent_t fork = nullptr, join[FAN] = {};
+    cudaStream_t fan[FAN_WIDE] = {};
+    cudaEvent_t fork = nullptr, join[FAN_WIDE] = {};
     // graph cache for device-resident replays
     cudaGraphExec_t graph = nullptr;
     const void *g_seq = nullptr, *g_jobs = nullptr, *g_out = nullptr;
@@ -44,6 +53,8 @@ struct BatchBufs {
     size_t g_n = 0;
     cudaStream_t g_stream = nullptr;
     ExtParams g_P{};
+    int nfan = 0;            // streams and join events that exist
+    size_t call_jobs = 0;    // jobs of the whole call when the batch is one chunk of it
     // per-SM room the bucket kernels leave for kernels running beside them
     int reserve_regs = 0, reserve_threads = 0;
     size_t jobs_cap = 0;  // jobs the work buffers are sized for (batched_enqueue, batched_reserve)
@@ -73,6 +84,18 @@ struct BatchedState {
     BatchBufs bufs[3];  // [0], [1]: host-pipeline slots; [2]: device-resident calls
 };
 
+// The first `fan` bucket streams and their join events.
+static cudaError_t fan_streams(BatchBufs &bb, int fan)
+{
+    for (; bb.nfan < fan; ++bb.nfan) {
+        const int f = bb.nfan;
+        cudaError_t e = bb.fan[f] ? cudaSuccess : cudaStreamCreateWithFlags(&bb.fan[f], cudaStreamNonBlocking);
+        if (e == cudaSuccess && !bb.join[f]) e = cudaEventCreateWithFlags(&bb.join[f], cudaEventDisableTiming);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 static int batched_init(bwacuda_ctx *c)
 {
     if (c->batched) return BWACUDA_OK;
@@ -91,10 +114,7 @@ static int batched_init(bwacuda_ctx *c)
         return cuda_status(e);
     }
     for (auto &bb : B->bufs) {
-        for (int f = 0; f < FAN; ++f) {
-            if ((e = cudaStreamCreateWithFlags(&bb.fan[f], cudaStreamNonBlocking)) != cudaSuccess) break;
-            if ((e = cudaEventCreateWithFlags(&bb.join[f], cudaEventDisableTiming)) != cudaSuccess) break;
-        }
+        e = fan_streams(bb, FAN);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&bb.fork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = bb.table.ensure(EXT_MAX_BUCKETS * 4 * sizeof(uint32_t));
         if (e != cudaSuccess) break;
@@ -109,10 +129,10 @@ void batched_release(bwacuda_ctx *c)
     if (!B) return;
     for (auto &bb : B->bufs) {
         if (bb.graph) cudaGraphExecDestroy(bb.graph);
-        for (int f = 0; f < FAN; ++f) {
+        for (int f = 0; f < FAN_WIDE; ++f) {
             if (bb.fan[f]) cudaStreamSynchronize(bb.fan[f]);
         }
-        for (int f = 0; f < FAN; ++f) {
+        for (int f = 0; f < FAN_WIDE; ++f) {
             if (bb.fan[f]) cudaStreamDestroy(bb.fan[f]);
             if (bb.join[f]) cudaEventDestroy(bb.join[f]);
         }
@@ -225,9 +245,16 @@ void batched_get_tuning(bwacuda_ctx *c, int *tb, int *grab, int *step)
     *step = B ? B->step : 32;
 }
 
-static cudaError_t ensure_bufs(BatchBufs &bb, size_t n)
+// Bucket streams of a batch of n jobs.
+static int batched_fan(const bwacuda_ctx *c, const BatchBufs &bb, size_t n)
+{
+    return std::max(n, bb.call_jobs) < (size_t)c->batched->nsm * EXT_WIDE_JOBS_PER_SM ? FAN_WIDE : FAN;
+}
+
+static cudaError_t ensure_bufs(BatchBufs &bb, size_t n, int fan = FAN)
 {
     cudaError_t e;
+    if ((e = fan_streams(bb, fan)) != cudaSuccess) return e;
     if ((e = bb.keys_in.ensure(n * 4 + 16)) != cudaSuccess) return e;
     if ((e = bb.keys_out.ensure(n * 4 + 16)) != cudaSuccess) return e;
     if ((e = bb.idx_in.ensure(n * 4 + 16)) != cudaSuccess) return e;
@@ -305,6 +332,7 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
     BatchedState *B = c->batched;
     const bool lanes = ext_pair_lanes_ok(P.sc.o_del, P.sc.e_del, P.sc.o_ins, P.sc.e_ins);
     if (lanes && batched_is_small(c, n, P)) return enqueue_small(c, bb, d_seq, d_jobs, n, P, d_out, s, err, cells);
+    const int fan = std::min(batched_fan(c, bb, n), bb.nfan);
     // two jobs a thread in the 8-bit buckets of large batches
     const bool dual = lanes && P.sc.m <= 5 && n >= (size_t)B->nsm * EXT_DUAL_JOBS_PER_SM;
     cudaError_t e = ext_sort_and_bucket(d_jobs, n, P.sc.max_sc, lanes, dual, d_seq, P.ug, P.zdrop, d_out,
@@ -317,7 +345,7 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
     uint32_t *work = static_cast<uint32_t *>(bb.xl.p);
     if ((e = cudaMemsetAsync(work, 0, XL_WORK_WORDS * 4, s)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(bb.fork, s)) != cudaSuccess) return e;
-    for (int f = 0; f < FAN; ++f)
+    for (int f = 0; f < fan; ++f)
         if ((e = cudaStreamWaitEvent(bb.fan[f], bb.fork, 0)) != cudaSuccess) return e;
     // Group-per-job buckets (the open-ended ones take queries of any length) one after
     // another on the first stream, then the deferred launches over the jobs whose bands
@@ -380,13 +408,13 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
     // thread-per-job buckets, largest first: they hold the long jobs
     for (int b = B->nb - 1, k = 1; b >= 0; --b) {
         if (B->defs[b].kernel == 1) continue;
-        L.stream = bb.fan[k++ % FAN];
+        L.stream = bb.fan[k++ % fan];
         uint32_t *tab = static_cast<uint32_t *>(bb.table.p) + 4 * b;
         e = dual && B->defs[b].cls == 0 && B->defs[b].qcap <= EXT_DUAL_QCAP ? ext_dual_launch(L, B->defs[b], tab, B->nsm)
                                         : ext_persist_launch(L, B->defs[b], tab, B->nsm, B->tb);
         if (e != cudaSuccess) return e;
     }
-    for (int f = 0; f < FAN; ++f) {
+    for (int f = 0; f < fan; ++f) {
         if ((e = cudaEventRecord(bb.join[f], bb.fan[f])) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(s, bb.join[f], 0)) != cudaSuccess) return e;
     }
@@ -399,7 +427,7 @@ int extend_device_batched(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda_de
     int rc = batched_init(c);
     if (rc) return rc;
     BatchBufs &bb = c->batched->bufs[2];
-    cudaError_t e = ensure_bufs(bb, n);
+    cudaError_t e = ensure_bufs(bb, n, batched_fan(c, bb, n));
     if (e != cudaSuccess) return cuda_status(e);
     // Replay a captured graph when the same batch comes back (same buffers, size,
     // scoring and stream); otherwise capture a new one.
@@ -442,6 +470,7 @@ void batched_set_reserve(BatchBufs *bb, int regs, int threads)
     bb->reserve_regs = regs;
     bb->reserve_threads = threads;
 }
+void batched_set_call(BatchBufs *bb, size_t jobs) { bb->call_jobs = jobs; }
 BatchBufs *batched_slot_bufs(bwacuda_ctx *c, int slot) { return &c->batched->bufs[slot & 1]; }
 int batched_nsm(bwacuda_ctx *c) { return c->batched->nsm; }
 // Launches of the bucket stage: one per bucket and the two deferred group-per-job launches.
@@ -449,11 +478,7 @@ int batched_bucket_count(bwacuda_ctx *c) { return c->batched->nb + 2 + (c->long_
 
 static cudaError_t bufs_streams(BatchBufs &bb)
 {
-    cudaError_t e = cudaSuccess;
-    for (int f = 0; f < FAN && e == cudaSuccess; ++f) {
-        e = cudaStreamCreateWithFlags(&bb.fan[f], cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&bb.join[f], cudaEventDisableTiming);
-    }
+    cudaError_t e = fan_streams(bb, FAN);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&bb.fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = bb.table.ensure(EXT_MAX_BUCKETS * 4 * sizeof(uint32_t));
     return e;
@@ -473,7 +498,7 @@ BatchBufs *batchbufs_create()
 void batchbufs_destroy(BatchBufs *bb)
 {
     if (!bb) return;
-    for (int f = 0; f < FAN; ++f) {
+    for (int f = 0; f < FAN_WIDE; ++f) {
         if (bb->fan[f]) cudaStreamSynchronize(bb->fan[f]);
         if (bb->fan[f]) cudaStreamDestroy(bb->fan[f]);
         if (bb->join[f]) cudaEventDestroy(bb->join[f]);
@@ -490,7 +515,7 @@ cudaError_t batched_enqueue(bwacuda_ctx *c, BatchBufs *bb, const uint8_t *d_seq,
                             size_t n, const ExtParams &P, bwacuda_ext_result *d_out, cudaStream_t s, uint32_t *err,
                             unsigned long long *cells)
 {
-    cudaError_t e = ensure_bufs(*bb, batched_grow_jobs(*bb, n));
+    cudaError_t e = ensure_bufs(*bb, batched_grow_jobs(*bb, n), batched_fan(c, *bb, n));
     if (e != cudaSuccess) return e;
     return enqueue_batched(c, *bb, d_seq, d_jobs, n, P, d_out, s, err, cells);
 }
@@ -511,7 +536,7 @@ int extend_batch_host_batched(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_
     if (rc) return rc;
     return extend_host_pipeline(c, jobs, n, m, mat, P, w, out, [c](int slot, const ExtChunkInfo &I, cudaStream_t s) {
         BatchBufs &bb = c->batched->bufs[slot];
-        cudaError_t e = ensure_bufs(bb, I.n);
+        cudaError_t e = ensure_bufs(bb, I.n, batched_fan(c, bb, I.n));
         if (e == cudaSuccess) e = enqueue_batched(c, bb, I.d_seq, I.d_jobs, I.n, I.P, I.d_out, s);
         c->stats.kernel_launches += 3 + (uint64_t)batched_bucket_count(c);
         return cuda_status(e);

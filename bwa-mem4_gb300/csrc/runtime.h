@@ -164,6 +164,7 @@ void batchbufs_destroy(BatchBufs *bb);
 cudaError_t batched_enqueue(bwacuda_ctx *c, BatchBufs *bb, const uint8_t *d_seq, const bwacuda_dev_ext_job *d_jobs,
                             size_t n, const ExtParams &P, bwacuda_ext_result *d_out, cudaStream_t s, uint32_t *err,
                             unsigned long long *cells);
+void batched_set_call(BatchBufs *bb, size_t jobs);  // jobs of the call whose chunks follow (0: batches by themselves)
 BatchBufs *batched_slot_bufs(bwacuda_ctx *c, int slot);  // work buffers of host-pipeline slot 0 or 1
 cudaError_t batched_reserve(BatchBufs *bb, size_t n);
 // registers / threads per SM that bb's bucket kernels leave free (0, 0: none)
