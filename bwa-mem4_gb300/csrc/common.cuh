@@ -110,12 +110,34 @@ __host__ __device__ inline uint32_t slice_words(const uint8_t *src, int len)
 // is stored at seq + base_0 + 16 x.  All 32 lanes must call it, and lane 0 must
 // carry a job (possibly empty).  CONSECUTIVE false: any 16-byte aligned bases, each
 // lane's own (two more shuffles a word).
-template <bool CONSECUTIVE = true>
-__device__ __forceinline__ void warp_gather_slices(uint64_t qa, uint64_t ta, uint64_t base, uint32_t qw, uint32_t tw,
-                                                   uint8_t *seq)
+// CHECK: whether a byte of this lane's words that lies in a slice is m or more (m at most 256), from
+// the registers on their way through: ends = slice_ends of the lane's job.
+__device__ __forceinline__ uint32_t slice_ends(uint64_t q, int qlen, uint64_t t, int tlen)
+{
+    return (uint32_t)(q & 15) | (uint32_t)((q + (uint64_t)qlen - 1) & 15) << 4 | (uint32_t)(t & 15) << 8 |
+           (uint32_t)((t + (uint64_t)tlen - 1) & 15) << 12;
+}
+// Whether one of the bytes lo .. hi of v is above those of top.
+__device__ __forceinline__ bool word_above(const uint4 &v, uint32_t lo, uint32_t hi, uint32_t top)
+{
+    const uint32_t in = (0xffffu << lo) & (0xffffu >> (15u - hi));  // a bit a byte
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    bool above = false;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const uint32_t keep = ((in >> (4 * c) & 15u) * 0x00204081u & 0x01010101u) * 0xffu;
+        above |= __vmaxu4(w[c] & keep, top) != top;
+    }
+    return above;
+}
+template <bool CONSECUTIVE = true, bool CHECK = false>
+__device__ __forceinline__ bool warp_gather_slices(uint64_t qa, uint64_t ta, uint64_t base, uint32_t qw, uint32_t tw,
+                                                   uint8_t *seq, uint32_t ends = 0u, uint32_t m = 256u)
 {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t wc = qw + tw;
+    const uint32_t top = (m - 1u) * 0x01010101u;
+    bool bad = false;
     uint32_t pre = wc;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -128,7 +150,8 @@ __device__ __forceinline__ void warp_gather_slices(uint64_t qa, uint64_t ta, uin
     constexpr int U = 8;
     for (uint32_t x0 = 0; x0 < total; x0 += 32u * U) {
         uint4 v[U];
-        uint64_t at[U];  // CONSECUTIVE false: destinations
+        uint64_t at[U];       // CONSECUTIVE false: destinations
+        uint64_t bounds = 0;  // CHECK: first and last byte of the slice in each word, 4 bits each
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint32_t x = x0 + (uint32_t)u * 32u + lane;
@@ -144,6 +167,15 @@ __device__ __forceinline__ void warp_gather_slices(uint64_t qa, uint64_t ta, uin
             const uint64_t ta_j = __shfl_sync(0xffffffffu, ta, j);
             const uint32_t wi = x - pre_j;
             if constexpr (!CONSECUTIVE) at[u] = __shfl_sync(0xffffffffu, base, j) + 16ull * wi;
+            if constexpr (CHECK) {
+                const uint32_t wc_j = __shfl_sync(0xffffffffu, wc, j);
+                uint32_t e_j = __shfl_sync(0xffffffffu, ends, j);
+                const bool isq = wi < qw_j;
+                e_j = isq ? e_j & 0xffu : e_j >> 8;
+                const uint32_t lo = wi == 0u || wi == qw_j ? e_j & 15u : 0u;
+                const uint32_t hi = wi + 1u == (isq ? qw_j : wc_j) ? e_j >> 4 : 15u;
+                bounds |= (uint64_t)(lo | hi << 4) << (8 * u);
+            }
             if (x < total)
                 v[u] = wi < qw_j ? reinterpret_cast<const uint4 *>(qa_j)[wi]
                                  : reinterpret_cast<const uint4 *>(ta_j)[wi - qw_j];
@@ -154,9 +186,14 @@ __device__ __forceinline__ void warp_gather_slices(uint64_t qa, uint64_t ta, uin
             if (x < total) {
                 if constexpr (CONSECUTIVE) dst[x] = v[u];
                 else *reinterpret_cast<uint4 *>(seq + at[u]) = v[u];
+                if constexpr (CHECK) {
+                    const uint32_t b = (uint32_t)(bounds >> (8 * u));
+                    bad |= word_above(v[u], b & 15u, b >> 4 & 15u, top);
+                }
             }
         }
     }
+    return bad;
 }
 #endif
 
