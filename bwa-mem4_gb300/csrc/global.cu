@@ -1114,8 +1114,10 @@ cudaError_t launch_tag_tb(const uint8_t *seq, const GlobalDevJob *jobs, const ui
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT - 1024);
     if (e != cudaSuccess) return e;
     const uint32_t threads = tr.single ? count : (count + 1) / 2;
-    kern<<<(threads + TB - 1) / TB, TB, smem, s>>>(seq, jobs, order, start, count, sc, tr, max_slots, max_sel, groups,
-                                                  gbase, z, score, ncig, GLB_TB_TAGGED, ERR_RANGE, err, cells);
+    const uint32_t blocks = (threads + TB - 1) / TB;
+    kern<<<tr.single ? blocks : 2 * blocks, TB, smem, s>>>(seq, jobs, order, start, count, sc, tr, max_slots, max_sel,
+                                                          groups, gbase, z, score, ncig, GLB_TB_TAGGED, ERR_RANGE, err,
+                                                          cells);
     return cudaGetLastError();
 }
 
@@ -1288,8 +1290,9 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
     for (size_t c0 = 0, cn = 0; c0 < n && rc == BWACUDA_OK; c0 += cn) {
         cn = std::min(chunk, n - c0);
         const bwacuda_global_job *hj = jobs + c0;
-        // one alignment a thread below a warp of them per SM: 300 alignments in 0.82 ms against 1.21 in
-        // pairs, of which some always differ and take two passes
+        // one alignment a thread below a warp of them per SM: 2,000 alignments 0.73 ms against 0.76 in
+        // pairs.  From there to 20,000 the two are within 4% (9,000 0.80 / 0.815, 18,000 0.84 / 0.855),
+        // then pairs lead: 28,000 0.93 / 0.885, 80,000 1.39 / 1.06
         trule.single = cn < (size_t)nsm * 32;
         // planning arrays: seq / cig / z sizes and offsets (cn + 1 each), keys and indices (two
         // copies each for the sort)
@@ -1373,8 +1376,8 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         // and its traceback on one of the side streams, so the later gathers run beside the DP and a
         // class's blocks fill the last partial wave of the ones before it: 500,000 alignments of 100,
         // 150 and 250 bases 4.34 ms with one gather in front and the tracebacks behind, 3.76 so; 200,000
-        // 2.20 and 2.03.  Below a warp of alignments per SM the gathers are launches, not link time:
-        // one for all classes, in the caller's order (2,000: 0.725 ms against 0.738).
+        // 2.20 and 2.03.  In single mode the gathers are launches, not link time: one for all
+        // classes, in the caller's order (2,000: 0.725 ms against 0.738).
         const uint32_t *hb = hf + 16, *hbd = hf + 48, *hbw = hf + 80;
         uint32_t gfirst[GLB_NBUCKETS + 1] = {0};  // first warp group of each tagged class
         for (int bk = 0; bk < GLB_NBUCKETS; ++bk)

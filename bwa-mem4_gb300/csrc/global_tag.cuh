@@ -54,7 +54,7 @@ struct TagRule {
     int ok, mn, mx, oe, e;  // mn = -min entry (>= 0), mx = max entry (>= 0), oe / e: the larger of the gaps'
     // 2, 4, 16 and -1: multipliers the compiler does not see, so that tag removal and direction nibbles
     // stay multiply-adds (as constants they become shifts and adds of the ALU pipe, which bounds this)
-    int single = 0;  // one alignment a thread (few alignments: a pair that does not match costs two passes)
+    int single = 0;  // one alignment a thread (batches that leave most SMs' slots empty)
     uint32_t k2 = 2u, k4 = 4u, k16 = 16u, km1 = 0xffffffffu;
 };
 
@@ -237,11 +237,13 @@ __device__ __forceinline__ void two_rows(uint2 *P, const uint8_t *S, int g0, int
     }
 }
 
-// The DP of sorted alignments [start, start + count): a thread takes positions 2t and 2t + 1 (one after
-// the other where they do not match), or in single mode one position; group gbase + t / 32 holds their
-// directions.  ncig[k] = done marks a finished alignment for the traceback.
+// The DP of sorted alignments [start, start + count): a thread takes positions 2t and 2t + 1, or in
+// single mode one position; group gbase + t / 32 holds their directions.  Where a pair does not match,
+// a thread of the grid's first half takes the second one (the others of that half leave at once): one
+// thread after the other doubled the latency of a small batch.  ncig[k] = done marks a finished alignment for the traceback.
 // Measured (GB300, 500,000 reads of 100 / 150 / 250 bp through host buffers): the call 8.08 -> 4.30 ms
-// against the predicate pair kernel.  About 40 instructions, 18 of them ALU, for a step's four cells;
+// against the predicate pair kernel; the grid's first half for the pairs that do not match: 14,000
+// alignments 1.32 -> 0.84 ms, 50,000 1.45 -> 1.00, 200,000 2.03 -> 1.74, 500,000 3.76 -> 3.65.  About 40 instructions, 18 of them ALU, for a step's four cells;
 // ALU pipe 43-57%, bound by the warps shared memory leaves (1.0 a scheduler at 250 bp, 1.7 at 150 bp).
 template <int TB, bool SYM, typename JobT>
 __global__ void __launch_bounds__(TB, 384 / TB)
@@ -264,7 +266,9 @@ tag_kernel(const uint8_t *__restrict__ seq, const JobT *__restrict__ jobs, const
         nt[t] = (uint32_t)(4 * (int)(int8_t)(sc.prof[t][1] & 0xffu) + 3) & 0xffffu;
     }
     __syncthreads();
-    const uint32_t tid = blockIdx.x * TB + threadIdx.x, t = rule.single ? tid >> 1 : tid;
+    const bool rest = !rule.single && blockIdx.x < gridDim.x / 2;
+    const uint32_t blk = rule.single || rest ? blockIdx.x : blockIdx.x - gridDim.x / 2;
+    const uint32_t tid = blk * TB + threadIdx.x, t = rule.single ? tid >> 1 : tid;
     if ((rule.single ? tid : 2 * t) >= count) return;
     uint2 *P = reinterpret_cast<uint2 *>(smem_raw) + TB + threadIdx.x;  // slot 0; slot -1 takes garbage
     uint8_t *S0 = reinterpret_cast<uint8_t *>(reinterpret_cast<uint2 *>(smem_raw) + (size_t)max_slots * TB) + threadIdx.x;
@@ -272,6 +276,7 @@ tag_kernel(const uint8_t *__restrict__ seq, const JobT *__restrict__ jobs, const
     const uint32_t k0 = order[start + 2 * t], k1 = has1 ? order[start + 2 * t + 1] : k0;
     const JobT A0 = jobs[k0], B0 = jobs[k1];
     const PairGeo first = pair_geo(A0.qlen, A0.tlen, A0.w, has1, B0.qlen, B0.tlen, B0.w, rule);
+    if (rest && (first.dual || !has1)) return;
     const WarpGroup wg = wgroups[gbase + (t >> 5)];
     uint4 *zw = reinterpret_cast<uint4 *>(z + wg.z_off) + (t & 31u);
     TagGaps gp;
@@ -285,96 +290,93 @@ tag_kernel(const uint8_t *__restrict__ seq, const JobT *__restrict__ jobs, const
     gp.km1 = rule.km1;
     unsigned long long ncells = 0;
     bool bad = false;
-    const int pass0 = rule.single ? (int)(tid & 1u) : 0;
-    const int passes = rule.single ? pass0 + 1 : (first.dual || !has1 ? 1 : 2);
-    for (int pass = pass0; pass < passes; ++pass) {
-        const uint32_t ka = pass ? k1 : k0, kb = first.dual ? k1 : ka;
-        const JobT A = pass ? B0 : A0, B = first.dual ? B0 : A;
-        const PairGeo g = first.dual ? first : pair_geo(A.qlen, A.tlen, A.w, false, A.qlen, A.tlen, A.w, rule);
-        const int Q = g.q, T = g.t, wl = g.wl, wr = g.wr, SN = steps(wl, wr);
-        if (slots(wl, wr) > max_slots || sel_count(Q, wl, wr) > max_sel || groups(wl, wr) > wg.ng) {
-            atomicOr(err, range_flag);  // the host sizes these from the launch's alignments
-            ncig_out[ka] = 0;
-            ncig_out[kb] = 0;
-            continue;
-        }
-        const uint8_t *qa = seq + A.q_off, *qb = seq + B.q_off;
-        bool slow = false;
-        for (int x = 0; x < LEFT_PAD; ++x) S0[x * TB] = (uint8_t)PAD_COLUMN;
-        for (int j = 0; j < Q + 16; j += 16) {
-            uint32_t va[4], vb[4];
-            load16(qa, A.qlen, j, va);
-            load16(qb, B.qlen, j, vb);
+    const int pass = rule.single ? (int)(tid & 1u) : (int)rest;
+    const uint32_t ka = pass ? k1 : k0, kb = first.dual ? k1 : ka;
+    const JobT A = pass ? B0 : A0, B = first.dual ? B0 : A;
+    const PairGeo g = first.dual ? first : pair_geo(A.qlen, A.tlen, A.w, false, A.qlen, A.tlen, A.w, rule);
+    const int Q = g.q, T = g.t, wl = g.wl, wr = g.wr, SN = steps(wl, wr);
+    if (slots(wl, wr) > max_slots || sel_count(Q, wl, wr) > max_sel || groups(wl, wr) > wg.ng) {
+        atomicOr(err, range_flag);  // the host sizes these from the launch's alignments
+        ncig_out[ka] = 0;
+        ncig_out[kb] = 0;
+        return;
+    }
+    const uint8_t *qa = seq + A.q_off, *qb = seq + B.q_off;
+    bool slow = false;
+    for (int x = 0; x < LEFT_PAD; ++x) S0[x * TB] = (uint8_t)PAD_COLUMN;
+    for (int j = 0; j < Q + 16; j += 16) {
+        uint32_t va[4], vb[4];
+        load16(qa, A.qlen, j, va);
+        load16(qb, B.qlen, j, vb);
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                const uint32_t ca = (va[u >> 2] >> (8 * (u & 3))) & 0xffu, cb = (vb[u >> 2] >> (8 * (u & 3))) & 0xffu;
-                bad |= ca >= (uint32_t)sc.m || cb >= (uint32_t)sc.m;
-                slow |= ca == 4u || cb == 4u;
-                if (j + u < Q + 16) S0[(LEFT_PAD + j + u) * TB] = (uint8_t)column_code(ca, cb);
-            }
+        for (int u = 0; u < 16; ++u) {
+            const uint32_t ca = (va[u >> 2] >> (8 * (u & 3))) & 0xffu, cb = (vb[u >> 2] >> (8 * (u & 3))) & 0xffu;
+            bad |= ca >= (uint32_t)sc.m || cb >= (uint32_t)sc.m;
+            slow |= ca == 4u || cb == 4u;
+            if (j + u < Q + 16) S0[(LEFT_PAD + j + u) * TB] = (uint8_t)column_code(ca, cb);
         }
-        // before row 0: H(-1, j - 1) and E(0, j - 1) at slot wl + j; column -1's E opens the leading
-        // deletion
-        const uint32_t neg_h = both(4 * NEG), neg_e = both(4 * NEG + 1);
-        const int ns = slots(wl, wr);
-        for (int b = -1; b < ns - 1; ++b) {
-            const int j = b - wl;
-            uint2 v = make_uint2(neg_h, neg_e);
-            if (j == 0) v = make_uint2(0u, both(-4 * (sc.o_del + sc.e_del) + 1));
-            else if (j > 0 && j <= wr) v.x = both(-4 * (sc.o_ins + sc.e_ins * j));
-            P[(ptrdiff_t)b * TB] = v;
-        }
-        TargetStream ta, tb;
-        ta.init(seq + A.t_off, A.tlen);
-        tb.init(seq + B.t_off, B.tlen);
-        int sa = 0, sb = 0;
-        for (int i = 0; i < T; i += 2) {
-            uint32_t c[4];
-#pragma unroll
-            for (int x = 0; x < 2; ++x) {
-                c[2 * x] = i + x < A.tlen ? ta.next() : 0u;
-                c[2 * x + 1] = i + x < B.tlen ? tb.next() : 0u;
-                bad |= c[2 * x] >= (uint32_t)sc.m || c[2 * x + 1] >= (uint32_t)sc.m;
-            }
-            const uint32_t pa0 = pt[c[0] & 7u], pb0 = pt[c[1] & 7u], pa1 = pt[c[2] & 7u], pb1 = pt[c[3] & 7u];
-            const int g0 = (wl - i - 1 > 0 ? wl - i - 1 : 0) >> 3;
-            const int last = min(SN - 1, Q - 1 - i + wl);
-            const int g1 = last >> 3;
-            const uint8_t *S = S0 + (ptrdiff_t)(8 * g0 + i - wl + LEFT_PAD) * TB;
-            uint4 *zr = zw + (size_t)(i >> 1) * wg.ng * 32;
-            const int ncomp = first.dual ? 2 : 1;
-            const bool fa = (A.tlen - 1) >> 1 == i >> 1, fb = (B.tlen - 1) >> 1 == i >> 1;
-            const int ca = fa ? A.qlen - 1 - i + wl : -1, cb = fb ? B.qlen - 1 - i + wl : -1;
-            const int ra = (A.tlen - 1) & 1, rb = (B.tlen - 1) & 1;
-            if (slow) {
-                const uint32_t n0 = nt[c[0] & 7u] | (nt[c[1] & 7u] << 16), n1 = nt[c[2] & 7u] | (nt[c[3] & 7u] << 16);
-                two_rows<TB, SYM, true, true>(P, S, g0, g1, gp, pa0, pb0, pa1, pb1, n0, n1, zr, ncomp, pass, ca, ra, cb,
-                                              rb, sa, sb);
-            } else if (fa || fb) {
-                two_rows<TB, SYM, false, true>(P, S, g0, g1, gp, pa0, pb0, pa1, pb1, 0u, 0u, zr, ncomp, pass, ca, ra, cb,
-                                               rb, sa, sb);
-            } else {
-                two_rows<TB, SYM, false, false>(P, S, g0, g1, gp, pa0, pb0, pa1, pb1, 0u, 0u, zr, ncomp, pass, -1, 0, -1,
-                                                0, sa, sb);
-            }
-            // nothing right of the band may pass an E back into it
-            P[(ptrdiff_t)(wl + wr + 1) * TB] = make_uint2(neg_h, neg_e);
-            P[(ptrdiff_t)(wl + wr + 2) * TB] = make_uint2(neg_h, neg_e);
-        }
-        score_out[ka] = sa;
-        ncig_out[ka] = done;
-        if (first.dual) {
-            score_out[kb] = sb;
-            ncig_out[kb] = done;
-        }
+    }
+    // before row 0: H(-1, j - 1) and E(0, j - 1) at slot wl + j; column -1's E opens the leading
+    // deletion
+    const uint32_t neg_h = both(4 * NEG), neg_e = both(4 * NEG + 1);
+    const int ns = slots(wl, wr);
+    for (int b = -1; b < ns - 1; ++b) {
+        const int j = b - wl;
+        uint2 v = make_uint2(neg_h, neg_e);
+        if (j == 0) v = make_uint2(0u, both(-4 * (sc.o_del + sc.e_del) + 1));
+        else if (j > 0 && j <= wr) v.x = both(-4 * (sc.o_ins + sc.e_ins * j));
+        P[(ptrdiff_t)b * TB] = v;
+    }
+    TargetStream ta, tb;
+    ta.init(seq + A.t_off, A.tlen);
+    tb.init(seq + B.t_off, B.tlen);
+    int sa = 0, sb = 0;
+    for (int i = 0; i < T; i += 2) {
+        uint32_t c[4];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
-            if (x == 1 && !first.dual) break;
-            // sum over rows of min(i + w + 1, qlen) - max(i - w, 0)
-            const long long q = x ? B.qlen : A.qlen, tl = x ? B.tlen : A.tlen, w = g.w;
-            const long long n1 = q - w < 0 ? 0 : (q - w < tl ? q - w : tl), lft = tl - 1 - w > 0 ? tl - 1 - w : 0;
-            ncells += (unsigned long long)(n1 * (w + 1) + n1 * (n1 - 1) / 2 + (tl - n1) * q - lft * (lft + 1) / 2);
+            c[2 * x] = i + x < A.tlen ? ta.next() : 0u;
+            c[2 * x + 1] = i + x < B.tlen ? tb.next() : 0u;
+            bad |= c[2 * x] >= (uint32_t)sc.m || c[2 * x + 1] >= (uint32_t)sc.m;
         }
+        const uint32_t pa0 = pt[c[0] & 7u], pb0 = pt[c[1] & 7u], pa1 = pt[c[2] & 7u], pb1 = pt[c[3] & 7u];
+        const int g0 = (wl - i - 1 > 0 ? wl - i - 1 : 0) >> 3;
+        const int last = min(SN - 1, Q - 1 - i + wl);
+        const int g1 = last >> 3;
+        const uint8_t *S = S0 + (ptrdiff_t)(8 * g0 + i - wl + LEFT_PAD) * TB;
+        uint4 *zr = zw + (size_t)(i >> 1) * wg.ng * 32;
+        const int ncomp = first.dual ? 2 : 1;
+        const bool fa = (A.tlen - 1) >> 1 == i >> 1, fb = (B.tlen - 1) >> 1 == i >> 1;
+        const int ca = fa ? A.qlen - 1 - i + wl : -1, cb = fb ? B.qlen - 1 - i + wl : -1;
+        const int ra = (A.tlen - 1) & 1, rb = (B.tlen - 1) & 1;
+        if (slow) {
+            const uint32_t n0 = nt[c[0] & 7u] | (nt[c[1] & 7u] << 16), n1 = nt[c[2] & 7u] | (nt[c[3] & 7u] << 16);
+            two_rows<TB, SYM, true, true>(P, S, g0, g1, gp, pa0, pb0, pa1, pb1, n0, n1, zr, ncomp, pass, ca, ra, cb,
+                                          rb, sa, sb);
+        } else if (fa || fb) {
+            two_rows<TB, SYM, false, true>(P, S, g0, g1, gp, pa0, pb0, pa1, pb1, 0u, 0u, zr, ncomp, pass, ca, ra, cb,
+                                           rb, sa, sb);
+        } else {
+            two_rows<TB, SYM, false, false>(P, S, g0, g1, gp, pa0, pb0, pa1, pb1, 0u, 0u, zr, ncomp, pass, -1, 0, -1,
+                                            0, sa, sb);
+        }
+        // nothing right of the band may pass an E back into it
+        P[(ptrdiff_t)(wl + wr + 1) * TB] = make_uint2(neg_h, neg_e);
+        P[(ptrdiff_t)(wl + wr + 2) * TB] = make_uint2(neg_h, neg_e);
+    }
+    score_out[ka] = sa;
+    ncig_out[ka] = done;
+    if (first.dual) {
+        score_out[kb] = sb;
+        ncig_out[kb] = done;
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        if (x == 1 && !first.dual) break;
+        // sum over rows of min(i + w + 1, qlen) - max(i - w, 0)
+        const long long q = x ? B.qlen : A.qlen, tl = x ? B.tlen : A.tlen, w = g.w;
+        const long long n1 = q - w < 0 ? 0 : (q - w < tl ? q - w : tl), lft = tl - 1 - w > 0 ? tl - 1 - w : 0;
+        ncells += (unsigned long long)(n1 * (w + 1) + n1 * (n1 - 1) / 2 + (tl - n1) * q - lft * (lft + 1) / 2);
     }
     if (bad) atomicOr(err, ERR_BASE);
     if (ncells) atomicAdd(cells_total, ncells);
