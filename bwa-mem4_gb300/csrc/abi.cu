@@ -712,9 +712,10 @@ namespace bwacuda {
 // queries against 750 bp windows on 152 SMs, microseconds:
 //   jobs      1 job in 32 / 16 / 8 lanes    2 jobs in 16 / 8 / 4 lanes
 //   1,024        309    323    408               407    480    666
-//   4,096        648    573    532               483    483    667
-//   16,384      2019   1657   1426              1155   1097    995
-//   200,000    22343  17663  14717             11283   9315   8603
+//   4,096        648    573    532               439    450    620
+//   16,384      2019   1657   1426              1092   1028    933
+//   65,536                                      3712   3087   2880
+//   262,144                                    14219  11335  10563
 // (100 x 400, 60 x 700 and 240 x 1200 bp order the same way.)
 struct RescueShape {
     int pair, lanes;

@@ -27,7 +27,8 @@ namespace bwacuda {
 constexpr int FAN = 4, FAN_WIDE = 8;
 constexpr int EXT_WIDE_JOBS_PER_SM = 2200;
 // Open-ended buckets: jobs per SM from which the band kernel gives a job 8 lanes, below it 32 (queries
-// of 2-10 kb on 152 SMs: 1,000 jobs 9.6 / 6.5 ms, 2,400 jobs 9.8 / 9.8, 20,000 jobs 23.1 / 42.4).
+// of 2-10 kb on 152 SMs: 1,000 jobs 9.6 / 6.5 ms, 2,400 jobs 9.8 / 9.8, 20,000 jobs 23.1 / 42.4; the 8 lanes 21.9 with the
+// finer target steps of the sort key).
 constexpr int BAND_LANES8_JOBS = 14;
 // Two jobs a thread (ext_dual.cuh) from this many jobs per SM on, in the 8-bit buckets of up to this
 // many columns (longer ones leave an SM too few of its warps).  Milliseconds on 152 SMs, one / two jobs

@@ -20,9 +20,9 @@ constexpr int TB = 64;
 // Measured (GB300): 10,000 queries of 1,500 bases in 3.24 ms with 8 lanes a job (5.06 with 150
 // registers and six blocks an SM before the bound, per-pair tests and selects, and chunk lengths
 // known at run time only), ALU pipe 73%, 537 instructions a warp row of four jobs, half of them the
-// fixed part; 20,000 queries of 2-10 kb 23.1 ms against 39.5 for a thread per job, whose longest warp
+// fixed part; 20,000 queries of 2-10 kb 21.9 ms against 39.5 for a thread per job, whose longest warp
 // set the time.  4 lanes a job: 14.1 against 14.7 ms on 60,000 of those 1,500-base jobs, but 29.8
-// against 23.1 ms on the 2-10 kb ones, so it is not built.
+// against 23.1 ms on the 2-10 kb ones (both in 1024-row sort steps), so it is not built.
 template <int L>
 __global__ void __launch_bounds__(TB, 10)
 ext_band_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__restrict__ jobs,

@@ -24,10 +24,11 @@
 // 128 >= o_del + e_del, at least the E step below that real cell loses; E and F only decay), and
 // their key's column byte is below every real column's, so they are never a row maximum.
 //
-// Per column and row: the score prmt, M0 = max(Hd + s, E, 0), H = max(M0, F), the key prmt and
-// half a 3-way key maximum, and E, F: with o_del + e_del == o_ins + e_ins both open from the
-// shared H - (o + e) (F opening from H equals F opening from M0 for o >= 0), 7.5 instructions
-// for two cells; otherwise F opens from M0 - (o_ins + e_ins), 8.5.  M0 of the next column is
+// Per column and row: the score prmt, M0 = max(Hd + s, E, 0), H = max(M0, F), the key (a
+// multiply-add of the FMA pipe) and half a 3-way key maximum, and E, F: with o_del + e_del ==
+// o_ins + e_ins both open from the shared H - (o + e) (F opening from H equals F opening from M0
+// for o >= 0), 6.5 instructions of the ALU pipe for two cells; otherwise F opens from M0 - (o_ins +
+// e_ins), 7.5.  M0 of the next column is
 // computed before H of this one, so the previous row's H is overwritten in place.
 //
 // The group's last lane stores each row's two keys (2 bytes a job and row, in the job's tracker
