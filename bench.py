@@ -532,12 +532,14 @@ def long_query_config(B, ctx, st, stream, timed, world, m=20000, seed=7000):
                       "ms_per_step": round(ms, 2), "identical": bool(np.array_equal(out, ref))}
 
     ctx.set_option(B.OPT_LONG_SLIDE, 0)
+    ctx.set_option(B.OPT_SMALL_BATCH, 0)  # a call of this size would run the band kernel unbucketed
     for lanes in (8, 16, 32):
         ctx.set_option(B.OPT_LONG_LANES, lanes)
         for path, name in ((B.PATH_PLAIN, "plain"), (B.PATH_BATCHED, "batched")):
             run(f"{name}_lanes{lanes}", path)
     ctx.set_option(B.OPT_LONG_LANES, 16)
     ctx.set_option(B.OPT_LONG_SLIDE, 1)
+    ctx.set_option(B.OPT_SMALL_BATCH, 350 * torch.cuda.get_device_properties(0).multi_processor_count)
     run("batched_window", B.PATH_BATCHED)
     best = max(rows, key=lambda k: rows[k]["value"])
     window = best == "batched_window"
