@@ -175,8 +175,10 @@ __device__ __forceinline__ void run_pair(uint32_t *__restrict__ cw, uint16_t *__
     A.init(JA, P, true);
     B.init(JB, P, two);
     const int qmax = A.qlen > B.qlen ? A.qlen : B.qlen;
-    // prmt selectors: A's score and its sign, B's and its sign (no query of this class holds an N: the
-    // sort keeps those in the 16-bit class)
+    // prmt selectors: A's score and its sign, B's and its sign (no query of this class holds a code of 4 or
+    // more: the sort keeps those in the 16-bit class, which checks them); alphabets of fewer than four
+    // letters are checked here
+    const uint32_t letters = m < 4 ? (uint32_t)m : 4u;
     for (int j = 0; j < qmax; j += 16) {
         uint32_t va[4], vb[4];
         load16(seq + JA.q_off, A.qlen, j, va);
@@ -184,7 +186,7 @@ __device__ __forceinline__ void run_pair(uint32_t *__restrict__ cw, uint16_t *__
 #pragma unroll
         for (int u = 0; u < 16; ++u) {
             const uint32_t a = (va[u >> 2] >> (8 * (u & 3))) & 0xffu, b = (vb[u >> 2] >> (8 * (u & 3))) & 0xffu;
-            bad |= a >= 4u || b >= 4u;
+            bad |= a >= letters || b >= letters;
             if (j + u < qmax) qs[(size_t)(j + u) * TB] = (uint16_t)(0xC480u + (a & 3u) * 0x11u + (b & 3u) * 0x1100u);
         }
     }
