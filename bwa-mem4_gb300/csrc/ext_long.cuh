@@ -206,10 +206,10 @@ ext_long_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__re
         }
         if (active && (J.qlen < min_qlen || ext_fits_i16(J.qlen, J.tlen, J.h0, P.sc.max_sc) == W32))
             active = false;  // another launch's job
-        // value bound: with gap extends capped at it (exact, see below) every F term stays in int
+        // gap extends capped at the value bound (exact, see below): W of them have to stay in int
         long long vb = active ? ext_value_bound(J.qlen, J.tlen, J.h0, P.sc.max_sc) : 1;
         if (vb < 1) vb = 1;
-        if (active && vb * (W + 1) >= (1LL << 31)) {
+        if (active && ((long long)e_ins < vb ? (long long)e_ins : vb) * (W + 1) >= (1LL << 31)) {
             if (k == 0) atomicOr(err, ERR_RANGE);
             active = false;
         }
@@ -271,14 +271,16 @@ ext_long_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__re
             const int ncol = run && beg < end ? end - beg : 0;
             const int nch = (ncol + W - 1) / W;
             const int nch_w = __reduce_max_sync(FULL, nch);
-            int fcarry = 0, hcarry = h1;
+            // F terms are kept W extends below their value: G(k') + (extends to the end of the chunk)
+            // would pass int for values near its end, less W extends it is at most the value itself
+            int fcarry = -W * ec, hcarry = h1;
             int kh = -1, kj = -1;                   // the lane's row maximum, later column on ties
             int first_live = INT_MAX, last_live = -1;
             int hlast_lane = h1;                    // H(i, end - 1) in the lane that holds it
             for (int ch = 0; ch < nch_w; ++ch) {
                 const int c0 = beg + ch * W + k * C;
                 int Mv[C], Ev[C], Gv[C], Hv[C], ENv[C];
-                int gl = INT_MIN / 2;
+                int gl = INT_MIN;
 #pragma unroll
                 for (int u = 0; u < C; ++u) {
                     const int col = c0 + u;
@@ -299,7 +301,7 @@ ext_long_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__re
                     ENv[u] = en > od ? en : od;         // E(i+1, col)
                     Mv[u] = M;
                     Ev[u] = e;
-                    Gv[u] = oi + (k * C + u + 1) * ec;
+                    Gv[u] = oi + (k * C + u + 1 - W) * ec;
                     gl = gl > Gv[u] ? gl : Gv[u];
                 }
                 // exclusive max-scan of the lanes' G maxima
@@ -310,12 +312,12 @@ ext_long_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__re
                     if (k >= o) sc = sc > x ? sc : x;
                 }
                 int ex = __shfl_up_sync(FULL, sc, 1, L);
-                if (k == 0) ex = INT_MIN / 2;
+                if (k == 0) ex = INT_MIN;
                 const int tot = __shfl_sync(FULL, sc, L - 1, L);
                 int runf = fcarry > ex ? fcarry : ex;
 #pragma unroll
                 for (int u = 0; u < C; ++u) {
-                    const int F = runf - (k * C + u) * ec;  // F(i, col)
+                    const int F = runf + (W - k * C - u) * ec;  // F(i, col)
                     runf = runf > Gv[u] ? runf : Gv[u];
                     int h = Mv[u] > Ev[u] ? Mv[u] : Ev[u];
                     Hv[u] = h > F ? h : F;
