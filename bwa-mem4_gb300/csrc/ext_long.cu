@@ -4,8 +4,7 @@
 //
 // A call makes up to two launches per cell class: the first with the caller's ring size
 // (enough for bands up to (R - 3) / 2 columns, or any band on queries of fewer than R
-// columns), and a deferred launch over the jobs the first one set aside, one 32-lane group
-// per block with the largest ring that fits a block's shared memory.
+// columns), and a deferred launch over the jobs the first one set aside, a warp per job.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -61,19 +60,19 @@ cudaError_t launch_first_lanes(const ExtLongLaunch &X, int nsm)
 }
 
 template <bool W32>
-cudaError_t launch_deferred(const ExtLongLaunch &X, const uint32_t *dbounds, uint32_t *dcounter, int nsm)
+cudaError_t launch_deferred(const ExtLongLaunch &X, const uint32_t *count, uint32_t *counter, uint32_t *counter_all,
+                            int nsm)
 {
-    constexpr int R = W32 ? xl::RING_MAX_32 : xl::RING_MAX_16;
-    auto kern = xl::ext_long_kernel<W32, 32, XL_C>;
-    const size_t smem = (size_t)xl::ring_words(R, W32) * 4;
+    constexpr int TB = 32 * xl::DEFER_WARPS;
+    auto kern = xl::ext_long_deferred_kernel<W32, XL_C>;
+    const size_t smem = (size_t)xl::ring_words(W32 ? xl::RING_MAX_32 : xl::RING_MAX_16, W32) * 4;
+    static_assert(xl::DEFER_WARPS * (xl::RING_MAX_16 / xl::DEFER_WARPS / 32) == xl::RING_MAX_16 / 32,
+                  "the warps' rings fill the largest one's words");
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EXT_SMEM_BLOCK_MAX);
     if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, smem)) != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidValue;
-    const uint32_t grid = (uint32_t)std::min<size_t>((size_t)per_sm * nsm, std::max<size_t>(X.njobs, 1));
-    kern<<<grid, 32, smem, X.stream>>>(X.seq, X.jobs, X.defer, dbounds, dcounter, X.njobs, 0, R, nullptr, nullptr, 0,
-                                      X.P, X.out, X.err, X.cells);
+    const uint32_t grid = (uint32_t)std::min<size_t>((size_t)nsm, std::max<size_t>(X.njobs, 1));
+    kern<<<grid, TB, smem, X.stream>>>(X.seq, X.jobs, X.defer, count, counter, counter_all, X.njobs, X.P, X.out, X.err,
+                                       X.cells);
     return cudaGetLastError();
 }
 
@@ -86,9 +85,9 @@ cudaError_t ext_long_launch(const ExtLongLaunch &X, bool w32, int nsm)
 
 cudaError_t ext_long_deferred_launch(const ExtLongLaunch &X, bool w32, uint32_t *work, int nsm)
 {
-    // work[0] = 0 and work[1] = the deferred count are the deferred launch's [start, stop)
-    return w32 ? launch_deferred<true>(X, work, work + XL_WORK_DCOUNTER32, nsm)
-               : launch_deferred<false>(X, work, work + XL_WORK_DCOUNTER16, nsm);
+    const uint32_t *count = work + XL_WORK_DCOUNT;
+    return w32 ? launch_deferred<true>(X, count, work + XL_WORK_DCOUNTER32, work + XL_WORK_DCOUNTER32 + 1, nsm)
+               : launch_deferred<false>(X, count, work + XL_WORK_DCOUNTER16, work + XL_WORK_DCOUNTER16 + 1, nsm);
 }
 
 int ext_long_ring_for_band(int w)

@@ -38,10 +38,10 @@ size_t ext_tpj_smem_limit_qcap(bool wide);
 // Group-per-job extension of any query length (ext_long.cu, ext_long.cuh).  Every call site
 // owns XL_WORK_WORDS device words, zeroed before its launches, and a deferred-job list of
 // njobs entries.
-constexpr int XL_WORK_DCOUNT = 1;                              // [0] stays 0, [1] deferred jobs
-constexpr int XL_WORK_DCOUNTER16 = 2, XL_WORK_DCOUNTER32 = 3;  // work counters of the deferred launches
-constexpr int XL_WORK_COUNTER16 = 4, XL_WORK_COUNTER32 = 5;    // work counters of unbucketed first launches
-constexpr int XL_WORK_BAND = 6;                                // work counter of a small batch's band launch
+constexpr int XL_WORK_DCOUNT = 0;                              // deferred jobs
+constexpr int XL_WORK_DCOUNTER16 = 1, XL_WORK_DCOUNTER32 = 3;  // work counters of the deferred launches, two each
+constexpr int XL_WORK_COUNTER16 = 5, XL_WORK_COUNTER32 = 6;    // work counters of unbucketed first launches
+constexpr int XL_WORK_BAND = 7;                                // work counter of a small batch's band launch
 constexpr int XL_WORK_WORDS = 8;
 constexpr int XL_RING_MIN = 256, XL_RING_FIRST_MAX = 4096;
 constexpr int XL_RING_DEFAULT = 512;  // first-launch ring when the bands are not known on the host
