@@ -35,6 +35,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "ext_job.cuh"
+#include "ext_long.cuh"
 #include "kernels.h"
 #include "runtime.h"
 
@@ -44,7 +45,7 @@ namespace {
 
 constexpr uint32_t ERR_INPUT = 8u;
 constexpr size_t ATS_MAX_CHUNK = size_t(1) << 24;  // 32-bit word indexing in the scatter
-constexpr int ATS_FLAG_BYTES = 32;                 // u32 input flag, pad, u64 bins[3]
+constexpr int ATS_FLAG_BYTES = 32;                 // u32 input flag, u32 jobs the band kernel leaves, u64 bins[3]
 // Blocks (of ATS_THREADS threads) of the pipeline's length / gather / scatter launches.  Later
 // chunks' lengths and gathers run beside the persistent DP kernels, in the room those leave free
 // (ATS_RESERVE_*), with a block for every other SM: eight 16-byte loads in flight per lane keep
@@ -81,16 +82,24 @@ __host__ __device__ __forceinline__ bool job_ok(const bwacuda_ext_job &J)
 // its device descriptor (the slice addresses, for now, in q_off / t_off; an invalid job empty)
 // for the gather, so the array crosses the host link once.
 __global__ void __launch_bounds__(ATS_THREADS) ats_lengths_kernel(const bwacuda_ext_job *__restrict__ hjobs,
-                                                                  uint32_t n, BinRule br,
+                                                                  uint32_t n, BinRule br, int small, int w,
+                                                                  const __grid_constant__ ExtParams P,
                                    uint64_t *__restrict__ sizes, uint32_t *__restrict__ flags,
                                    bwacuda_dev_ext_job *__restrict__ djobs)
 {
-    uint32_t bad = 0, bins[3] = {0, 0, 0};
+    uint32_t bad = 0, left = 0, bins[3] = {0, 0, 0};
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const bwacuda_ext_job J = hjobs[k];
         const bool ok = job_ok(J);
         bad |= !ok;
-        if (ok) bins[bin_label(br, J.qlen, J.tlen, J.h0)]++;
+        if (ok) {
+            bins[bin_label(br, J.qlen, J.tlen, J.h0)]++;
+            if (!small) left = 0;
+            else if (!ext_fits_i16(J.qlen, J.tlen, J.h0, P.sc.max_sc)) left |= EXT_LEFT_32;
+            else if (!xl::band_takes(J.qlen, clamp_band(w, J.qlen, P.sc.max_sc, P.end_bonus, P.sc.o_ins, P.sc.e_ins,
+                                                        P.sc.o_del, P.sc.e_del)))
+                left |= EXT_LEFT_16;
+        }
         // reserve, in bytes (a multiple of 16, so every job's base stays aligned)
         sizes[k] = ok ? 16ull * (slice_words(J.query, J.qlen) + slice_words(J.target, J.tlen)) : 0u;
         bwacuda_dev_ext_job D;
@@ -104,11 +113,13 @@ __global__ void __launch_bounds__(ATS_THREADS) ats_lengths_kernel(const bwacuda_
     }
     // every thread of the warp reaches this point
     bad = __reduce_or_sync(0xffffffffu, bad);
+    left = __reduce_or_sync(0xffffffffu, left);
     const uint32_t b0 = __reduce_add_sync(0xffffffffu, bins[0]);
     const uint32_t b1 = __reduce_add_sync(0xffffffffu, bins[1]);
     const uint32_t b2 = __reduce_add_sync(0xffffffffu, bins[2]);
     if ((threadIdx.x & 31) == 0) {
         if (bad) atomicOr(flags, ERR_INPUT);
+        if (left) atomicOr(flags + 1, left);
         unsigned long long *cnt = reinterpret_cast<unsigned long long *>(flags + 2);
         if (b0) atomicAdd(cnt + 0, (unsigned long long)b0);
         if (b1) atomicAdd(cnt + 1, (unsigned long long)b1);
@@ -245,7 +256,7 @@ int ats_retire(bwacuda_ctx *c, AtsChunk &R, uint32_t *input_flags)
 // caller's job array: each job lands in its device descriptor), the offset scan, the byte total
 // back to the host.  Enqueued while the previous chunk's gather runs.
 cudaError_t ats_plan_chunk(bwacuda_ctx *c, AtsChunk &R, const bwacuda_ext_job *hj, size_t cn, const BinRule &br,
-                           bool first)
+                           const ExtParams &P, int w, bool first)
 {
     cudaStream_t p = c->ats->pstream;
     cudaError_t e;
@@ -266,12 +277,16 @@ cudaError_t ats_plan_chunk(bwacuda_ctx *c, AtsChunk &R, const bwacuda_ext_job *h
     if ((e = cudaMemsetAsync(flags, 0, ATS_FLAG_BYTES, p)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(sizes + cn, 0, 8, p)) != cudaSuccess) return e;
     const uint32_t grid = ats_grid(cn, batched_nsm(c), first);
-    ats_lengths_kernel<<<grid, ATS_THREADS, 0, p>>>(hj, (uint32_t)cn, br, sizes, flags,
+    const bool small = batched_is_small(c, cn, P);
+    ats_lengths_kernel<<<grid, ATS_THREADS, 0, p>>>(hj, (uint32_t)cn, br, small ? 1 : 0, w, P, sizes, flags,
                                                     static_cast<bwacuda_dev_ext_job *>(R.djobs.p));
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = cub::DeviceScan::ExclusiveSum(R.scan_tmp.p, scan_bytes, sizes, offs, (int)cn + 1, p)) != cudaSuccess)
         return e;
-    if ((e = cudaMemcpyAsync(R.h_total.p, offs + cn, 8, cudaMemcpyDeviceToHost, p)) != cudaSuccess) return e;
+    uint64_t *h = static_cast<uint64_t *>(R.h_total.p);
+    if ((e = cudaMemcpyAsync(h, offs + cn, 8, cudaMemcpyDeviceToHost, p)) != cudaSuccess) return e;
+    h[1] = (uint64_t)(EXT_LEFT_16 | EXT_LEFT_32) << 32;
+    if (small && (e = cudaMemcpyAsync(h + 1, flags, 8, cudaMemcpyDeviceToHost, p)) != cudaSuccess) return e;
     return cudaEventRecord(R.planned, p);
 }
 
@@ -304,10 +319,12 @@ cudaError_t ats_extend_chunk(bwacuda_ctx *c, AtsChunk &R, int si, size_t cn, siz
     BatchBufs *bb = batched_slot_bufs(c, si);
     batched_set_reserve(bb, ATS_RESERVE_REGS, ATS_RESERVE_THREADS);
     batched_set_call(bb, n);
+    batched_set_left(bb, (int)(static_cast<const uint64_t *>(R.h_total.p)[1] >> 32));
     e = batched_enqueue(c, bb, static_cast<const uint8_t *>(R.seq.p), static_cast<const bwacuda_dev_ext_job *>(R.djobs.p),
                         cn, P, static_cast<bwacuda_ext_result *>(R.dout.p), s, nullptr, nullptr);
     batched_set_reserve(bb, 0, 0);
     batched_set_call(bb, 0);
+    batched_set_left(bb, EXT_LEFT_16 | EXT_LEFT_32);
     if (e != cudaSuccess) return e;
     const uint32_t words = (uint32_t)(cn * (sizeof(bwacuda_ext_result) / 4));
     const uint32_t grid = ats_grid(words, batched_nsm(c), true);
@@ -347,7 +364,7 @@ int ats_gather_ext(bwacuda_ctx *c, const bwacuda_ext_job *hj, size_t n, int w, D
     const int nsm = batched_nsm(c);
     const uint32_t grid = (uint32_t)std::min<size_t>((n + ATS_THREADS - 1) / ATS_THREADS, (size_t)nsm * 16);
     BinRule br{0, 0, 0};
-    ats_lengths_kernel<<<grid, ATS_THREADS, 0, s>>>(hj, (uint32_t)n, br, sizes, flags,
+    ats_lengths_kernel<<<grid, ATS_THREADS, 0, s>>>(hj, (uint32_t)n, br, 0, w, ExtParams{}, sizes, flags,
                                                     static_cast<bwacuda_dev_ext_job *>(djobs.p));
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
     if ((e = cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, sizes, offs, (int)n + 1, s)) != cudaSuccess)
@@ -431,7 +448,7 @@ int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int 
     {
         AtsChunk &R0 = c->ats->ring[0];
         if ((rc = ats_retire(c, R0, &input_flags)) == BWACUDA_OK) {
-            const cudaError_t e = ats_plan_chunk(c, R0, jobs, chunk_len(0, 0), br, true);
+            const cudaError_t e = ats_plan_chunk(c, R0, jobs, chunk_len(0, 0), br, P, w, true);
             if (e != cudaSuccess) rc = cuda_status(e);
         }
     }
@@ -451,7 +468,7 @@ int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int 
         if (c1 < n) {
             AtsChunk &R1 = c->ats->ring[(k + 1) % ATS_RING];
             if ((rc = ats_retire(c, R1, &input_flags)) != BWACUDA_OK) break;
-            if ((e = ats_plan_chunk(c, R1, jobs + c1, chunk_len(k + 1, c1), br, false)) != cudaSuccess) {
+            if ((e = ats_plan_chunk(c, R1, jobs + c1, chunk_len(k + 1, c1), br, P, w, false)) != cudaSuccess) {
                 rc = cuda_status(e);
                 break;
             }

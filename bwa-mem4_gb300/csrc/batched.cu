@@ -56,6 +56,7 @@ struct BatchBufs {
     ExtParams g_P{};
     int nfan = 0;            // streams and join events that exist
     size_t call_jobs = 0;    // jobs of the whole call when the batch is one chunk of it
+    int left = EXT_LEFT_16 | EXT_LEFT_32;  // what a small batch may hold besides the band kernel's jobs
     // per-SM room the bucket kernels leave for kernels running beside them
     int reserve_regs = 0, reserve_threads = 0;
     size_t jobs_cap = 0;  // jobs the work buffers are sized for (batched_enqueue, batched_reserve)
@@ -202,12 +203,13 @@ int batched_set_long(bwacuda_ctx *c, int long_qlo)
 int batched_get_long(bwacuda_ctx *c) { return c->batched ? c->batched->long_qlo : INT_MAX; }
 
 // Lanes per job of the group-per-job kernel; a new value invalidates captured graphs.
-int batched_set_long_lanes(bwacuda_ctx *c, int lanes)
+int batched_set_long_lanes(bwacuda_ctx *c, int lanes, bool by_option)
 {
     int rc = batched_init(c);
     if (rc) return rc;
-    if (c->long_lanes != lanes) {
+    if (c->long_lanes != lanes || (by_option && !c->long_lanes_set)) {
         c->long_lanes = lanes;
+        c->long_lanes_set |= by_option;
         c->batched->gen++;
     }
     return BWACUDA_OK;
@@ -270,12 +272,12 @@ bool batched_is_small(const bwacuda_ctx *c, size_t n, const ExtParams &P)
     return n <= c->small_jobs && !P.ug.enabled;
 }
 
-// A small batch: no buckets, the band kernel over every job and the
-// group-per-job kernels for what it leaves (32-bit values, queries and bands past its window).
-// Thread-per-job buckets take 0.3-0.5 ms however few jobs they hold.  32 lanes a job below 8 jobs
-// per SM, 16 below 20, else 8 (the times stand at EXT_SMALL_JOBS_PER_SM); with 8 the jobs are sorted
-// first, longest first: the four jobs of a warp step to its longest, and 20,000 queries of 2-10 kb in
-// caller order took 32.4 ms against 23.1.
+// A small batch: the band kernel over every job, and what it leaves (bb.left: 32-bit values, queries
+// and bands past its window) in the group-per-job kernels or, where it is many 32-bit jobs, in their
+// length buckets (EXT_SMALL_WIDE_PER_SM).  Thread-per-job buckets take 0.3-0.5 ms however few jobs they
+// hold.  32 lanes a job below 8 jobs per SM, 16 below 20, else 8 (the times stand at
+// EXT_SMALL_JOBS_PER_SM); with 8 the jobs are sorted first, longest first: the four jobs of a warp step to
+// its longest, and 20,000 queries of 2-10 kb in caller order took 32.4 ms against 23.1.
 static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d_seq,
                                  const bwacuda_dev_ext_job *d_jobs, size_t n, const ExtParams &P,
                                  bwacuda_ext_result *d_out, cudaStream_t s, uint32_t *err, unsigned long long *cells)
@@ -307,20 +309,57 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
     X.stream = s;
     const int lanes = n < (size_t)B->nsm * 8 ? 32 : (n < (size_t)B->nsm * 20 ? 16 : 8);
     if (lanes == 8) {
-        uint32_t *order = static_cast<uint32_t *>(bb.idx_out.p);
-        if ((e = ext_sort_jobs(d_jobs, n, P.sc.max_sc, 1u, false, d_seq, P.ug, P.zdrop, d_out,
-                               static_cast<uint32_t *>(bb.keys_in.p), static_cast<uint32_t *>(bb.keys_out.p),
-                               static_cast<uint32_t *>(bb.idx_in.p), order, bb.tmp.p, bb.tmp.cap, s)) != cudaSuccess)
+        uint32_t *order = static_cast<uint32_t *>(bb.idx_out.p), *keys = static_cast<uint32_t *>(bb.keys_out.p);
+        if ((e = ext_sort_jobs(d_jobs, n, P.sc.max_sc, 0u, false, d_seq, P.ug, P.zdrop, d_out,
+                               static_cast<uint32_t *>(bb.keys_in.p), keys, static_cast<uint32_t *>(bb.idx_in.p), order,
+                               bb.tmp.p, bb.tmp.cap, s, &P)) != cudaSuccess)
             return e;
         X.order = order;
+        uint32_t *table = static_cast<uint32_t *>(bb.table.p);
+        const uint32_t many = c->long_lanes_set ? UINT32_MAX : (uint32_t)(B->nsm * EXT_SMALL_LEFT8_PER_SM);
+        if (bb.left && (e = ext_small_bounds(keys, n, (uint32_t)(B->nsm * EXT_SMALL_WIDE_PER_SM), many,
+                                             static_cast<const ExtBucketDef *>(B->d_defs.p), B->nb, table, work, s)) !=
+                           cudaSuccess)
+            return e;
+        if ((bb.left & EXT_LEFT_32) && n >= (size_t)B->nsm * EXT_SMALL_WIDE_PER_SM) {
+            PersistLaunch L;
+            L.seq = d_seq;
+            L.jobs = d_jobs;
+            L.order = order;
+            L.P = P;
+            L.out = d_out;
+            L.err = X.err;
+            L.cells = X.cells;
+            L.grab = 1;
+            L.stream = s;
+            if ((e = ext_wide_launch(L, static_cast<const ExtBucketDef *>(B->d_defs.p), B->nb, table, work, B->nsm)) !=
+                cudaSuccess)
+                return e;
+        }
     }
     if ((e = ext_band_launch(X, lanes, work + XL_WORK_BAND, 0u, UINT32_MAX, B->nsm)) != cudaSuccess) return e;
-    for (int w32 = 0; w32 < 2; ++w32) {
-        X.counter = work + (w32 ? XL_WORK_COUNTER32 : XL_WORK_COUNTER16);
-        if ((e = ext_long_launch(X, w32 != 0, B->nsm)) != cudaSuccess) return e;
+    // the group-per-job kernels: [start, stop) of the sorted jobs, or every job in caller order
+    if (bb.left & EXT_LEFT_16) {
+        X.counter = work + XL_WORK_COUNTER16;
+        X.bounds = X.order ? work + XL_WORK_LEFT : nullptr;
+        if ((e = ext_long_launch(X, false, B->nsm)) != cudaSuccess) return e;
+        if (X.order && !c->long_lanes_set && n >= (size_t)B->nsm * EXT_SMALL_LEFT8_PER_SM) {
+            ExtLongLaunch Y = X;
+            Y.lanes = 8;
+            Y.counter = work + XL_WORK_COUNTER_MANY;
+            Y.bounds = work + XL_WORK_LEFT_MANY;
+            if ((e = ext_long_launch(Y, false, B->nsm)) != cudaSuccess) return e;
+        }
+    }
+    if (bb.left & EXT_LEFT_32) {
+        X.counter = work + XL_WORK_COUNTER32;
+        X.bounds = X.order ? work + XL_WORK_WIDE : nullptr;
+        if ((e = ext_long_launch(X, true, B->nsm)) != cudaSuccess) return e;
     }
     for (int w32 = 0; w32 < 2; ++w32)
-        if ((e = ext_long_deferred_launch(X, w32 != 0, work, B->nsm)) != cudaSuccess) return e;
+        if ((bb.left & (w32 ? EXT_LEFT_32 : EXT_LEFT_16)) &&
+            (e = ext_long_deferred_launch(X, w32 != 0, work, B->nsm)) != cudaSuccess)
+            return e;
     return cudaSuccess;
 }
 
@@ -472,6 +511,7 @@ void batched_set_reserve(BatchBufs *bb, int regs, int threads)
     bb->reserve_threads = threads;
 }
 void batched_set_call(BatchBufs *bb, size_t jobs) { bb->call_jobs = jobs; }
+void batched_set_left(BatchBufs *bb, int left) { bb->left = left; }
 BatchBufs *batched_slot_bufs(bwacuda_ctx *c, int slot) { return &c->batched->bufs[slot & 1]; }
 int batched_nsm(bwacuda_ctx *c) { return c->batched->nsm; }
 // Launches of the bucket stage: one per bucket and the two deferred group-per-job launches.

@@ -14,6 +14,7 @@
 
 #include "common.cuh"
 #include "ext_job.cuh"
+#include "ext_long.cuh"
 #include "kernels.h"
 #include "persist.h"
 
@@ -30,7 +31,20 @@ __device__ __forceinline__ uint32_t ext_cell_class(const bwacuda_dev_ext_job &J,
     return ext_fits_i16(J.qlen, J.tlen, J.h0, max_sc) ? 1u : 2u;
 }
 
-// Sort key of EXT_KEY_BITS: cell class (at least min_cls), query length descending (clamped at 1023),
+// What sets the classes of a sorted small batch: the band of a job (on: such a batch).
+struct SmallRule {
+    int on, end_bonus, o_ins, e_ins, o_del, e_del;
+};
+
+// Class of a job in a small batch: 0 = the band kernel's, 1 = the other 16-bit ones, 2 = 32-bit.
+__device__ __forceinline__ uint32_t ext_small_class(const bwacuda_dev_ext_job &J, int max_sc, const SmallRule &r)
+{
+    if (!ext_fits_i16(J.qlen, J.tlen, J.h0, max_sc)) return 2u;
+    const int w = clamp_band(J.w < 0 ? 0 : J.w, J.qlen, max_sc, r.end_bonus, r.o_ins, r.e_ins, r.o_del, r.e_del);
+    return xl::band_takes(J.qlen, w) ? 0u : 1u;
+}
+
+// Sort key of EXT_KEY_BITS: class, query length descending (clamped at 1023),
 // target length descending in 32-row steps, seed score descending in steps of 4; the queries of 1023
 // bases or more, whose rows the open-ended buckets' kernels run longest first with the jobs of a warp
 // in step, by target length alone (32-row steps up to 32,736 rows; 20,000 jobs of 2-10 kb: 23.2 ms in
@@ -38,10 +52,8 @@ __device__ __forceinline__ uint32_t ext_cell_class(const bwacuda_dev_ext_job &J,
 // seed score sets how far a row's live cells reach and how many rows live, so warps of equal scores
 // run nearly equal windows: 4.2M read pairs 13.39 -> 12.4 ms, 1M mixed lengths 4.22 -> 3.84 ms with
 // it.  Within a bucket the order sets only which jobs run together, never a result.
-__device__ __forceinline__ uint32_t ext_sort_key(const bwacuda_dev_ext_job &J, int max_sc, uint32_t min_cls)
+__device__ __forceinline__ uint32_t ext_sort_key(const bwacuda_dev_ext_job &J, uint32_t cls)
 {
-    uint32_t cls = ext_cell_class(J, max_sc);
-    cls = cls > min_cls ? cls : min_cls;
     const uint32_t ql = J.qlen < 0 ? 0u : (J.qlen > 1023 ? 1023u : (uint32_t)J.qlen);
     const uint32_t ts = J.tlen < 0 ? 0u : (uint32_t)J.tlen >> 5;
     if (ql == 1023u) return (cls << 20) | (1023u - (ts > 1023u ? 1023u : ts));
@@ -93,13 +105,15 @@ __device__ bool ungapped_hit(const uint8_t *q, int qlen, const uint8_t *t, int t
 // Sort keys; with the ungapped rule on, jobs it settles get their result here
 // and key class 3, which no bucket covers.
 __global__ void ext_keys_kernel(const bwacuda_dev_ext_job *__restrict__ jobs, uint32_t n, int max_sc,
-                                uint32_t min_cls, int n_to_16, const uint8_t *__restrict__ seq, const UngappedRule ug, int zdrop,
+                                uint32_t min_cls, int n_to_16, const SmallRule small,
+                                const uint8_t *__restrict__ seq, const UngappedRule ug, int zdrop,
                                 bwacuda_ext_result *__restrict__ out, uint32_t *__restrict__ keys,
                                 uint32_t *__restrict__ idx)
 {
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const bwacuda_dev_ext_job J = jobs[k];
-        uint32_t key = ext_sort_key(J, max_sc, min_cls);
+        uint32_t key = ext_sort_key(J, small.on ? ext_small_class(J, max_sc, small)
+                                                : max(ext_cell_class(J, max_sc), min_cls));
         if (n_to_16 && key < (1u << 20) && J.qlen > 0) {  // an 8-bit job: any code of 4 or more?
             uint32_t any = 0u;
             for (int j = 0; j < J.qlen; j += 16) {
@@ -119,6 +133,17 @@ __global__ void ext_keys_kernel(const bwacuda_dev_ext_job *__restrict__ jobs, ui
         keys[k] = key;
         idx[k] = k;
     }
+}
+
+// First and last sort key of a bucket.
+struct BucketKeys {
+    uint32_t lo, hi;
+};
+__device__ __forceinline__ BucketKeys bucket_keys(const ExtBucketDef &d)
+{
+    const uint32_t ql_hi = d.qhi > 1023 ? 1023u : (uint32_t)d.qhi;
+    const uint32_t ql_lo = d.qlo > 1023 ? 1023u : (uint32_t)d.qlo;
+    return {((uint32_t)d.cls << 20) | ((1023u - ql_hi) << 10), ((uint32_t)d.cls << 20) | ((1023u - ql_lo) << 10) | 1023u};
 }
 
 __device__ __forceinline__ uint32_t lower_bound(const uint32_t *a, uint32_t n, uint32_t v)
@@ -142,15 +167,43 @@ __global__ void ext_bucket_bounds_kernel(const uint32_t *__restrict__ keys, uint
 {
     const int b = threadIdx.x;
     if (b >= nb) return;
-    const ExtBucketDef d = defs[b];
-    const uint32_t ql_hi = d.qhi > 1023 ? 1023u : (uint32_t)d.qhi;
-    const uint32_t ql_lo = d.qlo > 1023 ? 1023u : (uint32_t)d.qlo;
-    const uint32_t key_lo = ((uint32_t)d.cls << 20) | ((1023u - ql_hi) << 10);
-    const uint32_t key_hi = ((uint32_t)d.cls << 20) | ((1023u - ql_lo) << 10) | 1023u;
-    table[b * 4 + 0] = lower_bound(keys, n, key_lo);
-    table[b * 4 + 1] = lower_bound(keys, n, key_hi + 1);
+    const BucketKeys k = bucket_keys(defs[b]);
+    table[b * 4 + 0] = lower_bound(keys, n, k.lo);
+    table[b * 4 + 1] = lower_bound(keys, n, k.hi + 1);
     table[b * 4 + 2] = 0;  // work counter
     table[b * 4 + 3] = 0;  // work counter of the band kernel (open-ended buckets)
+}
+
+// ext_small_bounds.  Longer queries come first in a class, so the 32-bit jobs past the thread-per-job
+// buckets lie in front of them.
+__global__ void ext_small_bounds_kernel(const uint32_t *__restrict__ keys, uint32_t n, uint32_t wide_min,
+                                        uint32_t many_min, const ExtBucketDef *__restrict__ defs, int nb,
+                                        uint32_t *__restrict__ table, uint32_t *__restrict__ work)
+{
+    __shared__ uint32_t first;  // of the 32-bit jobs in thread-per-job buckets
+    const int b = threadIdx.x;
+    const uint32_t c1 = lower_bound(keys, n, 1u << 20), c2 = lower_bound(keys, n, 2u << 20);
+    if (b == 0) first = n;
+    __syncthreads();
+    if (b < nb && defs[b].cls == 2 && defs[b].kernel == 0) {
+        const BucketKeys k = bucket_keys(defs[b]);
+        const uint32_t lo = lower_bound(keys, n, k.lo);
+        table[b * 4 + 0] = lo;
+        table[b * 4 + 1] = n - c2 >= wide_min ? lower_bound(keys, n, k.hi + 1) : lo;
+        table[b * 4 + 2] = 0;
+        atomicMin(&first, lo);
+    }
+    __syncthreads();
+    if (b == 0) {
+        const bool many = c2 - c1 >= many_min;
+        work[XL_WORK_WIDE] = c2;
+        work[XL_WORK_WIDE + 1] = n - c2 >= wide_min ? first : n;
+        work[XL_WORK_WIDE_BUCKETS] = n - c2 >= wide_min;
+        work[XL_WORK_LEFT] = c1;
+        work[XL_WORK_LEFT + 1] = many ? c1 : c2;
+        work[XL_WORK_LEFT_MANY] = c1;
+        work[XL_WORK_LEFT_MANY + 1] = many ? c2 : c1;
+    }
 }
 
 }  // namespace
@@ -203,10 +256,13 @@ int ext_bucket_defs(ExtBucketDef *defs, int max_defs, int step, int long_qlo)
 
 cudaError_t ext_sort_prefer_shared()
 {
-    // The bucket-bound kernel (one block, no shared memory) prefers the bucket kernels'
+    // The bucket-bound kernels (one block, next to no shared memory) prefer the bucket kernels'
     // maximum shared-memory carveout.  The key kernel keeps the default: its blocks live for
     // one pass only, and with the ungapped rule it reads every job's bases through L1.
-    return cudaFuncSetAttribute(ext_bucket_bounds_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+    const cudaError_t e = cudaFuncSetAttribute(ext_bucket_bounds_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                               cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(ext_small_bounds_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 cudaSharedmemCarveoutMaxShared);
 }
 
@@ -218,19 +274,19 @@ size_t ext_sort_temp_bytes(size_t n)
     return bytes;
 }
 
-// Keys and their sort: idx_out holds the job indices by key.  min_cls 1 sorts the 8- and 16-bit
-// classes as one; n_to_16 puts 8-bit jobs whose query holds an N into the 16-bit class (the kernel of
-// two jobs a thread scores codes 0..3 only).
 cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, uint32_t min_cls, bool n_to_16,
                           const uint8_t *seq, const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
                           uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp, size_t tmp_bytes,
-                          cudaStream_t s)
+                          cudaStream_t s, const ExtParams *small)
 {
     if (n == 0) return cudaSuccess;
+    SmallRule sr{};
+    if (small)
+        sr = SmallRule{1, small->end_bonus, small->sc.o_ins, small->sc.e_ins, small->sc.o_del, small->sc.e_del};
     uint32_t grid = (uint32_t)((n + 255) / 256);
     if (grid > 8192) grid = 8192;
-    ext_keys_kernel<<<grid, 256, 0, s>>>(jobs, (uint32_t)n, max_sc, min_cls, n_to_16 ? 1 : 0, seq, ug, zdrop, out, keys_in,
-                                         idx_in);
+    ext_keys_kernel<<<grid, 256, 0, s>>>(jobs, (uint32_t)n, max_sc, min_cls, n_to_16 ? 1 : 0, sr, seq, ug, zdrop, out,
+                                         keys_in, idx_in);
     return cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys_in, keys_out, idx_in, idx_out, (int)n, 0, EXT_KEY_BITS, s);
 }
 
@@ -245,6 +301,13 @@ cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int m
                                         idx_in, idx_out, tmp, tmp_bytes, s);
     if (e != cudaSuccess) return e;
     ext_bucket_bounds_kernel<<<1, EXT_MAX_BUCKETS, 0, s>>>(keys_out, (uint32_t)n, d_defs, nb, d_table);
+    return cudaGetLastError();
+}
+
+cudaError_t ext_small_bounds(const uint32_t *keys, size_t n, uint32_t wide_min, uint32_t many_min,
+                             const ExtBucketDef *d_defs, int nb, uint32_t *d_table, uint32_t *work, cudaStream_t s)
+{
+    ext_small_bounds_kernel<<<1, EXT_MAX_BUCKETS, 0, s>>>(keys, (uint32_t)n, wide_min, many_min, d_defs, nb, d_table, work);
     return cudaGetLastError();
 }
 

@@ -42,7 +42,12 @@ constexpr int XL_WORK_DCOUNT = 0;                              // deferred jobs
 constexpr int XL_WORK_DCOUNTER16 = 1, XL_WORK_DCOUNTER32 = 3;  // work counters of the deferred launches, two each
 constexpr int XL_WORK_COUNTER16 = 5, XL_WORK_COUNTER32 = 6;    // work counters of unbucketed first launches
 constexpr int XL_WORK_BAND = 7;                                // work counter of a small batch's band launch
-constexpr int XL_WORK_WORDS = 8;
+// of a sorted small batch (ext_small_bounds): [start, stop) of its 32-bit jobs and of its other jobs past
+// the band kernel's window, when those are few and when they are many; the latter's work counter; whether
+// the 32-bit jobs run in length buckets
+constexpr int XL_WORK_WIDE = 8, XL_WORK_LEFT = 10, XL_WORK_LEFT_MANY = 12, XL_WORK_COUNTER_MANY = 14;
+constexpr int XL_WORK_WIDE_BUCKETS = 15;
+constexpr int XL_WORK_WORDS = 16;
 constexpr int XL_RING_MIN = 256, XL_RING_FIRST_MAX = 4096;
 constexpr int XL_RING_DEFAULT = 512;  // first-launch ring when the bands are not known on the host
 
@@ -80,6 +85,17 @@ cudaError_t ext_long_launch(const ExtLongLaunch &X, bool w32, int nsm);
 //   65,536      812 / 1972      847 / 910    1966 / 2015    2017 / 2039
 //   131,072     907 / 2130     1597 / 1595
 constexpr int EXT_SMALL_JOBS_PER_SM = 350;
+// What the band kernel leaves of a small batch runs in the group-per-job kernels, except that 32-bit
+// jobs from EXT_SMALL_WIDE_PER_SM per SM on get a thread each in the length buckets; the 16-bit ones get
+// 8 lanes each from EXT_SMALL_LEFT8_PER_SM per SM on unless BWACUDA_OPT_LONG_LANES is set.
+// Microseconds on 152 SMs, buckets / 16 lanes / 8 lanes:
+//   jobs      150 bases, 32-bit      300 bases, band 200     600 bases, band 150
+//    3,500       990 /  505 /  568    1790 /   941 /  1131    3000 /  1964 /  2376
+//   10,000       961 / 1317 / 1170    3240 /  2452 /  2317    5660 /  4981 /  4817
+//   20,000      1772 / 2294 / 1921    4810 /  4435 /  3695   10070 /  9147 /  7614
+//   50,000      2610 / 5300 / 4324    9490 / 10531 /  8213   25180 / 22002 / 17157
+constexpr int EXT_SMALL_WIDE_PER_SM = 45;
+constexpr int EXT_SMALL_LEFT8_PER_SM = 60;
 constexpr int EXT_DIRECT_JOBS_PER_SM = 24;
 // The band kernel (ext_band.cuh) with 8, 16 or 32 lanes a job over X's jobs that band_takes admits,
 // when [start, stop) holds count_lo or more and fewer than count_hi; counter: a zeroed device word.

@@ -45,23 +45,35 @@ int ext_bucket_defs(ExtBucketDef *defs, int max_defs, int step, int long_qlo);
 size_t ext_sort_temp_bytes(size_t n);
 // the sort's own kernels prefer the maximum shared-memory carveout (once per device)
 cudaError_t ext_sort_prefer_shared();
-// keys + radix sort + bucket bounds; d_table holds 4 words per bucket
-// (start, end, work counter, spare).
-// With P.ug enabled the key kernel also settles ungapped hits (results written to out).
-// pair_lanes false (gap costs too large for 16-bit lanes) keeps every job out of
-// the 8-bit class.
-// An 8-bit bucket with two jobs per thread (ext_dual.cuh): scorings of at most five letters.
-cudaError_t ext_dual_launch(const PersistLaunch &L, const ExtBucketDef &d, uint32_t *d_bucket_table, int nsm);
+// Keys and radix sort: idx_out holds the job indices by class (at least min_cls), query length, target
+// length and seed score, each descending.  n_to_16 puts 8-bit jobs whose query holds a code of 4 or more
+// into the 16-bit class; with ug enabled the key kernel also settles ungapped hits (results written to
+// out).  small (a small batch's parameters): the classes are the band kernel's jobs, the other 16-bit
+// ones and the 32-bit ones.
 cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, uint32_t min_cls, bool n_to_16,
                           const uint8_t *seq, const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
                           uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp, size_t tmp_bytes,
-                          cudaStream_t s);
+                          cudaStream_t s, const ExtParams *small = nullptr);
+// ext_sort_jobs and the bucket bounds; d_table holds 4 words per bucket (start, end, work counter,
+// the band kernel's work counter).  pair_lanes false (gap costs too large for 16-bit lanes) keeps every
+// job out of the 8-bit class.
 cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, bool pair_lanes, bool n_to_16,
                                 const uint8_t *seq,
                                 const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
                                 uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp,
                                 size_t tmp_bytes, const ExtBucketDef *d_defs, int nb, uint32_t *d_table,
                                 cudaStream_t s);
+// Who runs what the band kernel leaves of a sorted small batch (keys of ext_sort_jobs with small): the
+// 32-bit jobs in their length buckets from wide_min on, below that in work[XL_WORK_WIDE], which always
+// holds those past the thread-per-job buckets; the 16-bit ones in work[XL_WORK_LEFT], or from many_min
+// on in work[XL_WORK_LEFT_MANY].
+cudaError_t ext_small_bounds(const uint32_t *keys, size_t n, uint32_t wide_min, uint32_t many_min,
+                             const ExtBucketDef *d_defs, int nb, uint32_t *d_table, uint32_t *work, cudaStream_t s);
+// Those buckets of 32-bit jobs, all in one launch (ext_wide.cu).
+cudaError_t ext_wide_launch(const PersistLaunch &L, const ExtBucketDef *d_defs, int nb, uint32_t *d_table,
+                            const uint32_t *work, int nsm);
+// An 8-bit bucket with two jobs per thread (ext_dual.cuh): scorings of at most five letters.
+cudaError_t ext_dual_launch(const PersistLaunch &L, const ExtBucketDef &d, uint32_t *d_bucket_table, int nsm);
 // per-grab instantiations (ext_persist_g1.cu, _g2.cu, _g4.cu)
 cudaError_t ext_persist_launch_g1(const PersistLaunch &L, const ExtBucketDef &d, uint32_t *table, int nsm, int tb);
 cudaError_t ext_persist_launch_g2(const PersistLaunch &L, const ExtBucketDef &d, uint32_t *table, int nsm, int tb);

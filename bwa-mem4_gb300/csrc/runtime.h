@@ -98,6 +98,7 @@ struct bwacuda_ctx {
     int rescue_pair = -1;  // lanes of a group holding two byte-range jobs (rescue_wf2.cuh): 4, 8, 16; 0 off; -1: not set
     bool ungapped = false;  // ungapped-diagonal fast path on the batched extension path
     int long_lanes = 16;    // lanes per job of the group-per-job extension kernel (8, 16, 32)
+    bool long_lanes_set = false;  // BWACUDA_OPT_LONG_LANES was set
     int long_slide = 1;     // band kernel on the open-ended buckets: 0 off, 1 lanes by the bucket's jobs, 2 always 8 lanes
     size_t small_jobs = 0;  // batched calls of up to this many jobs run unsorted in the band kernel (set from the SM count)
     int tune_candidates = 0;        // last autotune call
@@ -153,7 +154,7 @@ int batched_set_bucket_step(bwacuda_ctx *c, int step);
 void batched_get_tuning(bwacuda_ctx *c, int *tb, int *grab, int *step);
 int batched_set_long(bwacuda_ctx *c, int long_qlo);
 int batched_get_long(bwacuda_ctx *c);
-int batched_set_long_lanes(bwacuda_ctx *c, int lanes);
+int batched_set_long_lanes(bwacuda_ctx *c, int lanes, bool by_option = false);
 int batched_set_long_slide(bwacuda_ctx *c, int mode);
 int batched_set_small(bwacuda_ctx *c, size_t jobs);
 
@@ -165,6 +166,9 @@ cudaError_t batched_enqueue(bwacuda_ctx *c, BatchBufs *bb, const uint8_t *d_seq,
                             size_t n, const ExtParams &P, bwacuda_ext_result *d_out, cudaStream_t s, uint32_t *err,
                             unsigned long long *cells);
 void batched_set_call(BatchBufs *bb, size_t jobs);  // jobs of the call whose chunks follow (0: batches by themselves)
+// What a small batch may hold besides the band kernel's jobs, where the caller knows it.
+constexpr int EXT_LEFT_16 = 1, EXT_LEFT_32 = 2;
+void batched_set_left(BatchBufs *bb, int left);
 BatchBufs *batched_slot_bufs(bwacuda_ctx *c, int slot);  // work buffers of host-pipeline slot 0 or 1
 cudaError_t batched_reserve(BatchBufs *bb, size_t n);
 // registers / threads per SM that bb's bucket kernels leave free (0, 0: none)
