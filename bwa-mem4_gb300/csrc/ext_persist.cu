@@ -114,7 +114,16 @@ __global__ void ext_keys_kernel(const bwacuda_dev_ext_job *__restrict__ jobs, ui
         const bwacuda_dev_ext_job J = jobs[k];
         uint32_t key = ext_sort_key(J, small.on ? ext_small_class(J, max_sc, small)
                                                 : max(ext_cell_class(J, max_sc), min_cls));
-        if (n_to_16 && key < (1u << 20) && J.qlen > 0) {  // an 8-bit job: any code of 4 or more?
+        bool settled = false;
+        if (ug.enabled) {
+            bwacuda_ext_result r;
+            settled = ungapped_hit(seq + J.q_off, J.qlen, seq + J.t_off, J.tlen, J.h0, ug, zdrop, r);
+            if (settled) {
+                out[k] = r;
+                key = 3u << 20;
+            }
+        }
+        if (n_to_16 && !settled && key < (1u << 20) && J.qlen > 0) {  // an 8-bit job: any code of 4 or more?
             uint32_t any = 0u;
             for (int j = 0; j < J.qlen; j += 16) {
                 uint32_t v[4];
@@ -122,13 +131,6 @@ __global__ void ext_keys_kernel(const bwacuda_dev_ext_job *__restrict__ jobs, ui
                 any |= v[0] | v[1] | v[2] | v[3];
             }
             if (any & 0xfcfcfcfcu) key |= 1u << 20;
-        }
-        if (ug.enabled) {
-            bwacuda_ext_result r;
-            if (ungapped_hit(seq + J.q_off, J.qlen, seq + J.t_off, J.tlen, J.h0, ug, zdrop, r)) {
-                out[k] = r;
-                key = 3u << 20;
-            }
         }
         keys[k] = key;
         idx[k] = k;
