@@ -56,6 +56,7 @@ struct BatchBufs {
     ExtParams g_P{};
     int nfan = 0;            // streams and join events that exist
     size_t call_jobs = 0;    // jobs of the whole call when the batch is one chunk of it
+    bool shapes = false;     // the autotuner's runs: length buckets with a job a thread whatever the batch
     int left = EXT_LEFT_16 | EXT_LEFT_32;  // what a small batch may hold besides the band kernel's jobs
     // per-SM room the bucket kernels leave for kernels running beside them
     int reserve_regs = 0, reserve_threads = 0;
@@ -240,6 +241,15 @@ int batched_set_small(bwacuda_ctx *c, size_t jobs)
     return BWACUDA_OK;
 }
 
+// Device-resident calls as the autotuner times them: the launch shapes it turns (threads per block, jobs
+// per grab, bucket width, the group kernel's buckets) are those of the length buckets with a job a thread,
+// so small batches run in buckets too and no bucket runs two jobs a thread.
+void batched_set_shapes(bwacuda_ctx *c, bool on)
+{
+    c->batched->bufs[2].shapes = on;
+    c->batched->gen++;
+}
+
 void batched_get_tuning(bwacuda_ctx *c, int *tb, int *grab, int *step)
 {
     BatchedState *B = c->batched;
@@ -371,12 +381,13 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
 {
     BatchedState *B = c->batched;
     const bool lanes = ext_pair_lanes_ok(P.sc.o_del, P.sc.e_del, P.sc.o_ins, P.sc.e_ins);
-    if (lanes && batched_is_small(c, n, P)) return enqueue_small(c, bb, d_seq, d_jobs, n, P, d_out, s, err, cells);
+    if (lanes && !bb.shapes && batched_is_small(c, n, P))
+        return enqueue_small(c, bb, d_seq, d_jobs, n, P, d_out, s, err, cells);
     const int fan = std::min(batched_fan(c, bb, n), bb.nfan);
     // two jobs a thread in the 8-bit buckets of large batches; not behind the ungapped closed form, which
     // leaves the buckets the jobs whose rows end apart, and few (4M jobs, two / one a thread: read pairs
     // with 1% errors 6.43 / 5.84 ms, mixed lengths 3.98 / 3.79; 8.4M read pairs 2.85 / 2.85)
-    const bool dual = !P.ug.enabled && lanes && P.sc.m <= 5 && n >= (size_t)B->nsm * EXT_DUAL_JOBS_PER_SM;
+    const bool dual = !P.ug.enabled && !bb.shapes && lanes && P.sc.m <= 5 && n >= (size_t)B->nsm * EXT_DUAL_JOBS_PER_SM;
     cudaError_t e = ext_sort_and_bucket(d_jobs, n, P.sc.max_sc, lanes, dual, d_seq, P.ug, P.zdrop, d_out,
                                         static_cast<uint32_t *>(bb.keys_in.p),
                                         static_cast<uint32_t *>(bb.keys_out.p), static_cast<uint32_t *>(bb.idx_in.p),

@@ -157,6 +157,7 @@ int batched_get_long(bwacuda_ctx *c);
 int batched_set_long_lanes(bwacuda_ctx *c, int lanes, bool by_option = false);
 int batched_set_long_slide(bwacuda_ctx *c, int mode);
 int batched_set_small(bwacuda_ctx *c, size_t jobs);
+void batched_set_shapes(bwacuda_ctx *c, bool on);  // batched_prepare must have run
 
 struct BatchBufs;
 int batched_prepare(bwacuda_ctx *c);

@@ -141,7 +141,6 @@ extern "C" int bwacuda_autotune_extend(bwacuda_ctx *c, const uint8_t *d_seq, con
         const bwacuda_stats saved = c->stats;
         // candidates run as the calls they tune do: replayed graphs when the context uses them
         // (each shape is captured on its untimed first run), plain stream launches otherwise
-        const bool graphs = c->use_graphs;
         auto run = [&]() {
             return extend_device_batched(c, d_seq, static_cast<const bwacuda_dev_ext_job *>(jp), count, P,
                                          static_cast<bwacuda_ext_result *>(dout.p), s);
@@ -150,6 +149,12 @@ extern "C" int bwacuda_autotune_extend(bwacuda_ctx *c, const uint8_t *d_seq, con
         uint64_t cells = 0;
         rc = run();
         if (!rc) rc = collect_device_status(c, s, &cells);
+        // the candidates' runs keep to the length buckets with a job a thread: a small sample would
+        // otherwise run without buckets, and the short buckets of a large one two jobs a thread, where
+        // what is turned here has no say and the choice is the timing's noise (on 4.2M read pairs 64
+        // threads before there were such kernels, then 128 or 256 from run to run: 15.3 against 16.1 and
+        // 17.6 ms on as many jobs of the 16-bit class)
+        batched_set_shapes(c, true);
         // Every shape is timed; among those within 1.5% of the fastest the one closest to the
         // default (1 round per grab, 32-column buckets, 128 threads) wins.  Device-resident the
         // near-ties are noise, but a host-buffer call runs every chunk's buckets separately,
@@ -193,7 +198,6 @@ extern "C" int bwacuda_autotune_extend(bwacuda_ctx *c, const uint8_t *d_seq, con
                 best[0] = cd.tb; best[1] = cd.gr; best[2] = cd.st;
             }
         }
-        best_ms = chosen_ms;
         if (!rc) rc = batched_set_bucket_step(c, best[2]);
         if (!rc) rc = batched_set_block(c, best[0]);
         if (!rc) rc = batched_set_grab(c, best[1]);
@@ -218,12 +222,9 @@ extern "C" int bwacuda_autotune_extend(bwacuda_ctx *c, const uint8_t *d_seq, con
                 if (long_ms == 0 || ms < long_ms) { long_ms = ms; long_best = lq; lanes_best = ln; }
             }
         }
-        if (!rc && long_ms > 0 && long_ms * 1.015 < tpj_ms) {
-            best_ms = long_ms;
-        } else {
+        if (rc || long_ms <= 0 || long_ms * 1.015 >= tpj_ms) {
             long_best = INT_MAX;
             lanes_best = lanes0;
-            if (tpj_ms > 0) best_ms = std::min(best_ms, tpj_ms);
         }
         if (!rc) rc = batched_set_long(c, long_best);
         if (!rc) rc = batched_set_long_lanes(c, lanes_best);
@@ -231,10 +232,14 @@ extern "C" int bwacuda_autotune_extend(bwacuda_ctx *c, const uint8_t *d_seq, con
             batched_set_long(c, long0);
             batched_set_long_lanes(c, lanes0);
         }
+        batched_set_shapes(c, false);
+        if (!rc) {  // the sample as calls run it under the choice
+            best_ms = time_runs(T, s, 2, run);
+            if (best_ms < 0) rc = (int)best_ms;
+        }
         uint64_t dummy = 0;
         const int st = collect_device_status(c, s, &dummy);
         if (!rc) rc = st;
-        c->use_graphs = graphs;
         c->stats = saved;
         tmp.release();
         dout.release();
