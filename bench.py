@@ -148,8 +148,9 @@ def apply_tuning(B, ctx, t):
         ctx.set_option(B.OPT_GRAB, t["grab"])
         ctx.set_option(B.OPT_BUCKET_STEP, t["bucket_step"])
         ctx.set_option(B.OPT_RESCUE_KERNEL, t["rescue_kernel"])
-        ctx.set_option(B.OPT_RESCUE_LANES, t["rescue_lanes"])
-        ctx.set_option(B.OPT_RESCUE_PAIR, t.get("rescue_pair", 0))
+        if not t.get("rescue_auto"):  # else each launch picks its shape
+            ctx.set_option(B.OPT_RESCUE_LANES, t["rescue_lanes"])
+            ctx.set_option(B.OPT_RESCUE_PAIR, t.get("rescue_pair", 0))
         ctx.set_option(B.OPT_LONG_QLEN, t.get("long_qlen", 0))
         ctx.set_option(B.OPT_LONG_LANES, t.get("long_lanes", 16))
 

@@ -209,7 +209,7 @@ pub mod ffi {
         pub long_qlen: i32,
         pub long_lanes: i32,
         pub rescue_pair: i32,
-        pub reserved: i32,
+        pub rescue_auto: i32,
     }
 
     extern "C" {

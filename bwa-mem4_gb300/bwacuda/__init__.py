@@ -68,7 +68,7 @@ class Tuning(C.Structure):
     _fields_ = [("persist_block", C.c_int32), ("grab", C.c_int32), ("bucket_step", C.c_int32),
                 ("rescue_lanes", C.c_int32), ("rescue_kernel", C.c_int32), ("candidates", C.c_int32),
                 ("ext_gcups", C.c_double), ("rescue_gcups", C.c_double), ("long_qlen", C.c_int32),
-                ("long_lanes", C.c_int32), ("rescue_pair", C.c_int32), ("reserved", C.c_int32)]
+                ("long_lanes", C.c_int32), ("rescue_pair", C.c_int32), ("rescue_auto", C.c_int32)]
 
     def as_dict(self):
         return {n: getattr(self, n) for n, _ in self._fields_}

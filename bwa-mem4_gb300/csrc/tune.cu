@@ -109,7 +109,7 @@ extern "C" int bwacuda_get_tuning(bwacuda_ctx *c, bwacuda_tuning *out)
     out->long_qlen = lq == INT_MAX ? 0 : lq;
     out->long_lanes = c->long_lanes;
     out->rescue_pair = c->rescue_pair > 0 ? c->rescue_pair : 0;
-    out->reserved = 0;
+    out->rescue_auto = c->rescue_lanes == 0 && c->rescue_pair < 0;
     return BWACUDA_OK;
 }
 

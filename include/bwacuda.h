@@ -470,7 +470,9 @@ typedef struct {
     int32_t long_lanes;     /* lanes per job of the group-per-job kernel: 8, 16 or 32 */
     int32_t rescue_pair;    /* lanes of a group holding two byte-range rescue jobs, 4, 8 or 16 (0: off;
                                BWACUDA_OPT_RESCUE_PAIR) */
-    int32_t reserved;
+    int32_t rescue_auto;    /* 1: neither an option nor the autotuner has set a rescue shape and each launch
+                               picks one by its jobs; rescue_lanes and rescue_pair then are not settings
+                               to copy to another context, which would pin them there */
 } bwacuda_tuning;
 
 int bwacuda_get_tuning(bwacuda_ctx *ctx, bwacuda_tuning *out);
