@@ -463,7 +463,7 @@ int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int 
             break;
         }
         R.busy = true;
-        c->stats.kernel_launches += 3 + 3 + (uint64_t)batched_bucket_count(c);
+        c->stats.kernel_launches += 3 + (uint64_t)batched_launched(batched_slot_bufs(c, (int)(k & 1)));
         const size_t c1 = c0 + cn;
         if (c1 < n) {
             AtsChunk &R1 = c->ats->ring[(k + 1) % ATS_RING];

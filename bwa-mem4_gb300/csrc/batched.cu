@@ -56,6 +56,8 @@ struct BatchBufs {
     ExtParams g_P{};
     int nfan = 0;            // streams and join events that exist
     size_t call_jobs = 0;    // jobs of the whole call when the batch is one chunk of it
+    int launched = 0;        // kernel launches of the last sequence enqueued (the sort counted as one)
+    int g_launched = 0;      // of the captured one
     bool shapes = false;     // the autotuner's runs: length buckets with a job a thread whatever the batch
     int left = EXT_LEFT_16 | EXT_LEFT_32;  // what a small batch may hold besides the band kernel's jobs
     // per-SM room the bucket kernels leave for kernels running beside them
@@ -294,6 +296,7 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
 {
     BatchedState *B = c->batched;
     uint32_t *work = static_cast<uint32_t *>(bb.xl.p);
+    bb.launched = 1;  // the band kernel
     cudaError_t e = cudaMemsetAsync(work, 0, XL_WORK_WORDS * 4, s);
     if (e != cudaSuccess) return e;
     ExtLongLaunch X;
@@ -325,6 +328,7 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
                                bb.tmp.p, bb.tmp.cap, s, &P)) != cudaSuccess)
             return e;
         X.order = order;
+        bb.launched += 2 + (bb.left != 0);
         uint32_t *table = static_cast<uint32_t *>(bb.table.p);
         const uint32_t many = c->long_lanes_set ? UINT32_MAX : (uint32_t)(B->nsm * EXT_SMALL_LEFT8_PER_SM);
         if (bb.left && (e = ext_small_bounds(keys, n, (uint32_t)(B->nsm * EXT_SMALL_WIDE_PER_SM), many,
@@ -342,6 +346,7 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
             L.cells = X.cells;
             L.grab = 1;
             L.stream = s;
+            ++bb.launched;
             if ((e = ext_wide_launch(L, static_cast<const ExtBucketDef *>(B->d_defs.p), B->nb, table, work, B->nsm)) !=
                 cudaSuccess)
                 return e;
@@ -353,18 +358,21 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
         X.counter = work + XL_WORK_COUNTER16;
         X.bounds = X.order ? work + XL_WORK_LEFT : nullptr;
         if ((e = ext_long_launch(X, false, B->nsm)) != cudaSuccess) return e;
+        bb.launched += 2;  // and the deferred launch
         if (X.order && !c->long_lanes_set && n >= (size_t)B->nsm * EXT_SMALL_LEFT8_PER_SM) {
             ExtLongLaunch Y = X;
             Y.lanes = 8;
             Y.counter = work + XL_WORK_COUNTER_MANY;
             Y.bounds = work + XL_WORK_LEFT_MANY;
             if ((e = ext_long_launch(Y, false, B->nsm)) != cudaSuccess) return e;
+            ++bb.launched;
         }
     }
     if (bb.left & EXT_LEFT_32) {
         X.counter = work + XL_WORK_COUNTER32;
         X.bounds = X.order ? work + XL_WORK_WIDE : nullptr;
         if ((e = ext_long_launch(X, true, B->nsm)) != cudaSuccess) return e;
+        bb.launched += 2;
     }
     for (int w32 = 0; w32 < 2; ++w32)
         if ((bb.left & (w32 ? EXT_LEFT_32 : EXT_LEFT_16)) &&
@@ -395,6 +403,7 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
                                         static_cast<const ExtBucketDef *>(B->d_defs.p), B->nb,
                                         static_cast<uint32_t *>(bb.table.p), s);
     if (e != cudaSuccess) return e;
+    bb.launched = 3;  // keys, sort, bounds
     uint32_t *work = static_cast<uint32_t *>(bb.xl.p);
     if ((e = cudaMemsetAsync(work, 0, XL_WORK_WORDS * 4, s)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(bb.fork, s)) != cudaSuccess) return e;
@@ -435,6 +444,7 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
         X.counter = tab + 2;
         const bool w32 = B->defs[b].cls == 2;
         X.band = use_band && !w32 && B->defs[b].qhi == EXT_QHI_OPEN;
+        bb.launched += 1 + (X.band ? 1 + (cut != 0u) : 0);
         if (X.band) {  // one of the two runs the bucket, the other exits at once
             if ((e = ext_band_launch(X, 8, tab + 3, cut, UINT32_MAX, B->nsm)) != cudaSuccess) return e;
             if (cut && (e = ext_band_launch(X, 32, tab + 3, 1u, cut, B->nsm)) != cudaSuccess) return e;
@@ -445,6 +455,7 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
     }
     if (long16 && (e = ext_long_deferred_launch(X, false, work, B->nsm)) != cudaSuccess) return e;
     if (long32 && (e = ext_long_deferred_launch(X, true, work, B->nsm)) != cudaSuccess) return e;
+    bb.launched += (int)long16 + (int)long32;
     PersistLaunch L;
     L.seq = d_seq;
     L.jobs = d_jobs;
@@ -462,6 +473,7 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
     for (int b = B->nb - 1, k = 1; b >= 0; --b) {
         if (B->defs[b].kernel == 1) continue;
         L.stream = bb.fan[k++ % fan];
+        ++bb.launched;
         uint32_t *tab = static_cast<uint32_t *>(bb.table.p) + 4 * b;
         e = dual && B->defs[b].cls == 0 && B->defs[b].qcap <= EXT_DUAL_QCAP ? ext_dual_launch(L, B->defs[b], tab, B->nsm)
                                         : ext_persist_launch(L, B->defs[b], tab, B->nsm, B->tb);
@@ -504,14 +516,16 @@ int extend_device_batched(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda_de
         if (e != cudaSuccess) { bb.graph = nullptr; return cuda_status(e); }
         bb.g_seq = d_seq; bb.g_jobs = d_jobs; bb.g_out = d_out; bb.g_n = n; bb.g_stream = s; bb.g_P = P;
         bb.g_gen = c->batched->gen;
+        bb.g_launched = bb.launched;
         memcpy(bb.g_bufs, bufs, sizeof(bufs));
     }
     if (c->use_graphs) {
         if ((e = cudaGraphLaunch(bb.graph, s)) != cudaSuccess) return cuda_status(e);
+        bb.launched = bb.g_launched;
     } else if ((e = enqueue_batched(c, bb, d_seq, d_jobs, n, P, d_out, s)) != cudaSuccess) {
         return cuda_status(e);
     }
-    c->stats.kernel_launches += 3 + (uint64_t)batched_bucket_count(c);
+    c->stats.kernel_launches += (uint64_t)bb.launched;
     c->stats.ext_jobs += n;
     c->dev_pending_stream = s;
     return BWACUDA_OK;
@@ -527,8 +541,7 @@ void batched_set_call(BatchBufs *bb, size_t jobs) { bb->call_jobs = jobs; }
 void batched_set_left(BatchBufs *bb, int left) { bb->left = left; }
 BatchBufs *batched_slot_bufs(bwacuda_ctx *c, int slot) { return &c->batched->bufs[slot & 1]; }
 int batched_nsm(bwacuda_ctx *c) { return c->batched->nsm; }
-// Launches of the bucket stage: one per bucket and the two deferred group-per-job launches.
-int batched_bucket_count(bwacuda_ctx *c) { return c->batched->nb + 2 + (c->long_slide ? 2 : 0); }
+int batched_launched(const BatchBufs *bb) { return bb->launched; }
 
 static cudaError_t bufs_streams(BatchBufs &bb)
 {
@@ -592,7 +605,7 @@ int extend_batch_host_batched(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_
         BatchBufs &bb = c->batched->bufs[slot];
         cudaError_t e = ensure_bufs(bb, I.n, batched_fan(c, bb, I.n));
         if (e == cudaSuccess) e = enqueue_batched(c, bb, I.d_seq, I.d_jobs, I.n, I.P, I.d_out, s);
-        c->stats.kernel_launches += 3 + (uint64_t)batched_bucket_count(c);
+        if (e == cudaSuccess) c->stats.kernel_launches += (uint64_t)bb.launched;
         return cuda_status(e);
     });
 }

@@ -97,7 +97,7 @@ int retry_rounds(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda_dev_ext_job
     // round 0: every job, results straight into d_out
     e = batched_enqueue(c, batched_slot_bufs(c, 0), d_seq, d_jobs, n, P, d_out, s, nullptr, nullptr);
     if (e != cudaSuccess) return cuda_status(e);
-    c->stats.kernel_launches += 4 + (uint64_t)batched_bucket_count(c);
+    c->stats.kernel_launches += 1 + (uint64_t)batched_launched(batched_slot_bufs(c, 0));
     const bwacuda_dev_ext_job *desc = d_jobs;
     const uint32_t *map = nullptr;
     const bwacuda_ext_result *res = d_out;
@@ -128,7 +128,7 @@ int retry_rounds(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda_dev_ext_job
         e = batched_enqueue(c, batched_slot_bufs(c, 1), d_seq, desc, m, P,
                             static_cast<bwacuda_ext_result *>(R.res.p), s, nullptr, nullptr);
         if (e != cudaSuccess) return cuda_status(e);
-        c->stats.kernel_launches += 4 + (uint64_t)batched_bucket_count(c);
+        c->stats.kernel_launches += (uint64_t)batched_launched(batched_slot_bufs(c, 1));
         c->stats.ext_retry_jobs += m;
     }
     return BWACUDA_OK;

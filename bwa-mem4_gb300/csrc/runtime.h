@@ -176,7 +176,7 @@ cudaError_t batched_reserve(BatchBufs *bb, size_t n);
 void batched_set_reserve(BatchBufs *bb, int regs, int threads);
 int batched_nsm(bwacuda_ctx *c);
 bool batched_is_small(const bwacuda_ctx *c, size_t n, const ExtParams &P);
-int batched_bucket_count(bwacuda_ctx *c);
+int batched_launched(const BatchBufs *bb);  // kernel launches of the last sequence enqueued on bb
 
 // ats.cu
 int extend_batch_ats(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_t n, int m, const int8_t *mat,
