@@ -21,9 +21,9 @@ namespace bwacuda {
 // above, the buckets fill the GPU one after another, and the long ones finish later when they share it
 // from the start.  Device-resident, four streams / eight, microseconds, mixed lengths: 60,000 jobs
 // 2010 / 1240, 120,000 1970 / 1310, 250,000 2110 / 1870, 500,000 2500 / 2770, 1M 3840 / 4340; read
-// pairs: 250,000 1260 / 1120.  The others are created at their first use: every stream of a process
-// takes a place in the few hardware queues, and 2M read pairs through host buffers took 3% longer with
-// eight created and four in use.
+// pairs: 250,000 1260 / 1120.  The others are created at their first use, and small batches, which have
+// no buckets, never ask for them.  Created ones cost later calls nothing: 2M read pairs through host
+// buffers 7.80 ms in a fresh context, 7.73-7.79 after calls that use eight.
 constexpr int FAN = 4, FAN_WIDE = 8;
 constexpr int EXT_WIDE_JOBS_PER_SM = 2200;
 // Open-ended buckets: jobs per SM from which the band kernel gives a job 8 lanes, below it 32 (queries
@@ -218,8 +218,8 @@ int batched_set_long_lanes(bwacuda_ctx *c, int lanes, bool by_option)
     return BWACUDA_OK;
 }
 
-// Window kernel on the open-ended buckets: 0 off, 1 on buckets of a warp of jobs per SM or
-// more, 2 always; a new value invalidates captured graphs.
+// Band kernel on the open-ended buckets: 0 off, 1 with lanes a job by the bucket's jobs, 2 with 8; a new
+// value invalidates captured graphs.
 int batched_set_long_slide(bwacuda_ctx *c, int mode)
 {
     int rc = batched_init(c);
@@ -261,8 +261,9 @@ void batched_get_tuning(bwacuda_ctx *c, int *tb, int *grab, int *step)
 }
 
 // Bucket streams of a batch of n jobs.
-static int batched_fan(const bwacuda_ctx *c, const BatchBufs &bb, size_t n)
+static int batched_fan(const bwacuda_ctx *c, const BatchBufs &bb, size_t n, const ExtParams &P)
 {
+    if (batched_is_small(c, n, P) && ext_pair_lanes_ok(P.sc.o_del, P.sc.e_del, P.sc.o_ins, P.sc.e_ins)) return FAN;
     return std::max(n, bb.call_jobs) < (size_t)c->batched->nsm * EXT_WIDE_JOBS_PER_SM ? FAN_WIDE : FAN;
 }
 
@@ -391,7 +392,7 @@ static cudaError_t enqueue_batched(bwacuda_ctx *c, BatchBufs &bb, const uint8_t 
     const bool lanes = ext_pair_lanes_ok(P.sc.o_del, P.sc.e_del, P.sc.o_ins, P.sc.e_ins);
     if (lanes && !bb.shapes && batched_is_small(c, n, P))
         return enqueue_small(c, bb, d_seq, d_jobs, n, P, d_out, s, err, cells);
-    const int fan = std::min(batched_fan(c, bb, n), bb.nfan);
+    const int fan = std::min(batched_fan(c, bb, n, P), bb.nfan);
     // two jobs a thread in the 8-bit buckets of large batches; not behind the ungapped closed form, which
     // leaves the buckets the jobs whose rows end apart, and few (4M jobs, two / one a thread: read pairs
     // with 1% errors 6.43 / 5.84 ms, mixed lengths 3.98 / 3.79; 8.4M read pairs 2.85 / 2.85)
@@ -492,7 +493,7 @@ int extend_device_batched(bwacuda_ctx *c, const uint8_t *d_seq, const bwacuda_de
     int rc = batched_init(c);
     if (rc) return rc;
     BatchBufs &bb = c->batched->bufs[2];
-    cudaError_t e = ensure_bufs(bb, n, batched_fan(c, bb, n));
+    cudaError_t e = ensure_bufs(bb, n, batched_fan(c, bb, n, P));
     if (e != cudaSuccess) return cuda_status(e);
     // Replay a captured graph when the same batch comes back (same buffers, size,
     // scoring and stream); otherwise capture a new one.
@@ -582,7 +583,7 @@ cudaError_t batched_enqueue(bwacuda_ctx *c, BatchBufs *bb, const uint8_t *d_seq,
                             size_t n, const ExtParams &P, bwacuda_ext_result *d_out, cudaStream_t s, uint32_t *err,
                             unsigned long long *cells)
 {
-    cudaError_t e = ensure_bufs(*bb, batched_grow_jobs(*bb, n), batched_fan(c, *bb, n));
+    cudaError_t e = ensure_bufs(*bb, batched_grow_jobs(*bb, n), batched_fan(c, *bb, n, P));
     if (e != cudaSuccess) return e;
     return enqueue_batched(c, *bb, d_seq, d_jobs, n, P, d_out, s, err, cells);
 }
@@ -603,7 +604,7 @@ int extend_batch_host_batched(bwacuda_ctx *c, const bwacuda_ext_job *jobs, size_
     if (rc) return rc;
     return extend_host_pipeline(c, jobs, n, m, mat, P, w, out, [c](int slot, const ExtChunkInfo &I, cudaStream_t s) {
         BatchBufs &bb = c->batched->bufs[slot];
-        cudaError_t e = ensure_bufs(bb, I.n, batched_fan(c, bb, I.n));
+        cudaError_t e = ensure_bufs(bb, I.n, batched_fan(c, bb, I.n, I.P));
         if (e == cudaSuccess) e = enqueue_batched(c, bb, I.d_seq, I.d_jobs, I.n, I.P, I.d_out, s);
         if (e == cudaSuccess) c->stats.kernel_launches += (uint64_t)bb.launched;
         return cuda_status(e);

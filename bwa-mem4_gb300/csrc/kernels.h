@@ -73,7 +73,7 @@ struct ExtLongLaunch {
 };
 
 cudaError_t ext_long_launch(const ExtLongLaunch &X, bool w32, int nsm);
-// Batched calls of up to this many jobs per SM run unsorted in the band kernel, and host calls of up
+// Batched calls of up to this many jobs per SM run without length buckets in the band kernel, and host calls of up
 // to this many straight from the caller's arrays.  Device-resident calls on 152 SMs, microseconds
 // (read pairs / mixed lengths):
 //   jobs       sorted buckets   8 lanes (sorted)  16        32 lanes a job

@@ -100,7 +100,7 @@ struct bwacuda_ctx {
     int long_lanes = 16;    // lanes per job of the group-per-job extension kernel (8, 16, 32)
     bool long_lanes_set = false;  // BWACUDA_OPT_LONG_LANES was set
     int long_slide = 1;     // band kernel on the open-ended buckets: 0 off, 1 lanes by the bucket's jobs, 2 always 8 lanes
-    size_t small_jobs = 0;  // batched calls of up to this many jobs run unsorted in the band kernel (set from the SM count)
+    size_t small_jobs = 0;  // batched calls of up to this many jobs run without length buckets in the band kernel (set from the SM count)
     int tune_candidates = 0;        // last autotune call
     double tuned_ext_gcups = 0.0;   // best candidates' rates on their samples
     double tuned_rescue_gcups = 0.0;
