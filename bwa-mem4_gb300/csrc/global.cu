@@ -853,7 +853,6 @@ __global__ void glb_warp_groups_kernel(const int4 *__restrict__ dims, const uint
             sizes[w] = (uint64_t)((rows + 1u) / 2u) * ng * 512u;
             if (w < ngroups_max) {
                 gtag::WarpGroup g;
-                g.z_off = 0;
                 g.pos = pos;
                 g.count = (uint16_t)count;
                 g.ng = (uint16_t)ng;
@@ -863,14 +862,6 @@ __global__ void glb_warp_groups_kernel(const int4 *__restrict__ dims, const uint
     }
 }
 
-// The groups' offsets, once scanned.
-__global__ void glb_group_offsets_kernel(const uint64_t *__restrict__ offs, uint32_t ngroups,
-                                         gtag::WarpGroup *__restrict__ groups)
-{
-    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < ngroups; w += gridDim.x * blockDim.x)
-        groups[w].z_off = offs[w];
-}
-
 // Traceback over the tagged kernel's directions (sw.rs:700-738): warps 2w and 2w + 1 walk group w's
 // first and second alignments of the pairs, lane for lane as the DP's threads lay, so a warp's loads
 // fall into the same 512-byte rows.  In state M the walk usually stays on the diagonal, which keeps its
@@ -878,13 +869,14 @@ __global__ void glb_group_offsets_kernel(const uint64_t *__restrict__ offs, uint
 __global__ void __launch_bounds__(256) glb_tag_traceback_kernel(const GlobalDevJob *__restrict__ jobs,
                                                                 const uint32_t *__restrict__ order,
                                                                 const gtag::WarpGroup *__restrict__ groups,
+                                                                const uint64_t *__restrict__ zoffs, uint32_t g0,
                                                                 uint32_t ngroups, gtag::TagRule tr,
                                                                 const uint8_t *__restrict__ z,
                                                                 uint32_t *__restrict__ cig, int32_t *__restrict__ ncig)
 {
     const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t x = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < 2 * ngroups; x += (gridDim.x * blockDim.x) >> 5) {
-        const gtag::WarpGroup wg = groups[x >> 1];
+        const gtag::WarpGroup wg = groups[g0 + (x >> 1)];
         const uint32_t half = x & 1u, at = 2 * lane + half;
         if (at >= wg.count) continue;
         const uint32_t k = order[wg.pos + at];
@@ -896,7 +888,7 @@ __global__ void __launch_bounds__(256) glb_tag_traceback_kernel(const GlobalDevJ
             const gtag::PairGeo g = gtag::pair_geo(J.qlen, J.tlen, J.w, true, O.qlen, O.tlen, O.w, tr);
             if (g.dual) wl = g.wl;
         }
-        const uint32_t *zw = reinterpret_cast<const uint32_t *>(z + wg.z_off) + lane * 4u + half;
+        const uint32_t *zw = reinterpret_cast<const uint32_t *>(z + (zoffs[g0 + (x >> 1)] - zoffs[0])) + lane * 4u + half;
         const size_t prow = (size_t)wg.ng * 128u;  // words of a row pair
         uint32_t *cg = cig + J.cig_off;
         int nc = 0, i = J.tlen - 1, j = J.qlen - 1;
@@ -970,9 +962,7 @@ __global__ void __launch_bounds__(256) glb_tag_traceback_kernel(const GlobalDevJ
 // so the caller's job array crosses the host link once) and copies the slices as aligned 16-byte
 // words (warp_gather_slices).
 __global__ void __launch_bounds__(256) glb_gather_kernel(const uint32_t *__restrict__ order, uint32_t base, uint32_t count,
-                                                         const uint64_t *__restrict__ seq_off,
-                                                         const uint64_t *__restrict__ cig_off,
-                                                         const uint64_t *__restrict__ z_off,
+                                                         const uint64_t *__restrict__ offs, uint32_t n1,
                                                          uint8_t *__restrict__ seq, GlobalDevJob *__restrict__ dj)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -984,15 +974,15 @@ __global__ void __launch_bounds__(256) glb_gather_kernel(const uint32_t *__restr
         if (x < count) {
             const uint32_t k = order[base + x];
             GlobalDevJob D = dj[k];
-            at = seq_off[k];
+            at = offs[k];
             qa = D.q_off;
             ta = D.t_off;
             qw = slice_words(reinterpret_cast<const uint8_t *>(qa), D.qlen);
             tw = slice_words(reinterpret_cast<const uint8_t *>(ta), D.tlen);
             D.q_off = at + (qa & 15);
             D.t_off = at + 16ull * qw + (ta & 15);
-            D.z_off = z_off[k];
-            D.cig_off = cig_off[k];
+            D.cig_off = offs[n1 + k] - offs[n1];
+            D.z_off = offs[2 * (size_t)n1 + k] - offs[2 * (size_t)n1];
             dj[k] = D;
         }
         warp_gather_slices<false>(qa & ~15ull, ta & ~15ull, at, qw, tw, seq);
@@ -1105,7 +1095,8 @@ cudaError_t launch_global(const uint8_t *seq, const GlobalDevJob *jobs, const ui
 template <int TB>
 cudaError_t launch_tag_tb(const uint8_t *seq, const GlobalDevJob *jobs, const uint32_t *order, uint32_t start,
                           uint32_t count, const Scoring &sc, const gtag::TagRule &tr, int max_slots, int max_sel,
-                          size_t smem, const gtag::WarpGroup *groups, uint32_t gbase, uint8_t *z, int32_t *score,
+                          size_t smem, const gtag::WarpGroup *groups, const uint64_t *zoffs, uint32_t gbase, uint8_t *z,
+                          int32_t *score,
                           int32_t *ncig, uint32_t *err, unsigned long long *cells, cudaStream_t s)
 {
     const bool sym = sc.o_del + sc.e_del == sc.o_ins + sc.e_ins;
@@ -1116,7 +1107,7 @@ cudaError_t launch_tag_tb(const uint8_t *seq, const GlobalDevJob *jobs, const ui
     const uint32_t threads = tr.single ? count : (count + 1) / 2;
     const uint32_t blocks = (threads + TB - 1) / TB;
     kern<<<tr.single ? blocks : 2 * blocks, TB, smem, s>>>(seq, jobs, order, start, count, sc, tr, max_slots, max_sel,
-                                                          groups, gbase, z, score, ncig, GLB_TB_TAGGED, ERR_RANGE, err,
+                                                          groups, zoffs, gbase, z, score, ncig, GLB_TB_TAGGED, ERR_RANGE, err,
                                                           cells);
     return cudaGetLastError();
 }
@@ -1126,7 +1117,8 @@ size_t tag_smem(int wl, int wr, int qmax, int tb) { return gtag::thread_bytes(wl
 
 cudaError_t launch_tag(const uint8_t *seq, const GlobalDevJob *jobs, const uint32_t *order, uint32_t start,
                        uint32_t count, const Scoring &sc, const gtag::TagRule &tr, int wl, int wr, int qmax,
-                       const gtag::WarpGroup *groups, uint32_t gbase, uint8_t *z, int32_t *score, int32_t *ncig,
+                       const gtag::WarpGroup *groups, const uint64_t *zoffs, uint32_t gbase, uint8_t *z, int32_t *score,
+                       int32_t *ncig,
                        uint32_t *err, unsigned long long *cells, cudaStream_t s)
 {
     int best = 32, warps = 0;
@@ -1142,12 +1134,12 @@ cudaError_t launch_tag(const uint8_t *seq, const GlobalDevJob *jobs, const uint3
     const int ms = gtag::slots(wl, wr), mq = (gtag::sel_count(qmax, wl, wr) + 3) & ~3;
     const size_t smem = tag_smem(wl, wr, qmax, best);
     if (best == 128)
-        return launch_tag_tb<128>(seq, jobs, order, start, count, sc, tr, ms, mq, smem, groups, gbase, z, score, ncig,
+        return launch_tag_tb<128>(seq, jobs, order, start, count, sc, tr, ms, mq, smem, groups, zoffs, gbase, z, score, ncig,
                                   err, cells, s);
     if (best == 64)
-        return launch_tag_tb<64>(seq, jobs, order, start, count, sc, tr, ms, mq, smem, groups, gbase, z, score, ncig,
+        return launch_tag_tb<64>(seq, jobs, order, start, count, sc, tr, ms, mq, smem, groups, zoffs, gbase, z, score, ncig,
                                  err, cells, s);
-    return launch_tag_tb<32>(seq, jobs, order, start, count, sc, tr, ms, mq, smem, groups, gbase, z, score, ncig, err,
+    return launch_tag_tb<32>(seq, jobs, order, start, count, sc, tr, ms, mq, smem, groups, zoffs, gbase, z, score, ncig, err,
                              cells, s);
 }
 
@@ -1294,18 +1286,21 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         // pairs.  From there to 20,000 the two are within 4% (9,000 0.80 / 0.815, 18,000 0.84 / 0.855),
         // then pairs lead: 28,000 0.93 / 0.885, 80,000 1.39 / 1.06
         trule.single = cn < (size_t)nsm * 32;
-        // planning arrays: seq / cig / z sizes and offsets (cn + 1 each), keys and indices (two
-        // copies each for the sort)
+        // planning arrays: one list of sizes and its running sum (sequence bytes, CIGAR words and direction
+        // bytes of every alignment, cn + 1 each, the last 0, then the direction bytes of the tagged kernel's
+        // warp groups; a part's offsets count from its first), keys and indices (two copies each for the
+        // sort).  A scan for each, and a kernel that stored the groups' offsets, made 300 alignments past the
+        // tagged kernel's bands 0.79 ms instead of 0.76.
         const size_t n1 = cn + 1;
         const size_t ngmax = cn / 64 + GLB_NBUCKETS, g1n = ngmax + 1;
-        if ((e = b.d_sz.ensure(n1 * 6 * 8 + n1 * 16 + n1 * 4 * 4 + g1n * 16 + 256)) != cudaSuccess) break;
+        const size_t nsz = 3 * n1 + g1n;
+        if ((e = b.d_sz.ensure(nsz * 2 * 8 + n1 * 16 + n1 * 4 * 4 + 256)) != cudaSuccess) break;
         if ((e = b.d_groups.ensure(g1n * sizeof(gtag::WarpGroup))) != cudaSuccess) break;
-        uint64_t *seq_sz = static_cast<uint64_t *>(b.d_sz.p), *seq_off = seq_sz + n1;
-        uint64_t *cig_sz = seq_off + n1, *cig_off = cig_sz + n1;
-        uint64_t *z_sz = cig_off + n1, *z_off = z_sz + n1;
-        uint64_t *tz_sz = z_off + n1, *tz_off = tz_sz + g1n;  // the tagged kernel's warp groups
+        uint64_t *sizes = static_cast<uint64_t *>(b.d_sz.p), *offs = sizes + nsz;
+        uint64_t *seq_sz = sizes, *cig_sz = seq_sz + n1, *z_sz = cig_sz + n1, *tz_sz = z_sz + n1;
+        const uint64_t *tz_off = offs + 3 * n1;
         // 16-byte records from an aligned start
-        int4 *dims = reinterpret_cast<int4 *>((reinterpret_cast<uintptr_t>(tz_off + g1n) + 15) & ~(uintptr_t)15);
+        int4 *dims = reinterpret_cast<int4 *>((reinterpret_cast<uintptr_t>(offs + nsz) + 15) & ~(uintptr_t)15);
         uint32_t *keys = reinterpret_cast<uint32_t *>(dims + n1), *keys2 = keys + n1;
         uint32_t *idx = keys2 + n1, *order = idx + n1;
         gtag::WarpGroup *wgroups = static_cast<gtag::WarpGroup *>(b.d_groups.p);
@@ -1314,7 +1309,7 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         uint32_t *flags = static_cast<uint32_t *>(b.d_flags.p);
         uint32_t *bstat = flags + 16, *bounds = flags + 48, *bwide = flags + 80;
         size_t t1 = 0, t2 = 0, t3 = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, t1, (const uint64_t *)nullptr, (uint64_t *)nullptr, (int)cn + 1);
+        cub::DeviceScan::ExclusiveSum(nullptr, t1, (const uint64_t *)nullptr, (uint64_t *)nullptr, (int64_t)nsz);
         cub::DeviceScan::ExclusiveSum(nullptr, t2, (const int32_t *)nullptr, (uint64_t *)nullptr, (int)cn + 1);
         cub::DeviceRadixSort::SortPairs(nullptr, t3, (const uint32_t *)nullptr, (uint32_t *)nullptr,
                                         (const uint32_t *)nullptr, (uint32_t *)nullptr, (int)cn, 0, 32);
@@ -1329,25 +1324,21 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         glb_plan_kernel<<<grid, 256, 0, s>>>(hj, (uint32_t)cn, qlim, nrule, trule, seq_sz, cig_sz, z_sz, keys, idx, flags,
                                              bstat, bwide, dims, dj);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
-        if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, seq_sz, seq_off, (int)cn + 1, s)) != cudaSuccess) break;
-        if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, cig_sz, cig_off, (int)cn + 1, s)) != cudaSuccess) break;
-        if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, z_sz, z_off, (int)cn + 1, s)) != cudaSuccess) break;
         if ((e = cub::DeviceRadixSort::SortPairs(b.d_tmp.p, t3, keys, keys2, idx, order, (int)cn, 0, 32, s)) != cudaSuccess)
             break;
         glb_bucket_bounds_kernel<<<1, 32, 0, s>>>(keys2, (uint32_t)cn, bounds);
         glb_warp_groups_kernel<<<(uint32_t)std::min<size_t>((g1n * 32 + 255) / 256, (size_t)nsm * 8), 256, 0, s>>>(
             dims, order, bounds, trule, (uint32_t)ngmax, wgroups, tz_sz);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
-        if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, tz_sz, tz_off, (int)g1n, s)) != cudaSuccess) break;
-        glb_group_offsets_kernel<<<(uint32_t)std::min<size_t>((ngmax + 255) / 256, 1024), 256, 0, s>>>(
-            tz_off, (uint32_t)ngmax, wgroups);
-        if ((e = cudaGetLastError()) != cudaSuccess) break;
-        if ((e = cudaMemcpyAsync(ht + 0, seq_off + cn, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
-        if ((e = cudaMemcpyAsync(ht + 1, cig_off + cn, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
-        if ((e = cudaMemcpyAsync(ht + 2, z_off + cn, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
-        if ((e = cudaMemcpyAsync(ht + 3, tz_off + ngmax, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
+        if ((e = cub::DeviceScan::ExclusiveSum(b.d_tmp.p, t1, sizes, offs, (int64_t)nsz, s)) != cudaSuccess) break;
+        // where the second to fourth part begin, and the last one's end
+        if ((e = cudaMemcpy2DAsync(ht + 124, 8, offs + n1, n1 * 8, 8, 3, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
+        if ((e = cudaMemcpyAsync(ht + 127, tz_off + ngmax, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(ht + 4, flags, 512, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) break;
+        // bytes of the sequences, CIGAR words, direction bytes of the untagged and of the tagged alignments
+        ht[0] = ht[124];
+        for (int x = 1; x < 4; ++x) ht[x] = ht[124 + x] - ht[123 + x];
         const uint32_t *hf = reinterpret_cast<const uint32_t *>(ht + 4);
         if (hf[0] & 1u) {
             // an invalid job, or a query longer than the kernel takes: find which on the host
@@ -1395,7 +1386,7 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
                 const int tb = nl ? 128 : 256;
                 const size_t most = nl ? ((size_t)nsm + 1) / 2 : (size_t)nsm * 8;
                 glb_gather_kernel<<<(uint32_t)std::min<size_t>((gn + tb - 1) / tb, most), tb, 0, s>>>(
-                    trule.single ? idx : order, g0, gn, seq_off, cig_off, z_off, static_cast<uint8_t *>(b.d_seq.p), dj);
+                    trule.single ? idx : order, g0, gn, offs, (uint32_t)n1, static_cast<uint8_t *>(b.d_seq.p), dj);
                 if ((e = cudaGetLastError()) != cudaSuccess) break;
                 c->stats.kernel_launches += 1;
             }
@@ -1403,12 +1394,12 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
             if (bs != s && (e = cudaStreamWaitEvent(bs, G.ready, 0)) != cudaSuccess) break;
             if (bk < GLB_NBUCKETS) {
                 e = launch_tag(sq, dj, order, b0, cnt, sc, trule, (int)hbw[bk], (int)hb[2 * bk], (int)hb[2 * bk + 1],
-                               wgroups, gfirst[bk], static_cast<uint8_t *>(b.d_tz.p), d_score, d_ncig, d_err, d_cells,
+                               wgroups, tz_off, gfirst[bk], static_cast<uint8_t *>(b.d_tz.p), d_score, d_ncig, d_err, d_cells,
                                bs);
                 if (e != cudaSuccess) break;
                 const uint32_t ng = gfirst[bk + 1] - gfirst[bk];
                 glb_tag_traceback_kernel<<<(uint32_t)std::min<size_t>(((size_t)ng * 64 + 255) / 256, (size_t)nsm * 8), 256,
-                                           0, bs>>>(dj, order, wgroups + gfirst[bk], ng, trule,
+                                           0, bs>>>(dj, order, wgroups, tz_off, gfirst[bk], ng, trule,
                                                     static_cast<const uint8_t *>(b.d_tz.p),
                                                     static_cast<uint32_t *>(b.d_cig.p), d_ncig);
                 e = cudaGetLastError();
@@ -1440,7 +1431,7 @@ int global_batch_device(bwacuda_ctx *c, const bwacuda_global_job *jobs, size_t n
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) break;
         if (!cigar || out_base + ht[100] > cigar_cap) short_buf = true;
         out_base += ht[100];
-        c->stats.kernel_launches += 12;
+        c->stats.kernel_launches += 5;  // plan, sort, bounds, warp groups, store
     }
     if (e != cudaSuccess) return cuda_status(e);
     if (rc) {

@@ -159,9 +159,9 @@ __host__ __device__ inline PairGeo pair_geo(int q0, int t0, int w0, bool has1, i
     return g;
 }
 
-// The directions of sixty-four consecutive sorted alignments (a warp's pairs): where they lie and how.
+// The directions of sixty-four consecutive sorted alignments (a warp's pairs): how they lie; where is
+// the running sum of the groups' bytes.
 struct WarpGroup {
-    uint64_t z_off;     // bytes from the start of the direction buffer
     uint32_t pos;       // first sorted position
     uint16_t count;     // alignments, at most 64
     uint16_t ng;        // groups of eight steps a row pair holds
@@ -249,7 +249,8 @@ template <int TB, bool SYM, typename JobT>
 __global__ void __launch_bounds__(TB, 384 / TB)
 tag_kernel(const uint8_t *__restrict__ seq, const JobT *__restrict__ jobs, const uint32_t *__restrict__ order,
            uint32_t start, uint32_t count, const __grid_constant__ Scoring sc, const __grid_constant__ TagRule rule,
-           int max_slots, int max_sel, const WarpGroup *__restrict__ wgroups, uint32_t gbase, uint8_t *__restrict__ z,
+           int max_slots, int max_sel, const WarpGroup *__restrict__ wgroups, const uint64_t *__restrict__ zoffs,
+           uint32_t gbase, uint8_t *__restrict__ z,
            int32_t *__restrict__ score_out, int32_t *__restrict__ ncig_out, int done, uint32_t range_flag,
            uint32_t *__restrict__ err, unsigned long long *__restrict__ cells_total)
 {
@@ -278,7 +279,7 @@ tag_kernel(const uint8_t *__restrict__ seq, const JobT *__restrict__ jobs, const
     const PairGeo first = pair_geo(A0.qlen, A0.tlen, A0.w, has1, B0.qlen, B0.tlen, B0.w, rule);
     if (rest && (first.dual || !has1)) return;
     const WarpGroup wg = wgroups[gbase + (t >> 5)];
-    uint4 *zw = reinterpret_cast<uint4 *>(z + wg.z_off) + (t & 31u);
+    uint4 *zw = reinterpret_cast<uint4 *>(z + (zoffs[gbase + (t >> 5)] - zoffs[0])) + (t & 31u);
     TagGaps gp;
     gp.noe_del = both(-4 * (sc.o_del + sc.e_del));
     gp.noe_ins = both(-4 * (sc.o_ins + sc.e_ins));

@@ -3,8 +3,9 @@ work among them)."""
 import re
 
 
-def kernels(fn):
-    """Names without arguments of the kernels fn() launches; None where the trace is not to be had."""
+def kernels(fn, library=False):
+    """Names without arguments of the kernels fn() launches (library: and those of the sorts and scans); None
+    where the trace is not to be had."""
     import torch
     from torch.profiler import ProfilerActivity, profile
 
@@ -14,7 +15,8 @@ def kernels(fn):
             fn()
             torch.cuda.synchronize()
         names = [re.sub(r"^void ", "", e.name).replace("(anonymous namespace)::", "").split("(")[0] for e in p.events()]
-        names = [n.replace("bwacuda::", "").strip() for n in names if n.startswith("bwacuda::") or "bwacuda::" in n]
+        names = [n.replace("bwacuda::", "").strip() for n in names
+                 if "bwacuda::" in n or (library and n.startswith("cub::"))]
         if names:
             return names
     return None

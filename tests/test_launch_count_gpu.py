@@ -1,5 +1,5 @@
 """The kernel_launches statistic against the kernels a call launches (the device's own trace): small batches,
-length buckets, captured and replayed graphs, host calls and the retry rounds."""
+length buckets, captured and replayed graphs, host calls, the retry rounds and the CIGAR stage."""
 import numpy as np
 import pytest
 
@@ -60,3 +60,17 @@ def test_retry_rounds():
     with B.Context(0) as ctx:
         ctx.set_option(B.OPT_HOST_GATHER, B.GATHER_HOST)
         _check(ctx, lambda: ctx.extend_batch_retry(js, None, 2, w=3), 0)
+
+
+@pytest.mark.parametrize("n", [300, 6000])
+@pytest.mark.parametrize("w", [20, 200], ids=["tagged", "untagged"])
+def test_cigar_stage(w, n):
+    rng = np.random.default_rng(n)
+    ts = [rng.integers(0, 4, 150).astype(np.uint8) for _ in range(n)]
+    js = B.JobSet.from_lists(ts, ts, None, w)
+    with B.Context(0) as ctx:
+        call = lambda: ctx.ksw_global2_batch(js)  # noqa: E731
+        _check(ctx, call, 1)
+        # no more launches than before there was a tagged kernel: 16 at 300 alignments, 21 at 6,000, whose
+        # sort is six kernels instead of one
+        assert len(kernels(call, library=True)) <= (16 if n == 300 else 21)
