@@ -23,7 +23,9 @@
 // Columns left of beg hold H = E = 0 (the one the band drops is zeroed before the row; the ones the
 // live-cell scan passes are zero already) and beg never decreases, so the pairs left of p0 that the
 // leading lanes' chunks reach add nothing to M, E, F or the maximum and stay 0: no per-pair test.
-// A chunk that lies left of p0 altogether is moved into the PAD zero words in front of the row.
+// A chunk that lies left of p0 altogether is moved into the PAD zero words in front of the row.  S has
+// PAD selectors of its own in front, of code 0 like those past the query: without their sign bytes a score
+// of -65 or less reads as one near -32768, and a large gap open takes that around to a positive F.
 // Column `end` in an odd last pair is masked to zero on the way in and out of the maximum; it then
 // receives the sentinel (H of the last column, E = 0) by the ordinary stores.  The live-cell scans
 // of the adaptive band (sw.rs:465-482) look at the first and last cell, and probe L columns at once
@@ -55,7 +57,7 @@ static_assert(8 * kmax<8>() >= BAND_PAIRS && 16 * kmax<16>() >= BAND_PAIRS && 32
 template <int L>
 constexpr int pad() { return (kmax<L>() + 3) / 4 * 4; }
 template <int L>
-constexpr int row_words() { return 2 * (pad<L>() + PAIRS) + (PAIRS + 1) / 2; }  // X, Y, S (16 bits a pair)
+constexpr int row_words() { return 2 * (pad<L>() + PAIRS) + (pad<L>() + PAIRS + 1) / 2; }  // X, Y, S (16 bits a pair)
 // Shared words of a job: L modulo 32, so that with odd chunk lengths the warp's 32 lanes hit 32 banks
 // (lane k's word is k * K modulo L, each residue once; the jobs then differ by multiples of L).
 template <int L>
@@ -191,7 +193,7 @@ __device__ __forceinline__ bwacuda_ext_result band_run(uint32_t *__restrict__ sm
     constexpr int PAD = pad<L>();
     const int lane = threadIdx.x & 31, k = lane & (L - 1);
     uint32_t *X = sm + PAD, *Y = X + PAIRS + PAD;
-    uint16_t *S = reinterpret_cast<uint16_t *>(Y + PAIRS);
+    uint16_t *S = reinterpret_cast<uint16_t *>(Y + PAIRS) + PAD;
     uint16_t *X16 = reinterpret_cast<uint16_t *>(X), *Y16 = reinterpret_cast<uint16_t *>(Y);
     const int m = P.sc.m;
     const int o_del = P.sc.o_del, e_del = P.sc.e_del, o_ins = P.sc.o_ins, e_ins = P.sc.e_ins;
@@ -208,6 +210,7 @@ __device__ __forceinline__ bwacuda_ext_result band_run(uint32_t *__restrict__ sm
     for (int p = k; p < PAD; p += L) {
         X[p - PAD] = 0u;
         Y[p - PAD] = 0u;
+        S[p - PAD] = 0x8080u;
     }
     const bool moves = act && qlen + 4 > WC, any_moves = __any_sync(FULL, moves);
     uint32_t cells = 0;
