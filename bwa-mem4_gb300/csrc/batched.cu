@@ -316,6 +316,7 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
     X.defer = work + XL_WORK_WORDS;
     X.defer_count = work + XL_WORK_DCOUNT;
     X.band = 1;
+    X.small = 1;
     X.reserve_regs = bb.reserve_regs;
     X.reserve_threads = bb.reserve_threads;
     X.sm_regs = B->sm_regs;

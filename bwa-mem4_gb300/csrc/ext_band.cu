@@ -60,7 +60,9 @@ ext_band_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__re
             jid = order ? order[pos] : pos;
             act = jid < njobs;  // the group-per-job kernel flags an index past the jobs
             if (act) J = jobs[jid];
-            act = act && J.qlen >= 0 && J.tlen >= 0 && J.qlen >= min_qlen &&
+            // a negative target length: an empty target where a bucket's thread takes it so, else the
+            // group-per-job kernel's to flag
+            act = act && J.qlen >= 0 && (J.tlen >= 0 || J.qlen <= EXT_TPJ_QLEN_MAX) && J.qlen >= min_qlen &&
                   ext_fits_i16(J.qlen, J.tlen, J.h0, P.sc.max_sc);
             if (act) {
                 w = clamp_band(J.w < 0 ? 0 : J.w, J.qlen, P.sc.max_sc, P.end_bonus, P.sc.o_ins, P.sc.e_ins,

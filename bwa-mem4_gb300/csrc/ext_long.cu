@@ -46,7 +46,7 @@ cudaError_t launch_first(const ExtLongLaunch &X, int nsm)
     const size_t most = ((size_t)X.njobs * L + XL_BLOCK - 1) / XL_BLOCK;
     const uint32_t grid = (uint32_t)std::min<size_t>((size_t)per_sm * nsm, std::max<size_t>(most, 1));
     kern<<<grid, XL_BLOCK, smem, X.stream>>>(X.seq, X.jobs, X.order, X.bounds, X.counter, X.njobs, X.min_qlen, ring,
-                                            X.defer, X.defer_count, W32 ? 0 : X.band, X.P, X.out, X.err,
+                                            X.defer, X.defer_count, W32 ? 0 : X.band, X.small, X.P, X.out, X.err,
                                             X.cells);
     return cudaGetLastError();
 }
@@ -71,8 +71,8 @@ cudaError_t launch_deferred(const ExtLongLaunch &X, const uint32_t *count, uint3
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EXT_SMEM_BLOCK_MAX);
     if (e != cudaSuccess) return e;
     const uint32_t grid = (uint32_t)std::min<size_t>((size_t)nsm, std::max<size_t>(X.njobs, 1));
-    kern<<<grid, TB, smem, X.stream>>>(X.seq, X.jobs, X.defer, count, counter, counter_all, X.njobs, X.P, X.out, X.err,
-                                       X.cells);
+    kern<<<grid, TB, smem, X.stream>>>(X.seq, X.jobs, X.defer, count, counter, counter_all, X.njobs, X.small, X.P, X.out,
+                                       X.err, X.cells);
     return cudaGetLastError();
 }
 

@@ -36,6 +36,7 @@
 
 #include "common.cuh"
 #include "ext_job.cuh"
+#include "kernels.h"
 
 namespace bwacuda {
 namespace xl {
@@ -162,7 +163,7 @@ enum class Unfit { DEFER, SKIP, FAIL };
 template <bool W32, int L, int C>
 __device__ void run_warp(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__restrict__ jobs,
                          const uint32_t *__restrict__ order, uint32_t pos, uint32_t stop, uint32_t njobs, int min_qlen,
-                         const Ring<W32> &ring, int ring_cols, Unfit unfit, uint32_t *__restrict__ defer,
+                         const Ring<W32> &ring, int ring_cols, int small, Unfit unfit, uint32_t *__restrict__ defer,
                          uint32_t *__restrict__ defer_count, int band_beside, const ExtParams &P,
                          bwacuda_ext_result *__restrict__ out, uint32_t *__restrict__ err, unsigned long long &ncells)
 {
@@ -184,7 +185,7 @@ __device__ void run_warp(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_
             J = jobs[jid];
         }
     }
-    if (active && (J.qlen < 0 || J.tlen < 0)) {
+    if (active && (J.qlen < 0 || (J.tlen < 0 && !(small && J.qlen <= EXT_TPJ_QLEN_MAX)))) {
         if (k == 0) atomicOr(err, ERR_RANGE);
         active = false;
     }
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(128)
 ext_long_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__restrict__ jobs,
                 const uint32_t *__restrict__ order, const uint32_t *__restrict__ bounds,
                 uint32_t *__restrict__ counter, uint32_t njobs, int min_qlen, int ring_cols,
-                uint32_t *__restrict__ defer, uint32_t *__restrict__ defer_count, int band_beside,
+                uint32_t *__restrict__ defer, uint32_t *__restrict__ defer_count, int band_beside, int small,
                 const __grid_constant__ ExtParams P, bwacuda_ext_result *__restrict__ out,
                 uint32_t *__restrict__ err, unsigned long long *__restrict__ cells_total)
 {
@@ -442,7 +443,7 @@ ext_long_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__re
         base = __shfl_sync(FULL, base, 0);
         if (base >= stop - start) break;
         run_warp<W32, L, C>(seq, jobs, order, start + base + (uint32_t)grp, stop, njobs, min_qlen, ring, ring_cols,
-                            Unfit::DEFER, defer, defer_count, band_beside, P, out, err, ncells);
+                            small, Unfit::DEFER, defer, defer_count, band_beside, P, out, err, ncells);
     }
     add_cells(ncells, cells_total);
 }
@@ -456,7 +457,7 @@ template <bool W32, int C>
 __global__ void __launch_bounds__(32 * DEFER_WARPS)
 ext_long_deferred_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__restrict__ jobs,
                          const uint32_t *__restrict__ defer, const uint32_t *__restrict__ count,
-                         uint32_t *__restrict__ counter, uint32_t *__restrict__ counter_all, uint32_t njobs,
+                         uint32_t *__restrict__ counter, uint32_t *__restrict__ counter_all, uint32_t njobs, int small,
                          const __grid_constant__ ExtParams P, bwacuda_ext_result *__restrict__ out,
                          uint32_t *__restrict__ err, unsigned long long *__restrict__ cells_total)
 {
@@ -470,7 +471,7 @@ ext_long_deferred_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_
     Ring<W32> ring;
     ring.init(words + (size_t)warp * ring_words(R, W32), R);
     for (uint32_t pos = (uint32_t)warp * gridDim.x + blockIdx.x; pos < stop;) {
-        run_warp<W32, 32, C>(seq, jobs, defer, pos, stop, njobs, 0, ring, R, Unfit::SKIP, nullptr, nullptr, 0, P, out,
+        run_warp<W32, 32, C>(seq, jobs, defer, pos, stop, njobs, 0, ring, R, small, Unfit::SKIP, nullptr, nullptr, 0, P, out,
                              err, ncells);
         uint32_t b = 0;
         if (lane == 0) b = atomicAdd(counter, 1u);
@@ -488,7 +489,7 @@ ext_long_deferred_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_
                                                      needs_ring_above<W32>(jobs[defer[b + lane]], R, P));
             for (; large; large &= large - 1u)
                 run_warp<W32, 32, C>(seq, jobs, defer, b + (uint32_t)__ffs((int)large) - 1u, stop, njobs, 0, ring, RMAX,
-                                     Unfit::FAIL, nullptr, nullptr, 0, P, out, err, ncells);
+                                     small, Unfit::FAIL, nullptr, nullptr, 0, P, out, err, ncells);
         }
     }
     add_cells(ncells, cells_total);

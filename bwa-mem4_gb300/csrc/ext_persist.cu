@@ -39,6 +39,7 @@ struct SmallRule {
 // Class of a job in a small batch: 0 = the band kernel's, 1 = the other 16-bit ones, 2 = 32-bit.
 __device__ __forceinline__ uint32_t ext_small_class(const bwacuda_dev_ext_job &J, int max_sc, const SmallRule &r)
 {
+    if (J.qlen < 0) return 1u;  // the group-per-job kernel flags it
     if (!ext_fits_i16(J.qlen, J.tlen, J.h0, max_sc)) return 2u;
     const int w = clamp_band(J.w < 0 ? 0 : J.w, J.qlen, max_sc, r.end_bonus, r.o_ins, r.e_ins, r.o_del, r.e_del);
     return xl::band_takes(J.qlen, w) ? 0u : 1u;
@@ -214,7 +215,7 @@ __global__ void ext_small_bounds_kernel(const uint32_t *__restrict__ keys, uint3
 // `step` (16, 32 or 64: the autotuner's bucket granularity); longer queries
 // (16/32-bit cells only: an 8-bit job has h0 + min(qlen, tlen) * max_sc < 256)
 // take fixed caps; the last bucket of a class is open-ended.
-static const int kQcapLong[] = {385, 513, 769, 1023};
+static const int kQcapLong[] = {385, 513, 769, EXT_TPJ_QLEN_MAX + 1};
 
 static int max_qcap_of_class(int cls)
 {

@@ -68,9 +68,13 @@ struct ExtLongLaunch {
     uint32_t *defer;         // njobs entries: jobs set aside for the deferred launch
     uint32_t *defer_count;   // work + XL_WORK_DCOUNT
     int band = 0;  // 1: the band kernel runs beside this launch, which leaves it the jobs of band_takes
+    // 1: a small batch, all of whose jobs come here: a negative target length is an empty target on the
+    // queries that the length buckets run a thread each (EXT_TPJ_QLEN_MAX), as there
+    int small = 0;
     int reserve_regs = 0, reserve_threads = 0, sm_regs = 65536, sm_threads = 2048;
     cudaStream_t stream;
 };
+constexpr int EXT_TPJ_QLEN_MAX = 1022;  // longest query of a thread-per-job bucket
 
 cudaError_t ext_long_launch(const ExtLongLaunch &X, bool w32, int nsm);
 // Batched calls of up to this many jobs per SM run without length buckets in the band kernel, and host calls of up
