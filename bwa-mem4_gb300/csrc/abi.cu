@@ -319,7 +319,7 @@ extern "C" int bwacuda_set_option(bwacuda_ctx *c, int option, int64_t value)
         return batched_set_long(c, value == 0 ? INT_MAX : (int)value);
     case BWACUDA_OPT_LONG_LANES:
         if (value != 8 && value != 16 && value != 32) return BWACUDA_EINVAL;
-        return batched_set_long_lanes(c, (int)value, true);
+        return batched_set_long_lanes(c, (int)value);
     case BWACUDA_OPT_LONG_SLIDE:
         if (value < 0 || value > 2) return BWACUDA_EINVAL;
         return batched_set_long_slide(c, (int)value);

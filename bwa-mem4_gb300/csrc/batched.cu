@@ -206,13 +206,12 @@ int batched_set_long(bwacuda_ctx *c, int long_qlo)
 int batched_get_long(bwacuda_ctx *c) { return c->batched ? c->batched->long_qlo : INT_MAX; }
 
 // Lanes per job of the group-per-job kernel; a new value invalidates captured graphs.
-int batched_set_long_lanes(bwacuda_ctx *c, int lanes, bool by_option)
+int batched_set_long_lanes(bwacuda_ctx *c, int lanes)
 {
     int rc = batched_init(c);
     if (rc) return rc;
-    if (c->long_lanes != lanes || (by_option && !c->long_lanes_set)) {
+    if (c->long_lanes != lanes) {
         c->long_lanes = lanes;
-        c->long_lanes_set |= by_option;
         c->batched->gen++;
     }
     return BWACUDA_OK;
@@ -322,6 +321,7 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
     X.sm_regs = B->sm_regs;
     X.sm_threads = B->sm_threads;
     X.stream = s;
+    const bool left8 = c->long_lanes == XL_LANES_DEFAULT && n >= (size_t)B->nsm * EXT_SMALL_LEFT8_PER_SM;
     const int lanes = n < (size_t)B->nsm * 8 ? 32 : (n < (size_t)B->nsm * 20 ? 16 : 8);
     if (lanes == 8) {
         uint32_t *order = static_cast<uint32_t *>(bb.idx_out.p), *keys = static_cast<uint32_t *>(bb.keys_out.p);
@@ -332,7 +332,7 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
         X.order = order;
         bb.launched += 2 + (bb.left != 0);
         uint32_t *table = static_cast<uint32_t *>(bb.table.p);
-        const uint32_t many = c->long_lanes_set ? UINT32_MAX : (uint32_t)(B->nsm * EXT_SMALL_LEFT8_PER_SM);
+        const uint32_t many = left8 ? (uint32_t)(B->nsm * EXT_SMALL_LEFT8_PER_SM) : UINT32_MAX;
         if (bb.left && (e = ext_small_bounds(keys, n, (uint32_t)(B->nsm * EXT_SMALL_WIDE_PER_SM), many,
                                              static_cast<const ExtBucketDef *>(B->d_defs.p), B->nb, table, work, s)) !=
                            cudaSuccess)
@@ -361,7 +361,7 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
         X.bounds = X.order ? work + XL_WORK_LEFT : nullptr;
         if ((e = ext_long_launch(X, false, B->nsm)) != cudaSuccess) return e;
         bb.launched += 2;  // and the deferred launch
-        if (X.order && !c->long_lanes_set && n >= (size_t)B->nsm * EXT_SMALL_LEFT8_PER_SM) {
+        if (left8) {
             ExtLongLaunch Y = X;
             Y.lanes = 8;
             Y.counter = work + XL_WORK_COUNTER_MANY;

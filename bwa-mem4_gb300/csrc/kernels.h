@@ -48,6 +48,7 @@ constexpr int XL_WORK_BAND = 7;                                // work counter o
 constexpr int XL_WORK_WIDE = 8, XL_WORK_LEFT = 10, XL_WORK_LEFT_MANY = 12, XL_WORK_COUNTER_MANY = 14;
 constexpr int XL_WORK_WIDE_BUCKETS = 15;
 constexpr int XL_WORK_WORDS = 16;
+constexpr int XL_LANES_DEFAULT = 16;  // lanes a job of the group-per-job kernel
 constexpr int XL_RING_MIN = 256, XL_RING_FIRST_MAX = 4096;
 constexpr int XL_RING_DEFAULT = 512;  // first-launch ring when the bands are not known on the host
 
@@ -91,7 +92,8 @@ cudaError_t ext_long_launch(const ExtLongLaunch &X, bool w32, int nsm);
 constexpr int EXT_SMALL_JOBS_PER_SM = 350;
 // What the band kernel leaves of a small batch runs in the group-per-job kernels, except that 32-bit
 // jobs from EXT_SMALL_WIDE_PER_SM per SM on get a thread each in the length buckets; the 16-bit ones get
-// 8 lanes each from EXT_SMALL_LEFT8_PER_SM per SM on unless BWACUDA_OPT_LONG_LANES is set.
+// 8 lanes each from EXT_SMALL_LEFT8_PER_SM per SM on unless the option or the tuner set other lanes than
+// the default.
 // Microseconds on 152 SMs, buckets / 16 lanes / 8 lanes:
 //   jobs      150 bases, 32-bit      300 bases, band 200     600 bases, band 150
 //    3,500       990 /  505 /  568    1790 /   941 /  1131    3000 /  1964 /  2376

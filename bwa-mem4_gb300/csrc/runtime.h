@@ -98,7 +98,6 @@ struct bwacuda_ctx {
     int rescue_pair = -1;  // lanes of a group holding two byte-range jobs (rescue_wf2.cuh): 4, 8, 16; 0 off; -1: not set
     bool ungapped = false;  // ungapped-diagonal fast path on the batched extension path
     int long_lanes = 16;    // lanes per job of the group-per-job extension kernel (8, 16, 32)
-    bool long_lanes_set = false;  // BWACUDA_OPT_LONG_LANES was set
     int long_slide = 1;     // band kernel on the open-ended buckets: 0 off, 1 lanes by the bucket's jobs, 2 always 8 lanes
     size_t small_jobs = 0;  // batched calls of up to this many jobs run without length buckets in the band kernel (set from the SM count)
     int tune_candidates = 0;        // last autotune call
@@ -154,7 +153,7 @@ int batched_set_bucket_step(bwacuda_ctx *c, int step);
 void batched_get_tuning(bwacuda_ctx *c, int *tb, int *grab, int *step);
 int batched_set_long(bwacuda_ctx *c, int long_qlo);
 int batched_get_long(bwacuda_ctx *c);
-int batched_set_long_lanes(bwacuda_ctx *c, int lanes, bool by_option = false);
+int batched_set_long_lanes(bwacuda_ctx *c, int lanes);
 int batched_set_long_slide(bwacuda_ctx *c, int mode);
 int batched_set_small(bwacuda_ctx *c, size_t jobs);
 void batched_set_shapes(bwacuda_ctx *c, bool on);  // batched_prepare must have run

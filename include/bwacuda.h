@@ -151,7 +151,8 @@ typedef struct bwacuda_ctx bwacuda_ctx;
  * the group) instead of thread-per-job; 0 (default) = only the open-ended buckets, which
  * hold the queries too long for a thread's shared-memory row.  Results never depend on it. */
 #define BWACUDA_OPT_LONG_QLEN 12
-/* Lanes per job of the group-per-job extension kernel: 8, 16 (default) or 32. */
+/* Lanes per job of the group-per-job extension kernel: 8, 16 (default; small batches with many such
+ * jobs then use 8) or 32. */
 #define BWACUDA_OPT_LONG_LANES 13
 /* Mate rescue, register wavefront: 4, 8 or 16 = jobs whose every value fits a byte
  * (qlen * max_sc <= 255, padded query <= 256 columns, bwa-shaped matrix) run two
