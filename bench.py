@@ -300,20 +300,20 @@ def other_configs(args, B, ctx, st, barrier, max_over_ranks, world, rank):
     res = {}
     stream = st.cuda_stream
 
-    def timed(fn, steps=3, warmup=1):
+    def timed(fn, steps=3, warmup=1, on=ctx):
         for _ in range(warmup):
             fn()
-        ctx.sync()
-        ctx.reset_stats()
+        on.sync()
+        on.reset_stats()
         barrier()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record(st)
         for _ in range(steps):
             fn()
         e1.record(st)
-        ctx.sync()
+        on.sync()
         barrier()
-        return max_over_ranks(e0.elapsed_time(e1)) / steps, ctx.stats()
+        return max_over_ranks(e0.elapsed_time(e1)) / steps, on.stats()
 
     # mixed read lengths 100/150/250 bp, w in {50, 100, 200} per job, h0 up to 250
     n = args.mixed_jobs
@@ -523,25 +523,23 @@ def long_query_config(B, ctx, st, stream, timed, world, m=20000, seed=7000):
     d_out = torch.zeros(m * 24, dtype=torch.uint8, device="cuda")
     rows, ref = {}, None
 
-    def run(name, path):
+    def run(c, name, path):
         nonlocal ref
-        ms, stt = timed(lambda: ctx.extend_device(d_seq.data_ptr(), d_jobs.data_ptr(), m, d_out.data_ptr(),
-                                                  path=path, stream=stream), steps=2)
+        ms, stt = timed(lambda: c.extend_device(d_seq.data_ptr(), d_jobs.data_ptr(), m, d_out.data_ptr(),
+                                                path=path, stream=stream), steps=2, on=c)
         out = d_out.cpu().numpy().copy()
         ref = out if ref is None else ref
         rows[name] = {"value": round(stt["ext_cells"] / 2 * world / (ms / 1e3) / 1e9, 2),
                       "ms_per_step": round(ms, 2), "identical": bool(np.array_equal(out, ref))}
 
-    ctx.set_option(B.OPT_LONG_SLIDE, 0)
-    ctx.set_option(B.OPT_SMALL_BATCH, 0)  # a call of this size would run the band kernel unbucketed
-    for lanes in (8, 16, 32):
-        ctx.set_option(B.OPT_LONG_LANES, lanes)
-        for path, name in ((B.PATH_PLAIN, "plain"), (B.PATH_BATCHED, "batched")):
-            run(f"{name}_lanes{lanes}", path)
-    ctx.set_option(B.OPT_LONG_LANES, 16)
-    ctx.set_option(B.OPT_LONG_SLIDE, 1)
-    ctx.set_option(B.OPT_SMALL_BATCH, 350 * torch.cuda.get_device_properties(0).multi_processor_count)
-    run("batched_window", B.PATH_BATCHED)
+    with B.Context(torch.cuda.current_device()) as group:  # a context of its own: ctx keeps its defaults
+        group.set_option(B.OPT_LONG_SLIDE, 0)
+        group.set_option(B.OPT_SMALL_BATCH, 0)  # a call of this size would run the band kernel without buckets
+        for lanes in (8, 16, 32):
+            group.set_option(B.OPT_LONG_LANES, lanes)
+            for path, name in ((B.PATH_PLAIN, "plain"), (B.PATH_BATCHED, "batched")):
+                run(group, f"{name}_lanes{lanes}", path)
+    run(ctx, "batched_window", B.PATH_BATCHED)
     best = max(rows, key=lambda k: rows[k]["value"])
     window = best == "batched_window"
     del d_seq, d_jobs, d_out
