@@ -323,21 +323,37 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
     X.stream = s;
     const bool left8 = c->long_lanes == XL_LANES_DEFAULT && n >= (size_t)B->nsm * EXT_SMALL_LEFT8_PER_SM;
     const int lanes = n < (size_t)B->nsm * 8 ? 32 : (n < (size_t)B->nsm * 20 ? 16 : 8);
+    uint32_t *keys = static_cast<uint32_t *>(bb.keys_out.p), *order = static_cast<uint32_t *>(bb.idx_out.p);
+    uint32_t *kinds = work + XL_WORK_KINDS;
     if (lanes == 8) {
-        uint32_t *order = static_cast<uint32_t *>(bb.idx_out.p), *keys = static_cast<uint32_t *>(bb.keys_out.p);
         if ((e = ext_sort_jobs(d_jobs, n, P.sc.max_sc, 0u, false, d_seq, P.ug, P.zdrop, d_out,
                                static_cast<uint32_t *>(bb.keys_in.p), keys, static_cast<uint32_t *>(bb.idx_in.p), order,
-                               bb.tmp.p, bb.tmp.cap, s, &P)) != cudaSuccess)
+                               bb.tmp.p, bb.tmp.cap, s, &P, kinds)) != cudaSuccess)
             return e;
         X.order = order;
-        bb.launched += 2 + (bb.left != 0);
-        uint32_t *table = static_cast<uint32_t *>(bb.table.p);
-        const uint32_t many = left8 ? (uint32_t)(B->nsm * EXT_SMALL_LEFT8_PER_SM) : UINT32_MAX;
-        if (bb.left && (e = ext_small_bounds(keys, n, (uint32_t)(B->nsm * EXT_SMALL_WIDE_PER_SM), many,
-                                             static_cast<const ExtBucketDef *>(B->d_defs.p), B->nb, table, work, s)) !=
-                           cudaSuccess)
-            return e;
-        if ((bb.left & EXT_LEFT_32) && n >= (size_t)B->nsm * EXT_SMALL_WIDE_PER_SM) {
+        bb.launched += 2;
+    }
+    if ((e = ext_band_launch(X, lanes, work + XL_WORK_BAND, 0u, UINT32_MAX, B->nsm)) != cudaSuccess) return e;
+    // the group-per-job kernels: a kind of the sorted jobs, or every job in caller order
+    X.bounds = X.order ? kinds : nullptr;
+    if (bb.left & EXT_LEFT_16) {
+        X.counter = work + XL_WORK_COUNTER16;
+        X.part = X.order ? XL_PART_LEFT : XL_PART_ALL;
+        X.part_min = left8 ? (uint32_t)(B->nsm * EXT_SMALL_LEFT8_PER_SM) : UINT32_MAX;
+        if ((e = ext_long_launch(X, false, B->nsm)) != cudaSuccess) return e;
+        bb.launched += 2;  // and the deferred launch
+        if (left8) {
+            ExtLongLaunch Y = X;
+            Y.lanes = 8;
+            Y.counter = work + XL_WORK_COUNTER_MANY;
+            Y.part = XL_PART_LEFT_MANY;
+            if ((e = ext_long_launch(Y, false, B->nsm)) != cudaSuccess) return e;
+            ++bb.launched;
+        }
+    }
+    if (bb.left & EXT_LEFT_32) {
+        const uint32_t wide_min = (uint32_t)(B->nsm * EXT_SMALL_WIDE_PER_SM);
+        if (X.order && n >= wide_min) {
             PersistLaunch L;
             L.seq = d_seq;
             L.jobs = d_jobs;
@@ -349,30 +365,13 @@ static cudaError_t enqueue_small(bwacuda_ctx *c, BatchBufs &bb, const uint8_t *d
             L.grab = 1;
             L.stream = s;
             ++bb.launched;
-            if ((e = ext_wide_launch(L, static_cast<const ExtBucketDef *>(B->d_defs.p), B->nb, table, work, B->nsm)) !=
-                cudaSuccess)
+            if ((e = ext_wide_launch(L, keys, (uint32_t)n, wide_min, static_cast<const ExtBucketDef *>(B->d_defs.p), B->nb,
+                                     work, B->nsm)) != cudaSuccess)
                 return e;
         }
-    }
-    if ((e = ext_band_launch(X, lanes, work + XL_WORK_BAND, 0u, UINT32_MAX, B->nsm)) != cudaSuccess) return e;
-    // the group-per-job kernels: [start, stop) of the sorted jobs, or every job in caller order
-    if (bb.left & EXT_LEFT_16) {
-        X.counter = work + XL_WORK_COUNTER16;
-        X.bounds = X.order ? work + XL_WORK_LEFT : nullptr;
-        if ((e = ext_long_launch(X, false, B->nsm)) != cudaSuccess) return e;
-        bb.launched += 2;  // and the deferred launch
-        if (left8) {
-            ExtLongLaunch Y = X;
-            Y.lanes = 8;
-            Y.counter = work + XL_WORK_COUNTER_MANY;
-            Y.bounds = work + XL_WORK_LEFT_MANY;
-            if ((e = ext_long_launch(Y, false, B->nsm)) != cudaSuccess) return e;
-            ++bb.launched;
-        }
-    }
-    if (bb.left & EXT_LEFT_32) {
         X.counter = work + XL_WORK_COUNTER32;
-        X.bounds = X.order ? work + XL_WORK_WIDE : nullptr;
+        X.part = X.order ? XL_PART_WIDE : XL_PART_ALL;
+        X.part_min = wide_min;
         if ((e = ext_long_launch(X, true, B->nsm)) != cudaSuccess) return e;
         bb.launched += 2;
     }

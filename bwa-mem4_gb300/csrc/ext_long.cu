@@ -45,9 +45,9 @@ cudaError_t launch_first(const ExtLongLaunch &X, int nsm)
     }
     const size_t most = ((size_t)X.njobs * L + XL_BLOCK - 1) / XL_BLOCK;
     const uint32_t grid = (uint32_t)std::min<size_t>((size_t)per_sm * nsm, std::max<size_t>(most, 1));
-    kern<<<grid, XL_BLOCK, smem, X.stream>>>(X.seq, X.jobs, X.order, X.bounds, X.counter, X.njobs, X.min_qlen, ring,
-                                            X.defer, X.defer_count, W32 ? 0 : X.band, X.small, X.P, X.out, X.err,
-                                            X.cells);
+    kern<<<grid, XL_BLOCK, smem, X.stream>>>(X.seq, X.jobs, X.order, X.bounds, X.part, X.part_min, X.counter, X.njobs,
+                                            X.min_qlen, ring, X.defer, X.defer_count, W32 ? 0 : X.band, X.small, X.P,
+                                            X.out, X.err, X.cells);
     return cudaGetLastError();
 }
 

@@ -413,12 +413,12 @@ __device__ __forceinline__ void add_cells(unsigned long long ncells, unsigned lo
 }
 
 // Jobs come from order[bounds[0] .. bounds[1]) (order nullptr: the identity; bounds nullptr:
-// [0, njobs)), taken G = 32 / L at a time per warp from *counter; one whose band needs a larger ring
-// than ring_cols goes to defer[] (count in *defer_count).
+// [0, njobs); part: see ExtLongLaunch), taken G = 32 / L at a time per warp from *counter; one whose band
+// needs a larger ring than ring_cols goes to defer[] (count in *defer_count).
 template <bool W32, int L, int C>
 __global__ void __launch_bounds__(128)
 ext_long_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__restrict__ jobs,
-                const uint32_t *__restrict__ order, const uint32_t *__restrict__ bounds,
+                const uint32_t *__restrict__ order, const uint32_t *__restrict__ bounds, int part, uint32_t part_min,
                 uint32_t *__restrict__ counter, uint32_t njobs, int min_qlen, int ring_cols,
                 uint32_t *__restrict__ defer, uint32_t *__restrict__ defer_count, int band_beside, int small,
                 const __grid_constant__ ExtParams P, bwacuda_ext_result *__restrict__ out,
@@ -433,8 +433,17 @@ ext_long_kernel(const uint8_t *__restrict__ seq, const bwacuda_dev_ext_job *__re
     uint32_t start = 0, stop = njobs;
     if (bounds) {
         // device-written bounds, clamped to the launch's job count
-        stop = min(bounds[1], njobs);
-        start = min(bounds[0], stop);
+        if (part == XL_PART_ALL) {
+            start = bounds[0];
+            stop = bounds[1];
+        } else {
+            const uint32_t n0 = bounds[0], n1 = bounds[1], n2 = bounds[2];
+            start = part == XL_PART_WIDE ? n0 + n1 : n0;
+            stop = part == XL_PART_WIDE ? (n2 >= part_min ? bounds[XL_WORK_WIDE_STOP - XL_WORK_KINDS] : njobs) : n0 + n1;
+            if (part == (n1 >= part_min ? XL_PART_LEFT : XL_PART_LEFT_MANY)) return;
+        }
+        stop = min(stop, njobs);
+        start = min(start, stop);
     }
     unsigned long long ncells = 0;
     for (;;) {

@@ -109,12 +109,14 @@ __global__ void ext_keys_kernel(const bwacuda_dev_ext_job *__restrict__ jobs, ui
                                 uint32_t min_cls, int n_to_16, const SmallRule small,
                                 const uint8_t *__restrict__ seq, const UngappedRule ug, int zdrop,
                                 bwacuda_ext_result *__restrict__ out, uint32_t *__restrict__ keys,
-                                uint32_t *__restrict__ idx)
+                                uint32_t *__restrict__ idx, uint32_t *__restrict__ kinds)
 {
+    uint32_t kind[3] = {0u, 0u, 0u};
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const bwacuda_dev_ext_job J = jobs[k];
-        uint32_t key = ext_sort_key(J, small.on ? ext_small_class(J, max_sc, small)
-                                                : max(ext_cell_class(J, max_sc), min_cls));
+        const uint32_t cls = small.on ? ext_small_class(J, max_sc, small) : max(ext_cell_class(J, max_sc), min_cls);
+        uint32_t key = ext_sort_key(J, cls);
+        if (small.on) ++kind[cls];
         bool settled = false;
         if (ug.enabled) {
             bwacuda_ext_result r;
@@ -136,28 +138,13 @@ __global__ void ext_keys_kernel(const bwacuda_dev_ext_job *__restrict__ jobs, ui
         keys[k] = key;
         idx[k] = k;
     }
-}
-
-// First and last sort key of a bucket.
-struct BucketKeys {
-    uint32_t lo, hi;
-};
-__device__ __forceinline__ BucketKeys bucket_keys(const ExtBucketDef &d)
-{
-    const uint32_t ql_hi = d.qhi > 1023 ? 1023u : (uint32_t)d.qhi;
-    const uint32_t ql_lo = d.qlo > 1023 ? 1023u : (uint32_t)d.qlo;
-    return {((uint32_t)d.cls << 20) | ((1023u - ql_hi) << 10), ((uint32_t)d.cls << 20) | ((1023u - ql_lo) << 10) | 1023u};
-}
-
-__device__ __forceinline__ uint32_t lower_bound(const uint32_t *a, uint32_t n, uint32_t v)
-{
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (a[mid] < v) lo = mid + 1;
-        else hi = mid;
+    if (small.on) {
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            const uint32_t c = __reduce_add_sync(0xffffffffu, kind[x]);
+            if ((threadIdx.x & 31u) == 0 && c) atomicAdd(kinds + x, c);
+        }
     }
-    return lo;
 }
 
 // Bucket b covers sorted keys [key_lo, key_hi]; writes its [start, end) and
@@ -175,38 +162,6 @@ __global__ void ext_bucket_bounds_kernel(const uint32_t *__restrict__ keys, uint
     table[b * 4 + 1] = lower_bound(keys, n, k.hi + 1);
     table[b * 4 + 2] = 0;  // work counter
     table[b * 4 + 3] = 0;  // work counter of the band kernel (open-ended buckets)
-}
-
-// ext_small_bounds.  Longer queries come first in a class, so the 32-bit jobs past the thread-per-job
-// buckets lie in front of them.
-__global__ void ext_small_bounds_kernel(const uint32_t *__restrict__ keys, uint32_t n, uint32_t wide_min,
-                                        uint32_t many_min, const ExtBucketDef *__restrict__ defs, int nb,
-                                        uint32_t *__restrict__ table, uint32_t *__restrict__ work)
-{
-    __shared__ uint32_t first;  // of the 32-bit jobs in thread-per-job buckets
-    const int b = threadIdx.x;
-    const uint32_t c1 = lower_bound(keys, n, 1u << 20), c2 = lower_bound(keys, n, 2u << 20);
-    if (b == 0) first = n;
-    __syncthreads();
-    if (b < nb && defs[b].cls == 2 && defs[b].kernel == 0) {
-        const BucketKeys k = bucket_keys(defs[b]);
-        const uint32_t lo = lower_bound(keys, n, k.lo);
-        table[b * 4 + 0] = lo;
-        table[b * 4 + 1] = n - c2 >= wide_min ? lower_bound(keys, n, k.hi + 1) : lo;
-        table[b * 4 + 2] = 0;
-        atomicMin(&first, lo);
-    }
-    __syncthreads();
-    if (b == 0) {
-        const bool many = c2 - c1 >= many_min;
-        work[XL_WORK_WIDE] = c2;
-        work[XL_WORK_WIDE + 1] = n - c2 >= wide_min ? first : n;
-        work[XL_WORK_WIDE_BUCKETS] = n - c2 >= wide_min;
-        work[XL_WORK_LEFT] = c1;
-        work[XL_WORK_LEFT + 1] = many ? c1 : c2;
-        work[XL_WORK_LEFT_MANY] = c1;
-        work[XL_WORK_LEFT_MANY + 1] = many ? c2 : c1;
-    }
 }
 
 }  // namespace
@@ -259,13 +214,10 @@ int ext_bucket_defs(ExtBucketDef *defs, int max_defs, int step, int long_qlo)
 
 cudaError_t ext_sort_prefer_shared()
 {
-    // The bucket-bound kernels (one block, next to no shared memory) prefer the bucket kernels'
+    // The bucket-bound kernel (one block, no shared memory) prefers the bucket kernels'
     // maximum shared-memory carveout.  The key kernel keeps the default: its blocks live for
     // one pass only, and with the ungapped rule it reads every job's bases through L1.
-    const cudaError_t e = cudaFuncSetAttribute(ext_bucket_bounds_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                               cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(ext_small_bounds_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+    return cudaFuncSetAttribute(ext_bucket_bounds_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 cudaSharedmemCarveoutMaxShared);
 }
 
@@ -280,7 +232,7 @@ size_t ext_sort_temp_bytes(size_t n)
 cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, uint32_t min_cls, bool n_to_16,
                           const uint8_t *seq, const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
                           uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp, size_t tmp_bytes,
-                          cudaStream_t s, const ExtParams *small)
+                          cudaStream_t s, const ExtParams *small, uint32_t *kinds)
 {
     if (n == 0) return cudaSuccess;
     SmallRule sr{};
@@ -289,7 +241,7 @@ cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc,
     uint32_t grid = (uint32_t)((n + 255) / 256);
     if (grid > 8192) grid = 8192;
     ext_keys_kernel<<<grid, 256, 0, s>>>(jobs, (uint32_t)n, max_sc, min_cls, n_to_16 ? 1 : 0, sr, seq, ug, zdrop, out,
-                                         keys_in, idx_in);
+                                         keys_in, idx_in, kinds);
     return cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys_in, keys_out, idx_in, idx_out, (int)n, 0, EXT_KEY_BITS, s);
 }
 
@@ -304,13 +256,6 @@ cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int m
                                         idx_in, idx_out, tmp, tmp_bytes, s);
     if (e != cudaSuccess) return e;
     ext_bucket_bounds_kernel<<<1, EXT_MAX_BUCKETS, 0, s>>>(keys_out, (uint32_t)n, d_defs, nb, d_table);
-    return cudaGetLastError();
-}
-
-cudaError_t ext_small_bounds(const uint32_t *keys, size_t n, uint32_t wide_min, uint32_t many_min,
-                             const ExtBucketDef *d_defs, int nb, uint32_t *d_table, uint32_t *work, cudaStream_t s)
-{
-    ext_small_bounds_kernel<<<1, EXT_MAX_BUCKETS, 0, s>>>(keys, (uint32_t)n, wide_min, many_min, d_defs, nb, d_table, work);
     return cudaGetLastError();
 }
 

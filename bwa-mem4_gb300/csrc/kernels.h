@@ -42,21 +42,26 @@ constexpr int XL_WORK_DCOUNT = 0;                              // deferred jobs
 constexpr int XL_WORK_DCOUNTER16 = 1, XL_WORK_DCOUNTER32 = 3;  // work counters of the deferred launches, two each
 constexpr int XL_WORK_COUNTER16 = 5, XL_WORK_COUNTER32 = 6;    // work counters of unbucketed first launches
 constexpr int XL_WORK_BAND = 7;                                // work counter of a small batch's band launch
-// of a sorted small batch (ext_small_bounds): [start, stop) of its 32-bit jobs and of its other jobs past
-// the band kernel's window, when those are few and when they are many; the latter's work counter; whether
-// the 32-bit jobs run in length buckets
-constexpr int XL_WORK_WIDE = 8, XL_WORK_LEFT = 10, XL_WORK_LEFT_MANY = 12, XL_WORK_COUNTER_MANY = 14;
-constexpr int XL_WORK_WIDE_BUCKETS = 15;
-constexpr int XL_WORK_WORDS = 16;
+// Of a sorted small batch: the jobs of its three kinds (the band kernel's, the other 16-bit ones, the
+// 32-bit ones; they lie in this order), the work counter of a second launch over the 16-bit ones, where the
+// 32-bit jobs of the length buckets begin and those buckets' work counters.
+constexpr int XL_WORK_KINDS = 8, XL_WORK_COUNTER_MANY = 11, XL_WORK_WIDE_STOP = 12, XL_WORK_WIDE_COUNTERS = 16;
+constexpr int XL_WORK_WORDS = 16 + 64;
 constexpr int XL_LANES_DEFAULT = 16;  // lanes a job of the group-per-job kernel
 constexpr int XL_RING_MIN = 256, XL_RING_FIRST_MAX = 4096;
 constexpr int XL_RING_DEFAULT = 512;  // first-launch ring when the bands are not known on the host
 
+enum { XL_PART_ALL = 0, XL_PART_LEFT, XL_PART_LEFT_MANY, XL_PART_WIDE };
 struct ExtLongLaunch {
     const uint8_t *seq;
     const bwacuda_dev_ext_job *jobs;
     const uint32_t *order;   // job index list (nullptr: the identity)
     const uint32_t *bounds;  // [start, stop) of positions in order, device words (nullptr: [0, njobs))
+    // other than XL_PART_ALL: bounds is work + XL_WORK_KINDS and the launch runs one kind of a small batch,
+    // the other 16-bit jobs when there are fewer than part_min (LEFT) or that many (LEFT_MANY), or the
+    // 32-bit ones, without those of the length buckets when there are part_min or more (WIDE)
+    int part = 0;
+    uint32_t part_min = 0;
     uint32_t *counter;       // zeroed work counter of the first launch
     uint32_t njobs;          // jobs of the call: bounds every position and job index
     int min_qlen;            // shorter jobs belong to another launch
@@ -97,9 +102,9 @@ constexpr int EXT_SMALL_JOBS_PER_SM = 350;
 // Microseconds on 152 SMs, buckets / 16 lanes / 8 lanes:
 //   jobs      150 bases, 32-bit      300 bases, band 200     600 bases, band 150
 //    3,500       990 /  505 /  568    1790 /   941 /  1131    3000 /  1964 /  2376
-//   10,000       961 / 1317 / 1170    3240 /  2452 /  2317    5660 /  4981 /  4817
-//   20,000      1772 / 2294 / 1921    4810 /  4435 /  3695   10070 /  9147 /  7614
-//   50,000      2610 / 5300 / 4324    9490 / 10531 /  8213   25180 / 22002 / 17157
+//   10,000       884 / 1317 / 1170    3240 /  2452 /  2317    5660 /  4981 /  4817
+//   20,000      1640 / 2294 / 1921    4810 /  4435 /  3695   10070 /  9147 /  7614
+//   50,000      2408 / 5300 / 4324    9490 / 10531 /  8213   25180 / 22002 / 17157
 constexpr int EXT_SMALL_WIDE_PER_SM = 45;
 constexpr int EXT_SMALL_LEFT8_PER_SM = 60;
 constexpr int EXT_DIRECT_JOBS_PER_SM = 24;

@@ -23,6 +23,28 @@ struct ExtBucketDef {
 constexpr int EXT_MAX_BUCKETS = 64;  // one thread each in the bucket-bounds kernel
 constexpr int32_t EXT_QHI_OPEN = 1 << 30;  // qhi of a class's open-ended last bucket
 
+// First and last sort key of a bucket: class, then query length (clamped at 1023) descending, then ten
+// more bits.
+struct BucketKeys {
+    uint32_t lo, hi;
+};
+__device__ __forceinline__ BucketKeys bucket_keys(const ExtBucketDef &d)
+{
+    const uint32_t ql_hi = d.qhi > 1023 ? 1023u : (uint32_t)d.qhi;
+    const uint32_t ql_lo = d.qlo > 1023 ? 1023u : (uint32_t)d.qlo;
+    return {((uint32_t)d.cls << 20) | ((1023u - ql_hi) << 10), ((uint32_t)d.cls << 20) | ((1023u - ql_lo) << 10) | 1023u};
+}
+__device__ __forceinline__ uint32_t lower_bound(const uint32_t *a, uint32_t n, uint32_t v)
+{
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (a[mid] < v) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
 struct PersistLaunch {
     const uint8_t *seq;
     const bwacuda_dev_ext_job *jobs;
@@ -49,11 +71,11 @@ cudaError_t ext_sort_prefer_shared();
 // length and seed score, each descending.  n_to_16 puts 8-bit jobs whose query holds a code of 4 or more
 // into the 16-bit class; with ug enabled the key kernel also settles ungapped hits (results written to
 // out).  small (a small batch's parameters): the classes are the band kernel's jobs, the other 16-bit
-// ones and the 32-bit ones.
+// ones and the 32-bit ones, and their numbers are added to kinds[0 .. 3).
 cudaError_t ext_sort_jobs(const bwacuda_dev_ext_job *jobs, size_t n, int max_sc, uint32_t min_cls, bool n_to_16,
                           const uint8_t *seq, const UngappedRule &ug, int zdrop, bwacuda_ext_result *out, uint32_t *keys_in,
                           uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp, size_t tmp_bytes,
-                          cudaStream_t s, const ExtParams *small = nullptr);
+                          cudaStream_t s, const ExtParams *small = nullptr, uint32_t *kinds = nullptr);
 // ext_sort_jobs and the bucket bounds; d_table holds 4 words per bucket (start, end, work counter,
 // the band kernel's work counter).  pair_lanes false (gap costs too large for 16-bit lanes) keeps every
 // job out of the 8-bit class.
@@ -63,15 +85,11 @@ cudaError_t ext_sort_and_bucket(const bwacuda_dev_ext_job *jobs, size_t n, int m
                                 uint32_t *keys_out, uint32_t *idx_in, uint32_t *idx_out, void *tmp,
                                 size_t tmp_bytes, const ExtBucketDef *d_defs, int nb, uint32_t *d_table,
                                 cudaStream_t s);
-// Who runs what the band kernel leaves of a sorted small batch (keys of ext_sort_jobs with small): the
-// 32-bit jobs in their length buckets from wide_min on, below that in work[XL_WORK_WIDE], which always
-// holds those past the thread-per-job buckets; the 16-bit ones in work[XL_WORK_LEFT], or from many_min
-// on in work[XL_WORK_LEFT_MANY].
-cudaError_t ext_small_bounds(const uint32_t *keys, size_t n, uint32_t wide_min, uint32_t many_min,
-                             const ExtBucketDef *d_defs, int nb, uint32_t *d_table, uint32_t *work, cudaStream_t s);
-// Those buckets of 32-bit jobs, all in one launch (ext_wide.cu).
-cudaError_t ext_wide_launch(const PersistLaunch &L, const ExtBucketDef *d_defs, int nb, uint32_t *d_table,
-                            const uint32_t *work, int nsm);
+// The 32-bit jobs of a sorted small batch (its sort keys and kinds) in their thread-per-job length buckets,
+// all in one launch (ext_wide.cu), when there are wide_min or more of them: work[XL_WORK_WIDE_STOP] is then
+// where those begin.
+cudaError_t ext_wide_launch(const PersistLaunch &L, const uint32_t *keys, uint32_t n, uint32_t wide_min,
+                            const ExtBucketDef *d_defs, int nb, uint32_t *work, int nsm);
 // An 8-bit bucket with two jobs per thread (ext_dual.cuh): scorings of at most five letters.
 cudaError_t ext_dual_launch(const PersistLaunch &L, const ExtBucketDef &d, uint32_t *d_bucket_table, int nsm);
 // per-grab instantiations (ext_persist_g1.cu, _g2.cu, _g4.cu)
