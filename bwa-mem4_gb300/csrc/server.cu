@@ -31,6 +31,8 @@
 #include <unordered_map>
 #include <vector>
 
+#include "ext_job.cuh"
+#include "ext_long.cuh"
 #include "kernels.h"
 #include "runtime.h"
 
@@ -97,6 +99,7 @@ struct Request {
     uint64_t seq_bytes = 0, scr_entries = 0;
     int qmax = 0;
     bool wide = false;  // rescue: needs 32-bit cells
+    int left = 0;       // extension: what the band kernel may leave (EXT_LEFT_*)
     ReqState state = PENDING;
     int rc = BWACUDA_OK;
     Clock::time_point t_submit, t_done;
@@ -216,6 +219,7 @@ int plan_request(Request *r, int m)
     uint64_t seq = 0, scr = 0;
     int qmax = 0;
     bool wide = false;
+    long long top = 0;  // extension: largest value bound
     if (r->dev) {
         r->goff.resize(r->n);
         if (r->kind == 1) r->gsoff.resize(r->n);
@@ -235,7 +239,9 @@ int plan_request(Request *r, int m)
             seq += (uint64_t)ql + (uint64_t)tl;
         }
         qmax = std::max(qmax, ql);
-        if (r->kind == 1) {
+        if (r->kind == 0) {
+            top = std::max(top, ext_value_bound(ql, tl, r->ejobs[k].h0, r->P.sc.max_sc));
+        } else {
             if (r->dev) r->gsoff[k] = scr;
             scr += rescue_scratch_entries(tl);
             if ((long long)std::min(ql, tl) * std::max(r->max_sc, 0) >= 32768) wide = true;
@@ -244,6 +250,8 @@ int plan_request(Request *r, int m)
     (void)m;
     r->qmax = qmax;
     r->wide = wide;
+    // (a job's clamped band is at most the request's)
+    r->left = (top >= 32768 || qmax >= 65535 ? EXT_LEFT_32 : 0) | (xl::band_takes(qmax, r->w) ? 0 : EXT_LEFT_16);
     r->seq_bytes = seq;
     r->scr_entries = scr;
     const size_t rsz = r->kind == 0 ? sizeof(bwacuda_ext_result) : sizeof(bwacuda_rescue_result);
@@ -480,7 +488,7 @@ bool launch_wave(ServerState *S)
     if (lead->kind == 1 && (e = srv_grow(slot->soff, n * 8 + 64)) != cudaSuccess) return fail(e);
     // gather descriptors (and tracker offsets) of the wave
     size_t at = 0;
-    int qmax = 0;
+    int qmax = 0, left = 0;
     bool wide = false;
     for (Request *r : group) {
         if ((e = cudaMemcpyAsync((char *)slot->desc.p + at * 32, S->d_arena + r->off + r->desc_at, r->n * 32,
@@ -490,11 +498,13 @@ bool launch_wave(ServerState *S)
         at += r->n;
         qmax = std::max(qmax, r->qmax);
         wide |= r->wide;
+        left |= r->left;
     }
     uint32_t *err = static_cast<uint32_t *>(slot->flags.p);
     unsigned long long *cells = reinterpret_cast<unsigned long long *>((char *)slot->flags.p + 8);
     if ((e = cudaMemsetAsync(slot->flags.p, 0, 16, s)) != cudaSuccess) return fail(e);
     if (lead->kind == 0) {
+        batched_set_left(slot->bb, left);
         e = batched_enqueue(S->c, slot->bb, S->d_arena, static_cast<const bwacuda_dev_ext_job *>(slot->desc.p), n,
                             lead->P, static_cast<bwacuda_ext_result *>(slot->out.p), s, err, cells);
         if (e != cudaSuccess) return fail(e);

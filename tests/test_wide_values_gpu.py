@@ -143,3 +143,21 @@ def test_small_batches_left_by_the_band_kernel_take_no_longer(n, qlen, w, h0):
         ctx.set_option(B.OPT_SMALL_BATCH, 0)
         buckets = d.best_ms()
     assert small < 1.05 * buckets, (small, buckets)
+
+
+def test_serving_waves_with_and_without_such_jobs():
+    """Small requests through the serving loop, whose waves launch what their requests' jobs may need."""
+    with B.Context(0) as ctx:
+        ctx.server_start(hbm_budget_bytes=256 << 20, max_waves=2)
+        try:
+            reqs = []
+            for k in range(24):
+                n = [1, 40, 700, 3500, 9500][k % 5]
+                js = _flat(n, [30, 100, 250] if k % 2 else [30, 268, 269, 300, 1100], seed=k, w=[100, 150][k // 2 % 2])
+                if k % 3 == 0:
+                    js.h0[n // 2:] = 33000
+                reqs.append((ctx.submit_extend(js, w=int(js.w[0])), js))
+            for rid, js in reqs:
+                assert np.array_equal(ctx.wait(rid)[0], oracle.extend_batch(js)[0])
+        finally:
+            ctx.server_stop()
