@@ -717,15 +717,24 @@ namespace bwacuda {
 //   65,536                                      3712   3087   2880
 //   262,144                                    14219  11335  10563
 // (100 x 400, 60 x 700 and 240 x 1200 bp order the same way.)
+// The forward pass alone (mode 2) stops each job at its own score, which a pair can only do together, and
+// tells its group so with two shuffles and a vote a row: one job a group up to 200 jobs per SM.  Through
+// host buffers, jobs that stop at 100 of 150 / that never stop:
+//   jobs      1 job in 16 lanes       in 8 lanes       2 jobs in 8 lanes      in 4 lanes
+//   3,000         431 / 442            480 / 494          717 / 710           855 / 863
+//   5,000         561 / 669            611 / 628          766 / 750           856 / 870
+//   20,000       1426 / 1814          1424 / 1612        1562 / 1518         1695 / 1777
+//   60,000       3757 / 5007          3589 / 4176        3440 / 3711         3518 / 3581
 struct RescueShape {
     int pair, lanes;
 };
-static RescueShape rescue_shape(const bwacuda_ctx *c, size_t n)
+static RescueShape rescue_shape(const bwacuda_ctx *c, size_t n, int mode)
 {
     const size_t per_sm = n / (size_t)c->nsm;
     const int lanes = c->rescue_lanes ? c->rescue_lanes : (per_sm < 8 ? 32 : (per_sm < 24 ? 16 : 8));
     if (c->rescue_pair >= 0) return {c->rescue_pair, c->rescue_lanes ? c->rescue_lanes : 16};
-    if (c->rescue_lanes || per_sm < 16) return {0, lanes};  // lanes set by the caller: the kernel they name
+    // lanes set by the caller: the kernel they name
+    if (c->rescue_lanes || per_sm < (mode == 2 ? 200 : 16)) return {0, lanes};
     return {per_sm < 64 ? 8 : 4, lanes};
 }
 
@@ -735,7 +744,7 @@ static RescueShape rescue_shape(const bwacuda_ctx *c, size_t n)
 cudaError_t rescue_narrow_launch(bwacuda_ctx *c, const RescueLaunch &L)
 {
     if (c->rescue_kernel == BWACUDA_RESCUE_AUTO && L.qcap <= rescue_wf_max_qpad() && L.only_wide != 2) {
-        const RescueShape sh = rescue_shape(c, L.n);
+        const RescueShape sh = rescue_shape(c, L.n, L.mode);
         if (!sh.pair) return rescue_wf_launch(L, L.qcap, sh.lanes);
         // jobs whose values fit a byte: two per group; the rest in the 32-bit wavefront
         int cols = 0;
