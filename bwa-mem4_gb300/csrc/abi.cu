@@ -725,16 +725,31 @@ namespace bwacuda {
 //   5,000         561 / 669            611 / 628          766 / 750           856 / 870
 //   20,000       1426 / 1814          1424 / 1612        1562 / 1518         1695 / 1777
 //   60,000       3757 / 5007          3589 / 4176        3440 / 3711         3518 / 3581
+// Short queries want pairs from a little later on (16 lanes a job / pairs: 36 bases, 3,000 jobs 171 / 212 us,
+// 4,000 203 / 204; 100 bases, 3,000 251 / 276, 4,000 296 / 277; 250 bases, 2,500 557 / 536).  Jobs past a
+// byte among the others take a launch behind the pairs', whose latency a small batch does not win back
+// (240-256 bases, 3,000 jobs 560 / 882, 10,000 1461 / 1566, 16,000 2188 / 2117).
 struct RescueShape {
     int pair, lanes;
 };
-static RescueShape rescue_shape(const bwacuda_ctx *c, size_t n, int mode)
+static RescueShape rescue_shape(const bwacuda_ctx *c, const RescueLaunch &L)
 {
-    const size_t per_sm = n / (size_t)c->nsm;
+    const size_t per_sm = L.n / (size_t)c->nsm;
+    const int cols = L.qcap - 16;
+    size_t from = L.mode == 2 ? 200 : (cols <= 128 ? 24 : (cols <= 208 ? 20 : 16));
+    if (L.beside) {  // the column classes of a ragged batch fill the GPU together
+        const bool mixed = L.npair > 0 && L.npair < L.n;
+        from = L.mode == 2 && L.beside / (size_t)c->nsm < 200 ? ~(size_t)0 : (mixed ? 32 : 16);
+    } else if (L.npair == 0) {
+        from = ~(size_t)0;
+    } else if (L.npair == RESCUE_NPAIR_UNKNOWN ? (long long)cols * L.sc.max_sc > 255 : L.npair < L.n) {
+        from = std::max(from, (size_t)100);
+        if (L.npair < L.n / 4) from = ~(size_t)0;
+    }
     const int lanes = c->rescue_lanes ? c->rescue_lanes : (per_sm < 8 ? 32 : (per_sm < 24 ? 16 : 8));
     if (c->rescue_pair >= 0) return {c->rescue_pair, c->rescue_lanes ? c->rescue_lanes : 16};
     // lanes set by the caller: the kernel they name
-    if (c->rescue_lanes || per_sm < (mode == 2 ? 200 : 16)) return {0, lanes};
+    if (c->rescue_lanes || per_sm < from) return {0, lanes};
     return {per_sm < 64 ? 8 : 4, lanes};
 }
 
@@ -744,7 +759,7 @@ static RescueShape rescue_shape(const bwacuda_ctx *c, size_t n, int mode)
 cudaError_t rescue_narrow_launch(bwacuda_ctx *c, const RescueLaunch &L)
 {
     if (c->rescue_kernel == BWACUDA_RESCUE_AUTO && L.qcap <= rescue_wf_max_qpad() && L.only_wide != 2) {
-        const RescueShape sh = rescue_shape(c, L.n, L.mode);
+        const RescueShape sh = rescue_shape(c, L);
         if (!sh.pair) return rescue_wf_launch(L, L.qcap, sh.lanes);
         // jobs whose values fit a byte: two per group; the rest in the 32-bit wavefront
         int cols = 0;
@@ -768,6 +783,7 @@ struct ResChunk {
     int qcap;
     uint32_t nwide;
     uint64_t cells;
+    size_t npair = 0;
 };
 
 template <typename JobT>
@@ -777,7 +793,7 @@ ResChunk pack_res_chunk(bwacuda_ctx *c, Slot &sl, const JobT *jobs, size_t c0, s
     ResChunk ch{c0, cn, 0, 0, 0, 0, 0};
     *rc = BWACUDA_OK;
     const int P = c->pool.size();
-    std::vector<uint64_t> part_bytes(P, 0), part_scr(P, 0), part_cells(P, 0);
+    std::vector<uint64_t> part_bytes(P, 0), part_scr(P, 0), part_cells(P, 0), part_pairs(P, 0);
     std::vector<int> part_q(P, 0), part_bad(P, 0);
     std::vector<std::vector<uint32_t>> part_wide(P);
     auto range = [&](int id, size_t &b, size_t &e) {
@@ -787,7 +803,7 @@ ResChunk pack_res_chunk(bwacuda_ctx *c, Slot &sl, const JobT *jobs, size_t c0, s
     c->pool.run([&](int id) {
         size_t b, e;
         range(id, b, e);
-        uint64_t sum = 0, scr = 0, cells = 0;
+        uint64_t sum = 0, scr = 0, cells = 0, pairs = 0;
         int qc = 0;
         for (size_t k = b; k < e; ++k) {
             const JobT &J = jobs[c0 + k];
@@ -799,6 +815,7 @@ ResChunk pack_res_chunk(bwacuda_ctx *c, Slot &sl, const JobT *jobs, size_t c0, s
             sum += (uint64_t)J.qlen + (uint64_t)J.tlen;
             scr += rescue_scratch_entries(J.tlen);
             cells += (uint64_t)J.qlen * (uint64_t)J.tlen;
+            pairs += (long long)J.qlen * max_sc <= 255;
             // room for the padded forward query and the reverse pass's padding
             int q16 = (J.qlen + 15) / 16 * 16;
             int ln = lanes ? lanes : (J.qlen * max_sc < 250 ? 16 : 8);
@@ -812,6 +829,7 @@ ResChunk pack_res_chunk(bwacuda_ctx *c, Slot &sl, const JobT *jobs, size_t c0, s
         part_scr[id] = scr;
         part_q[id] = qc;
         part_cells[id] = cells;
+        part_pairs[id] = pairs;
     });
     for (int id = 0; id < P; ++id) {
         if (part_bad[id]) { *rc = BWACUDA_EINVAL; return ch; }
@@ -820,6 +838,7 @@ ResChunk pack_res_chunk(bwacuda_ctx *c, Slot &sl, const JobT *jobs, size_t c0, s
         ch.qcap = std::max(ch.qcap, part_q[id]);
         ch.nwide += (uint32_t)part_wide[id].size();
         ch.cells += part_cells[id];
+        ch.npair += part_pairs[id];
     }
     cudaError_t e;
     const size_t jb = cn * sizeof(bwacuda_dev_rescue_job);
@@ -898,6 +917,7 @@ int run_res_chunk(bwacuda_ctx *c, Slot &sl, const ResChunk &ch, const Scoring &s
     L.order = nullptr;
     L.count_ptr = nullptr;
     L.n = ch.cn;
+    L.npair = ch.npair;
     L.sc = sc;
     L.mode = mode;
     L.lanes = lanes;

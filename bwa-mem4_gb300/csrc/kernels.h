@@ -123,7 +123,10 @@ int ext_long_ring_for_band(int w);
 
 // Rescue (ksw_local_fwd / ksw_align2).  mode: 0 = batched_ksw_align2,
 // 1 = scalar ksw_align2, 2 = forward pass only (per-job minsc / endsc).
+constexpr size_t RESCUE_NPAIR_UNKNOWN = ~(size_t)0;
 struct RescueLaunch {
+    size_t npair = RESCUE_NPAIR_UNKNOWN;  // jobs of the launch whose values fit a byte, where the caller knows
+    size_t beside = 0;  // jobs of the launches that run side by side, this one among them (0: it runs alone)
     const uint8_t *seq;
     const bwacuda_dev_rescue_job *jobs;
     const uint32_t *order;

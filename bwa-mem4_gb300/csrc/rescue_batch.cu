@@ -48,6 +48,7 @@ struct RescueStat {
     uint32_t nwide;     // jobs whose values need 32-bit cells
     uint32_t not_u8, not_i16;  // some job leaves the reference's 8- / 16-bit batch width
     uint32_t hist[RC_CLASSES];
+    uint32_t pairs[RC_CLASSES];  // those of a class whose values fit a byte
     unsigned long long useful;  // sum over jobs of class columns x target rows
     unsigned long long cells;   // sum of qlen x tlen
 };
@@ -62,6 +63,7 @@ struct SurveyAcc {
         tmax = max(tmax, tlen);
         const int cls = rescue_class(qlen);
         atomicAdd(hist_s + cls, 1u);
+        if ((long long)qlen * max_sc <= 255) atomicAdd(hist_s + RC_CLASSES + cls, 1u);
         useful += (unsigned long long)rescue_class_cols(cls < 7 ? cls : 7, qlen) * (unsigned)tlen;
         cells += (unsigned long long)(unsigned)qlen * (unsigned)tlen;
         const long long top = (long long)min(qlen, tlen) * max_sc;
@@ -94,7 +96,11 @@ struct SurveyAcc {
             if (cells) atomicAdd(&st->cells, cells);
         }
         __syncthreads();  // every thread's counts are in hist_s
-        if (threadIdx.x < RC_CLASSES && hist_s[threadIdx.x]) atomicAdd(st->hist + threadIdx.x, hist_s[threadIdx.x]);
+        if (threadIdx.x < RC_CLASSES && hist_s[threadIdx.x]) {
+            atomicAdd(st->hist + threadIdx.x, hist_s[threadIdx.x]);
+            const uint32_t p = hist_s[RC_CLASSES + threadIdx.x];
+            if (p) atomicAdd(st->pairs + threadIdx.x, p);
+        }
     }
 };
 
@@ -108,8 +114,8 @@ __device__ __forceinline__ uint16_t rescue_sort_key(int qlen, int tlen)
 __global__ void rescue_survey_kernel(const bwacuda_dev_rescue_job *__restrict__ jobs, uint32_t n, int max_sc,
                                      RescueStat *__restrict__ st)
 {
-    __shared__ uint32_t hist_s[RC_CLASSES];
-    if (threadIdx.x < RC_CLASSES) hist_s[threadIdx.x] = 0u;
+    __shared__ uint32_t hist_s[2 * RC_CLASSES];  // jobs of a class, and those whose values fit a byte
+    if (threadIdx.x < 2 * RC_CLASSES) hist_s[threadIdx.x] = 0u;
     __syncthreads();
     SurveyAcc a;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
@@ -197,6 +203,8 @@ cudaError_t rescue_launch_classes(bwacuda_ctx *c, RescueWork &W, const RescueSta
     const bool sort = L.only_wide != 2 && c->rescue_kernel == BWACUDA_RESCUE_AUTO && L.n >= (size_t)c->nsm * 8 &&
                       all > 1.125 * (double)st.useful;
     if (!sort) {
+        L.npair = 0;
+        for (int b = 0; b < RC_CLASSES; ++b) L.npair += st.pairs[b];
         c->stats.kernel_launches += 1;
         return rescue_narrow_launch(c, L);
     }
@@ -230,6 +238,8 @@ cudaError_t rescue_launch_classes(bwacuda_ctx *c, RescueWork &W, const RescueSta
         RescueLaunch X = L;
         X.order = i1 + at[b];
         X.n = st.hist[b];
+        X.npair = st.pairs[b];
+        X.beside = n;
         X.qcap = std::min(L.qcap, rescue_class_cols(b, st.qmax) + 16);
         X.stream = nl % (RescueState::NSIDE + 1) ? R.side[nl % (RescueState::NSIDE + 1) - 1] : s;
         e = rescue_narrow_launch(c, X);
@@ -352,8 +362,8 @@ __global__ void __launch_bounds__(RG_THREADS) rescue_plan_kernel(const JobT *__r
                                                                  bwacuda_dev_rescue_job *__restrict__ djobs,
                                                                  RescueStat *__restrict__ st)
 {
-    __shared__ uint32_t hist_s[RC_CLASSES];
-    if (threadIdx.x < RC_CLASSES) hist_s[threadIdx.x] = 0u;
+    __shared__ uint32_t hist_s[2 * RC_CLASSES];  // jobs of a class, and those whose values fit a byte
+    if (threadIdx.x < 2 * RC_CLASSES) hist_s[threadIdx.x] = 0u;
     __syncthreads();
     SurveyAcc a;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {

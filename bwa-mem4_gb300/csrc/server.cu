@@ -99,6 +99,7 @@ struct Request {
     uint64_t seq_bytes = 0, scr_entries = 0;
     int qmax = 0;
     bool wide = false;  // rescue: needs 32-bit cells
+    size_t npair = 0;   // rescue: jobs whose values fit a byte
     int left = 0;       // extension: what the band kernel may leave (EXT_LEFT_*)
     ReqState state = PENDING;
     int rc = BWACUDA_OK;
@@ -220,6 +221,7 @@ int plan_request(Request *r, int m)
     int qmax = 0;
     bool wide = false;
     long long top = 0;  // extension: largest value bound
+    size_t npair = 0;
     if (r->dev) {
         r->goff.resize(r->n);
         if (r->kind == 1) r->gsoff.resize(r->n);
@@ -242,6 +244,7 @@ int plan_request(Request *r, int m)
         if (r->kind == 0) {
             top = std::max(top, ext_value_bound(ql, tl, r->ejobs[k].h0, r->P.sc.max_sc));
         } else {
+            npair += (long long)ql * r->max_sc <= 255;
             if (r->dev) r->gsoff[k] = scr;
             scr += rescue_scratch_entries(tl);
             if ((long long)std::min(ql, tl) * std::max(r->max_sc, 0) >= 32768) wide = true;
@@ -250,6 +253,7 @@ int plan_request(Request *r, int m)
     (void)m;
     r->qmax = qmax;
     r->wide = wide;
+    r->npair = npair;
     // (a job's clamped band is at most the request's)
     r->left = (top >= 32768 || qmax >= 65535 ? EXT_LEFT_32 : 0) | (xl::band_takes(qmax, r->w) ? 0 : EXT_LEFT_16);
     r->seq_bytes = seq;
@@ -489,6 +493,7 @@ bool launch_wave(ServerState *S)
     // gather descriptors (and tracker offsets) of the wave
     size_t at = 0;
     int qmax = 0, left = 0;
+    size_t npair = 0;
     bool wide = false;
     for (Request *r : group) {
         if ((e = cudaMemcpyAsync((char *)slot->desc.p + at * 32, S->d_arena + r->off + r->desc_at, r->n * 32,
@@ -499,6 +504,7 @@ bool launch_wave(ServerState *S)
         qmax = std::max(qmax, r->qmax);
         wide |= r->wide;
         left |= r->left;
+        npair += r->npair;
     }
     uint32_t *err = static_cast<uint32_t *>(slot->flags.p);
     unsigned long long *cells = reinterpret_cast<unsigned long long *>((char *)slot->flags.p + 8);
@@ -515,6 +521,7 @@ bool launch_wave(ServerState *S)
         L.order = nullptr;
         L.count_ptr = nullptr;
         L.n = n;
+        L.npair = npair;
         L.sc = lead->sc;
         L.mode = 0;
         L.lanes = 0;
