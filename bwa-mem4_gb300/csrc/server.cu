@@ -510,7 +510,11 @@ bool launch_wave(ServerState *S)
     unsigned long long *cells = reinterpret_cast<unsigned long long *>((char *)slot->flags.p + 8);
     if ((e = cudaMemsetAsync(slot->flags.p, 0, 16, s)) != cudaSuccess) return fail(e);
     if (lead->kind == 0) {
-        batched_set_left(slot->bb, left);
+        // The hints save a small wave launches that find nothing (12 requests of up to 12,473 jobs 1.83 -> 1.80 ms, 30 of
+        // up to 7,796 3.57 -> 3.46).  Past 100 jobs per SM there is nothing to win, and 12 requests of up to 96,208 jobs
+        // measured 6.33 ms with them, 6.24 without.
+        const bool hints = n < (size_t)batched_nsm(S->c) * 100;
+        batched_set_left(slot->bb, hints ? left : EXT_LEFT_16 | EXT_LEFT_32);
         e = batched_enqueue(S->c, slot->bb, S->d_arena, static_cast<const bwacuda_dev_ext_job *>(slot->desc.p), n,
                             lead->P, static_cast<bwacuda_ext_result *>(slot->out.p), s, err, cells);
         if (e != cudaSuccess) return fail(e);
